@@ -436,9 +436,9 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
     const unsigned np = fcp->np, nt = fcp->nt;
     const float t_end = (float)nt + 1.f;  // x_tr' at or above this: rejected, a bin of margin
     // accepted range of p with one bin of margin each side: x = p - pmin in
-    // [-1, np + 1]; |p| <= np + 1 for auto-correlations
-    const float p_lo = RMU ? -(float)(nt + 1u) : (AUTO ? -(float)(np + 1u) : pmin_f - 1.f);
-    const float p_hi = RMU ? (float)(nt + 1u) : (AUTO ? (float)(np + 1u) : pmin_f + (float)np + 1.f);
+    // [-1, np + 1]; |p| <= pmin + np + 1 for auto-correlations
+    const float p_hi = RMU ? (float)(nt + 1u) : pmin_f + (float)np + 1.f;
+    const float p_lo = RMU || AUTO ? -p_hi : pmin_f - 1.f;
     const float inv_mu = fcp->inv_mu, mu_off = fcp->mu_off, g_mu0 = fcp->g_mu0;
     const int hs = fcp->hstride;
     const CfSmem L = cf_smem(nbins, max_pix1, nwarps);
