@@ -197,6 +197,14 @@ int launch_cf_xi_fp64(const Binning &b, const pg_forest_set &s1, const pg_forest
                       const int64_t *nbr_offsets, const int32_t *nbr_index, const double *nbr_angle,
                       const int32_t *work_order, int64_t num_work, const pg_xi_rows &out,
                       Scratch *scratch, int num_sms, cudaStream_t stream);
+// FP64 sums with FP32 decisions (pg_pairs_runs64.cu), and what it covers.
+bool runs64_covers(const Binning &b, const pg_forest_set &s1, const pg_forest_set &s2,
+                   int64_t num_work);
+int launch_cf_xi_runs64(const Binning &b, const pg_forest_set &s1, const pg_forest_set &s2,
+                        const int64_t *nbr_offsets, const int32_t *nbr_index,
+                        const double *nbr_angle, const int32_t *work_order, int64_t num_work,
+                        const pg_xi_rows &out, Scratch *scratch, int num_sms,
+                        cudaStream_t stream);
 int launch_xcf_xi_fp64(const Binning &b, const pg_forest_set &forests, const pg_forest_set &objs,
                        const int64_t *nbr_offsets, const int32_t *nbr_index, const double *nbr_angle,
                        const int32_t *work_order, int64_t num_work, const pg_xi_rows &out,

@@ -1,4 +1,6 @@
-// Plain all-FP64 pair accumulation (the "plain GPU drop-in" form).
+// Plain all-FP64 pair accumulation (the "plain GPU drop-in" form): the
+// angular and r-mu binnings, forests too long for the shared memory of
+// pg_pairs_runs64.cu, and the correlation with quasars.
 //
 // Persistent kernel: each CTA pops a work item (one forest of set 1 with all
 // of its neighbours) from a global counter, accumulates every pixel pair in
@@ -277,6 +279,9 @@ int launch_cf_xi_fp64(const Binning &b, const pg_forest_set &s1, const pg_forest
                       const int32_t *work_order, int64_t num_work, const pg_xi_rows &out,
                       Scratch *scratch, int num_sms, cudaStream_t stream) {
     if (num_work <= 0) return PG_OK;
+    if (runs64_covers(b, s1, s2, num_work))
+        return launch_cf_xi_runs64(b, s1, s2, nbr_offsets, nbr_index, nbr_angle, work_order,
+                                   num_work, out, scratch, num_sms, stream);
     const size_t smem = hist64_bytes(b.nbins);
     int grid = 0, rc;
     if (smem <= 220 * 1024) {
