@@ -415,6 +415,24 @@ int pg_mlp_colsum(const uint16_t *x, int32_t m, int32_t n, int64_t ldx, float *o
 int pg_mlp_mse_grad(const float *y, const float *t, int32_t m, int32_t n, uint16_t *dy,
                     float *loss, void *stream);
 
+/* The 66-256-256-256-2 network's training forward pass in one call: x
+ * [m, stride] bf16 (stride a multiple of 8, columns 0..65 used), params16 /
+ * params as pg_mlp_to_bf16 makes them; writes the hidden activations h[0..2]
+ * ([m, 256] bf16), the pre-activations z[0..2] ([m, 256] FP32; z or an entry
+ * may be NULL) and y [m, 2]. z and h are host arrays of device pointers,
+ * 16-byte aligned like x and params16 (y: 8 bytes). */
+int pg_mlp_train_forward(const uint16_t *params16, const float *params, const uint16_t *x,
+                         int32_t m, int32_t stride, float *const *z, uint16_t *const *h, float *y,
+                         void *stream);
+
+/* Its backward pass: loss[0] = sum (y - target)^2 / m and the gradients of
+ * all parameters in grads (the layout of params). work: (3 * 256 + 8) m bf16,
+ * 16-byte aligned. */
+int pg_mlp_train_backward(const uint16_t *params16, const uint16_t *x, int32_t m, int32_t stride,
+                          const float *const *z, const uint16_t *const *h, const float *y,
+                          const float *target, uint16_t *work, float *grads, float *loss,
+                          void *stream);
+
 /* One Adam step on n FP32 parameters (bias-corrected, optional decoupled
  * weight decay); writes the bf16 copy when params_bf16 is not NULL. */
 int pg_mlp_adam(float *params, const float *grads, float *m1, float *m2, uint16_t *params_bf16,

@@ -3,14 +3,13 @@
 // sums for bias gradients, the MSE-loss gradient and Adam). The reference
 // has no counterpart; see include/picca_gb300.h.
 //
-// GEMM: C[M,N] = A[M,K] B[K,N] with arbitrary element strides for A and B
-// (so X W, dZ W^T and X^T dZ all use one kernel). CTA tile 64 x 64 x 32,
+// GEMM: C[M,N] = A[M,K] B[K,N] with arbitrary element strides for A and B:
+// the form for operands that the asynchronous tile GEMM (pg_mlp_train.cu)
+// does not take (odd strides or bases). CTA tile 64 x 64 x 32,
 // four warps in a 2 x 2 arrangement, each warp 32 x 32 built from
 // mma.sync m16n8k16 BF16 -> FP32 tiles. Operands are staged through shared
 // memory with bounds checks (zero fill), so M, N and K need no padding.
-#include <cuda_bf16.h>
-
-#include "pg_internal.cuh"
+#include "pg_mlp_common.cuh"
 
 namespace pg {
 namespace {
@@ -18,47 +17,6 @@ namespace {
 constexpr int kBM = 64, kBN = 64, kBK = 32;
 constexpr int kGemmThreads = 128;
 constexpr int kPadA = 8, kPadB = 8;
-
-__device__ __forceinline__ uint32_t pack_bf16(__nv_bfloat16 lo, __nv_bfloat16 hi) {
-    uint32_t l = (uint32_t)__bfloat16_as_ushort(lo);
-    uint32_t h = (uint32_t)__bfloat16_as_ushort(hi);
-    return l | (h << 16);
-}
-
-__device__ __forceinline__ void mma_bf16(float d[4], const uint32_t a[4], const uint32_t b[2]) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 "
-        "{%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-
-__device__ __forceinline__ float gelu(float x) {
-    return 0.5f * x * (1.f + erff(x * 0.70710678118654752f));
-}
-
-__device__ __forceinline__ float gelu_grad(float x) {
-    const float cdf = 0.5f * (1.f + erff(x * 0.70710678118654752f));
-    const float pdf = 0.39894228040143268f * expf(-0.5f * x * x);
-    return cdf + x * pdf;
-}
-
-struct GemmArgs {
-    const __nv_bfloat16 *a;
-    int64_t sam, sak;
-    const __nv_bfloat16 *b;
-    int64_t sbk, sbn;
-    int m, n, k;
-    const float *bias;         // [n] or nullptr
-    int epilogue;              // PG_MLP_EPI_* flags
-    const float *zin;          // pre-activations for the GELU backward, [m, ldz]
-    float *zout;               // pre-activations written by the forward, [m, ldz]
-    int64_t ldz;
-    __nv_bfloat16 *c;          // bf16 output [m, ldc] or nullptr
-    float *cf;                 // fp32 output [m, ldc] or nullptr
-    int64_t ldc;
-    float beta;                // fp32 output: cf = acc + beta * cf
-};
 
 __global__ void __launch_bounds__(kGemmThreads) gemm_bf16_kernel(const GemmArgs g) {
     __shared__ __align__(16) __nv_bfloat16 As[kBM][kBK + kPadA];
@@ -210,6 +168,8 @@ int pg_mlp_gemm(const uint16_t *a, int64_t sam, int64_t sak, const uint16_t *b, 
     g.m = m; g.n = n; g.k = k;
     g.bias = bias; g.epilogue = epilogue; g.zin = zin; g.zout = zout; g.ldz = ldz;
     g.c = reinterpret_cast<__nv_bfloat16 *>(c); g.cf = cf; g.ldc = ldc; g.beta = beta;
+    const int rc = launch_mlp_gemm_tile(g, static_cast<cudaStream_t>(stream));
+    if (rc != PG_ERR_UNSUPPORTED) return rc;
     const dim3 grid((unsigned)((n + kBN - 1) / kBN), (unsigned)((m + kBM - 1) / kBM));
     gemm_bf16_kernel<<<grid, kGemmThreads, 0, static_cast<cudaStream_t>(stream)>>>(g);
     return check_cuda(cudaGetLastError());

@@ -5,9 +5,10 @@ forest's flux divided by the current mean continuum (64 rest-frame bins),
 its redshift and signal-to-noise, the continuum parameters relative to the
 reference starting point a0 (the ivar-weighted mean flux,
 expected_fluxes/utils.py:92): targets (a/a0 - 1, b/a0). Training runs every
-matrix product in the library's BF16 GEMM with FP32 accumulation (forward
-with fused bias + GELU, backward with fused GELU derivative) and the
-library's Adam kernel on FP32 master weights; inference (the warm start)
+matrix product in the library's BF16 tile GEMM with FP32 accumulation (forward
+with fused bias + GELU, backward with fused GELU derivative; a call each,
+pg_mlp_train_forward and pg_mlp_train_backward) and the library's Adam kernel
+on FP32 master weights; inference (the warm start)
 runs the whole network in one fused tcgen05 kernel (pg_mlp_forward).
 
 The plain fit stays the reference: ``warm_fit`` starts the damped Newton
@@ -51,7 +52,9 @@ def _bind():
     lib.pg_mlp_forward.argtypes = [vp, vp, vp, vp, i64, i32, vp, vp]
     lib.pg_mlp_warm_start.argtypes = [vp, ctypes.POINTER(continuum.SpectraC),
                                       ctypes.POINTER(continuum.ContModelC), vp, vp, vp, vp, vp]
-    for name in ("pg_mlp_gemm", "pg_mlp_colsum", "pg_mlp_mse_grad", "pg_mlp_adam",
+    lib.pg_mlp_train_forward.argtypes = [vp, vp, vp, i32, i32, vp, vp, vp, vp]
+    lib.pg_mlp_train_backward.argtypes = [vp, vp, i32, i32, vp, vp, vp, vp, vp, vp, vp, vp]
+    for name in ("pg_mlp_gemm", "pg_mlp_train_forward", "pg_mlp_train_backward", "pg_mlp_colsum", "pg_mlp_mse_grad", "pg_mlp_adam",
                  "pg_mlp_to_bf16", "pg_mlp_features", "pg_mlp_pack", "pg_mlp_forward",
                  "pg_mlp_warm_start"):
         getattr(lib, name).restype = ctypes.c_int
@@ -61,6 +64,15 @@ def _bind():
 
 def _ptr(t):
     return None if t is None else t.data_ptr()
+
+
+def _ptrs(tensors):
+    return (ctypes.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
+
+
+def _aligned(t, nbytes):
+    """The tensor, or a copy where its storage starts off a wide load's boundary."""
+    return t.clone() if t.data_ptr() % nbytes else t
 
 
 class WarmStartMLP:
@@ -159,54 +171,37 @@ class WarmStartMLP:
     def forward(self, x16, keep=False):
         """x16: bf16 [m, FEATURE_STRIDE] (first 66 columns used). Returns
         the FP32 output [m, 2] and, with keep=True, the activations."""
+        lib = _bind()
         m = x16.shape[0]
-        w16 = self._views(self.params16)
-        w32 = self._views(self.params)
-        acts = {"x": x16}
-        h = x16
-        ld_in, k_in = FEATURE_STRIDE, NUM_FEATURES
-        for layer in range(3):
-            z = torch.empty(m, HIDDEN, dtype=torch.float32, device=self.device) if keep else None
-            out = torch.empty(m, HIDDEN, dtype=torch.bfloat16, device=self.device)
-            self.gemm(h, ld_in, 1, w16[layer][0], HIDDEN, 1, m, HIDDEN, k_in,
-                      bias=w32[layer][1], epilogue=EPI_GELU, zout=z, ldz=HIDDEN, c=out,
-                      ldc=HIDDEN)
-            acts[f"z{layer}"] = z
-            acts[f"h{layer}"] = out
-            h, ld_in, k_in = out, HIDDEN, HIDDEN
+        x16 = _aligned(x16, 16)
+        h = torch.empty(3, m, HIDDEN, dtype=torch.bfloat16, device=self.device).unbind(0)
+        z = torch.empty(3, m, HIDDEN, dtype=torch.float32, device=self.device).unbind(0) \
+            if keep else None
         y = torch.empty(m, NUM_OUT, dtype=torch.float32, device=self.device)
-        self.gemm(h, HIDDEN, 1, w16[3][0], NUM_OUT, 1, m, NUM_OUT, HIDDEN, bias=w32[3][1],
-                  cf=y, ldc=NUM_OUT)
-        return (y, acts) if keep else y
+        check(lib.pg_mlp_train_forward(self.params16.data_ptr(), self.params.data_ptr(),
+                                       x16.data_ptr(), m, FEATURE_STRIDE,
+                                       _ptrs(z) if keep else None, _ptrs(h), y.data_ptr(),
+                                       self._stream()), "mlp training forward")
+        if not keep:
+            return y
+        acts = {"x": x16}
+        for layer in range(3):
+            acts[f"z{layer}"], acts[f"h{layer}"] = z[layer], h[layer]
+        return y, acts
 
     def backward(self, acts, y, target):
         """Gradients of the MSE loss into self.grads; returns the loss."""
         lib = _bind()
         m = y.shape[0]
-        loss = torch.zeros(1, dtype=torch.float32, device=self.device)
-        dz = torch.empty(m, NUM_OUT, dtype=torch.bfloat16, device=self.device)
-        check(lib.pg_mlp_mse_grad(y.data_ptr(), target.data_ptr(), m, NUM_OUT, dz.data_ptr(),
-                                  loss.data_ptr(), self._stream()), "mse grad")
-        w16 = self._views(self.params16)
-        g32 = self._views(self.grads)
-        width = NUM_OUT
-        for layer in (3, 2, 1, 0):
-            h_in = acts["x"] if layer == 0 else acts[f"h{layer - 1}"]
-            ld_in = FEATURE_STRIDE if layer == 0 else HIDDEN
-            fan_in = NUM_FEATURES if layer == 0 else HIDDEN
-            # dW = h_in^T dz
-            self.gemm(h_in, 1, ld_in, dz, width, 1, fan_in, width, m, cf=g32[layer][0],
-                      ldc=width)
-            check(lib.pg_mlp_colsum(dz.data_ptr(), m, width, width, g32[layer][1].data_ptr(),
-                                    self._stream()), "colsum")
-            if layer == 0:
-                break
-            # dz_prev = (dz W^T) * gelu'(z_prev)
-            dprev = torch.empty(m, HIDDEN, dtype=torch.bfloat16, device=self.device)
-            self.gemm(dz, width, 1, w16[layer][0], 1, width, m, HIDDEN, width,
-                      epilogue=EPI_GELU_GRAD, zin=acts[f"z{layer - 1}"], ldz=HIDDEN, c=dprev,
-                      ldc=HIDDEN)
-            dz, width = dprev, HIDDEN
+        y, target = _aligned(y, 8), _aligned(target, 8)
+        loss = torch.empty(1, dtype=torch.float32, device=self.device)
+        work = torch.empty(m * (3 * HIDDEN + 8), dtype=torch.bfloat16, device=self.device)
+        z, h = ([acts[f"{kind}{layer}"] for layer in range(3)] for kind in "zh")
+        check(lib.pg_mlp_train_backward(self.params16.data_ptr(), acts["x"].data_ptr(), m,
+                                        FEATURE_STRIDE, _ptrs(z), _ptrs(h), y.data_ptr(),
+                                        target.data_ptr(), work.data_ptr(),
+                                        self.grads.data_ptr(), loss.data_ptr(), self._stream()),
+              "mlp training backward")
         return loss
 
     def adam_step(self, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.0):
