@@ -616,7 +616,8 @@ typedef struct pg_wick_sums {
  * slices: entry q then does slice unit_slice[q] of unit_slices[q] (both
  * optional: NULL = one slice per entry); every slice of a pair must be
  * listed exactly once. work: pg_cf_wick_work_bytes() bytes of device
- * scratch (16-byte aligned); fewer bytes run fewer CTAs. Forests must have
+ * scratch (16-byte aligned; max_ctas: the number of units, for a smaller
+ * buffer when there are few); fewer bytes run fewer units at a time. Forests must have
  * at most 32767 pixels. */
 int pg_cf_wick_work_bytes(pg_plan *plan, const pg_corr_params *params, int32_t max_pixels1,
                           int32_t max_pixels2, int64_t max_ctas, uint64_t *bytes);

@@ -696,6 +696,9 @@ int pg_cf_wick_work_bytes(pg_plan *plan, const pg_corr_params *params, int32_t m
     if ((rc = wick_t123_grid(nb, plan->num_sms, &grid))) return rc;
     if (max_ctas > 0) grid = (int)std::min<int64_t>(grid, max_ctas);
     *bytes = (uint64_t)grid * (uint64_t)max_pixels1 * (uint64_t)max_pixels2 * sizeof(uint32_t);
+    const uint64_t lists = wick_segments_bytes(nb, max_pixels1, max_pixels2, max_ctas);
+    if (wick_segments_covers(nb, max_pixels1, max_pixels2, lists))
+        *bytes = std::max<uint64_t>(*bytes, lists);
     return PG_OK;
 }
 
@@ -731,6 +734,11 @@ int pg_cf_wick(pg_plan *plan, const pg_corr_params *params, const pg_forest_set 
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     plan->last_stream = st;
     if ((rc = reset_scratch(plan, st))) return rc;
+    if (wick_segments_covers(nb, s1->max_pixels, t->max_pixels, work_bytes))
+        return launch_wick_segments(*params, *s1, *t, zw1, zw2, x_offsets1, arena1, x_offsets2,
+                                    arena2, pair_first, pair_second, pair_angle, unit_slice,
+                                    num_pairs, work, work_bytes, *out, scratch_of(plan),
+                                    plan->num_sms, st);
     return launch_wick_t123(*params, *s1, *t, zw1, zw2, x_offsets1, arena1, x_offsets2, arena2,
                             pair_first, pair_second, pair_angle, unit_slice, unit_slices, num_pairs,
                             static_cast<uint32_t *>(work), cap, grid, *out, scratch_of(plan), st);

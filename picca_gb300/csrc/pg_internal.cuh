@@ -281,6 +281,18 @@ int launch_wick_t123(const pg_corr_params &p, const pg_forest_set &s1, const pg_
                      int64_t cap, int grid, const pg_wick_sums &out, Scratch *scratch,
                      cudaStream_t stream);
 
+// T1-T3 over row and column segments (pg_wick_segments.cu): the work buffer
+// it wants for num_pairs pairs, and what it covers.
+uint64_t wick_segments_bytes(int nb, int max1, int max2, int64_t num_pairs);
+bool wick_segments_covers(int nb, int max1, int max2, uint64_t work_bytes);
+int launch_wick_segments(const pg_corr_params &p, const pg_forest_set &s1,
+                         const pg_forest_set &s2, const double *zw1, const double *zw2,
+                         const int64_t *xo1, const double *xa1, const int64_t *xo2,
+                         const double *xa2, const int32_t *pair_first, const int32_t *pair_second,
+                         const double *pair_angle, const int32_t *unit_slice, int64_t num_pairs,
+                         void *work, uint64_t work_bytes, const pg_wick_sums &out,
+                         Scratch *scratch, int num_sms, cudaStream_t stream);
+
 int64_t xwick_cta_bytes(int64_t cap, int64_t max_quasars);
 int xwick_grid(int nb, int num_sms, int *grid);
 int launch_xwick(const pg_corr_params &p, const pg_forest_set &forests, const pg_forest_set &objs,

@@ -18,7 +18,10 @@
 //    reference recomputes it for every pair). The diagonal is stored as 0:
 //    no term uses it, and a zero there lets T3 run without branches. xi_1d
 //    is scipy's nearest-neighbour rule (count of cell bounds below |dll|).
-//  * wick_t123_kernel: one CTA per forest pair (persistent). It counts the
+//  * wick_t123_kernel: one CTA per forest pair (persistent), for what the
+//    segment form (pg_wick_segments.cu) does not cover: forests of more than
+//    about 780 pixels, more bins than its lists hold, or a work buffer too
+//    small for them. It counts the
 //    listed pixel pairs per bin in shared memory (with WALL, NB and the
 //    diagonal T1), sorts them by bin into a per-CTA list (counting sort),
 //    then every warp takes 32 pixel pairs a of one bin P and sweeps all b
