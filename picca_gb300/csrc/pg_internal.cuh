@@ -18,6 +18,10 @@ constexpr double kPi = 3.141592653589793;
 // 2 arcsec in radians, py/picca/constants.py:16
 constexpr double kSmallAngle = 2. / 3600. * 3.141592653589793 / 180.;
 
+// Dynamic shared memory of a CTA: the 227 KB of an SM less what the kernels'
+// static arrays take (at most 1,360 bytes).
+constexpr size_t kMaxDynSmem = 227 * 1024 - 1536;
+
 // Scratch owned by a plan (device memory, a few hundred bytes).
 struct Scratch {
     int32_t work_counter;      // persistent-kernel work queue head

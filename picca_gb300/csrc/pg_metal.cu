@@ -528,7 +528,7 @@ __global__ void __launch_bounds__(kMrWarps * 32, 5) metal_runs_kernel(
 // What the sweeps cover: both forests staged, pixel indices of 16 bits.
 bool metal_runs_covers(const pg_forest_set &s1, const pg_forest_set &s2) {
     return s1.max_pixels <= 65535 && s2.max_pixels <= 65535 &&
-           mr_smem(s1.max_pixels, s2.max_pixels).total <= 227 * 1024;
+           mr_smem(s1.max_pixels, s2.max_pixels).total <= kMaxDynSmem;
 }
 
 int launch_metal_runs(const MetalConst &c, const pg_forest_set &s1, const pg_forest_set &s2,

@@ -3,6 +3,7 @@
 // which also sums in FP32, and pg_pairs_runs64.cu, which sums in FP64).
 #pragma once
 
+#include "pg_f64_bits.cuh"
 #include "pg_internal.cuh"
 
 namespace pg {
@@ -56,9 +57,25 @@ __device__ __forceinline__ ParGuard par_guard(const FastConst *fcp, float max_rh
 // FP32 value of a weight that stays nonzero when the FP64 weight is nonzero
 // (a weight below the FP32 range still counts its pairs, as in FP64).
 __device__ __forceinline__ float weight32(double w) {
-    const float f = (float)w;
-    if (f == 0.f && w != 0.) return w > 0 ? 1.401298464e-45f : -1.401298464e-45f;
-    return f;
+    const float f = f64_to_f32(w);  // subnormal results come as 0
+    if (f != 0.f) return f;
+    const float g = (float)w;
+    if (g == 0.f && w != 0.) return w > 0 ? 1.401298464e-45f : -1.401298464e-45f;
+    return g;
+}
+
+// x as an FP32 pair: hi the nearest FP32 (to the last bit on ties), lo the
+// rest (hi + lo equal to x to about 2^-48 of |x|), by integer and FP32
+// operations; values near the ends of the FP32 range by conversions.
+__device__ __forceinline__ float2 split_near(double x) {
+    const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7FFu;
+    if (e - 949u > 200u && x != 0.) {
+        const float hi = (float)x;
+        return make_float2(hi, (float)(x - (double)hi));
+    }
+    const float2 t = split_f64(x);  // hi truncated
+    const float hi = t.x + t.y;
+    return make_float2(hi, t.y - (hi - t.x));
 }
 
 // round(x) (as unsigned; negative results wrap to large values) and the

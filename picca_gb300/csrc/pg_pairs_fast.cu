@@ -62,7 +62,7 @@ namespace pg {
 namespace {
 
 constexpr int kQueue = 256;                   // FP64 recheck entries per warp (cross)
-constexpr int kCfQueue = 128;                 // FP64 recheck entries per warp (auto)
+constexpr int kCfQueue = 96;                  // FP64 recheck entries per warp (auto)
 constexpr int kAccQ = 64;                     // run ring per warp (<= 31 + 32 entries held)
 constexpr int kChunk = 128;                   // forest-2 pixels staged per warp at a time
 constexpr int kRunMax = 64;                   // pairs summed in FP32 registers per run
@@ -101,14 +101,19 @@ __device__ __forceinline__ void flush_rows(float *h, const FastConst &fc, const 
     const int nbins = fc.nbins, hs = fc.hstride;
     const size_t o = (size_t)row * nbins;
     int *hnb = reinterpret_cast<int *>(h + H_NB * hs);
+    const double per_p = 1. / fc.inv_p, per_t = 1. / fc.inv_t;
     for (int b = threadIdx.x; b < nbins; b += blockDim.x) {
         const int nb = hnb[b];
         if (nb == 0) continue;
-        atomicAdd(&out.weights[o + b], (double)h[H_WE * hs + b] + (double)h[H_WEL * hs + b]);
-        atomicAdd(&out.xi[o + b], (double)h[H_XI * hs + b] + (double)h[H_XIL * hs + b]);
-        atomicAdd(&out.r_par[o + b], (double)h[H_PW * hs + b] / fc.inv_p);
-        atomicAdd(&out.r_trans[o + b], (double)h[H_TW * hs + b] / fc.inv_t);
-        atomicAdd(&out.z[o + b], 0.5 * (double)h[H_ZW * hs + b]);
+        // four FP64 operations a bin (conversions on the integer pipe, the
+        // scales as products; with divisions and FP64-pipe conversions a flush
+        // of 2,500 bins was about 35 operations a bin, 23 us of the pipe)
+        auto at = [&](int k) { return f32_to_f64(h[k * hs + b]); };
+        atomicAdd(&out.weights[o + b], at(H_WE) + at(H_WEL));
+        atomicAdd(&out.xi[o + b], at(H_XI) + at(H_XIL));
+        atomicAdd(&out.r_par[o + b], at(H_PW) * per_p);
+        atomicAdd(&out.r_trans[o + b], at(H_TW) * per_t);
+        atomicAdd(&out.z[o + b], f32_to_f64(0.5f * h[H_ZW * hs + b]));
         atomicAdd((unsigned long long *)&out.num_pairs[o + b], (unsigned long long)nb);
 #pragma unroll
         for (int k = 0; k < H_NB; ++k) h[k * hs + b] = 0.f;
@@ -197,18 +202,17 @@ __device__ __forceinline__ bool stage_forest1(const pg_forest_set &s1, int64_t a
     float local_max = 0.f;
     for (int i = threadIdx.x; i < n1; i += blockDim.x) {
         const double w = s1.weights[a0 + i];
-        const double rho_d = s1.r_comov[a0 + i] - r_ref;
-        const float rho = (float)rho_d;
-        const float d = (float)s1.dist_m[a0 + i];
-        p1[i] = make_float4(rho, d, (float)s1.z[a0 + i], weight32(w));
-        const float2 dw = split2(s1.delta[a0 + i] * w);
-        p2[i] = make_float4(dw.x, dw.y, (float)(rho_d - (double)rho), 0.f);
-        local_max = fmaxf(local_max, fabsf(rho));
-        if (i + 1 < n1)
-            ordered &= (float)(s1.r_comov[a0 + i + 1] - r_ref) >= rho &&
-                       (float)s1.dist_m[a0 + i + 1] >= d;
+        const float2 rho = split_near(s1.r_comov[a0 + i] - r_ref);
+        p1[i] = make_float4(rho.x, f64_to_f32(s1.dist_m[a0 + i]), f64_to_f32(s1.z[a0 + i]),
+                            weight32(w));
+        const float2 dw = split_near(s1.delta[a0 + i] * w);
+        p2[i] = make_float4(dw.x, dw.y, rho.y, 0.f);
+        local_max = fmaxf(local_max, fabsf(rho.x));
     }
     if (local_max > 0.f) atomicMax(max_rho_bits, __float_as_uint(local_max));
+    __syncthreads();
+    for (int i = threadIdx.x; i + 1 < n1; i += blockDim.x)
+        ordered &= p1[i + 1].x >= p1[i].x && p1[i + 1].y >= p1[i].y;
     return __syncthreads_and(ordered) != 0;
 }
 
@@ -239,7 +243,7 @@ __device__ __forceinline__ void cf_drain(const Binning &b, const FastConst *__re
         const double w1 = s1.weights[ia], w2 = s2.weights[jb];
         const float w12 = weight32(w1) * weight32(w2);
         // delta_times_weight1 * delta_times_weight2 (py/picca/cf.py:367-369)
-        const float2 dw12 = split2((s1.delta[ia] * w1) * (s2.delta[jb] * w2));
+        const float2 dw12 = split_near((s1.delta[ia] * w1) * (s2.delta[jb] * w2));
         const float pv = (float)(r_par * inv_p);
         const float tv = (float)(r_trans * inv_t);
         const float zs = (float)z1 + (float)z2;
@@ -283,8 +287,10 @@ __host__ __device__ inline CfSmem cf_smem(int nbins, int max_pix1, int nwarps) {
     CfSmem l;
     const size_t mp = (size_t)((max_pix1 + 1) & ~1);
     l.cells = 0;
-    l.p1 = (size_t)((nbins + 3) & ~3) * H_COUNT * 4;
-    l.p1x = l.p1 + mp * 16;
+    // a lane off its diagonal's range reads up to kChunk + 31 pixels before
+    // forest 1 or kChunk after it (into the padding; the pair is not accepted)
+    l.p1 = (size_t)((nbins + 3) & ~3) * H_COUNT * 4 + (size_t)(kChunk + 32) * 16;
+    l.p1x = l.p1 + (mp + kChunk) * 16;
     l.warps = l.p1x + mp * 16;
     l.buf = 0;
     l.bufx = l.buf + (size_t)kChunk * 16;
@@ -337,7 +343,8 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
     const __grid_constant__ pg_forest_set s1, const __grid_constant__ pg_forest_set s2,
     const int64_t *__restrict__ nbr_offsets, const int32_t *__restrict__ nbr_index,
     const double *__restrict__ nbr_angle, const int32_t *__restrict__ work_order,
-    int64_t num_work, const __grid_constant__ pg_xi_rows out, Scratch *scratch, int max_pix1) {
+    int64_t num_work, int slices, const __grid_constant__ pg_xi_rows out, Scratch *scratch,
+    int max_pix1) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int item_slot;
     __shared__ unsigned max_rho_bits;
@@ -360,6 +367,9 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
     // [-1, np + 1]; |p| <= pmin + np + 1 for auto-correlations
     const float p_hi = RMU ? (float)(nt + 1u) : pmin_f + (float)np + 1.f;
     const float p_lo = RMU || AUTO ? -p_hi : pmin_f - 1.f;
+    // coordinates at or above these round past the last bin
+    const float x_end = (float)np - 0.5f, y_end = (float)nt - 0.5f;
+    const unsigned bin_off = kMagicBits * (nt + 1u);  // of the bins of a sweep
     const float inv_mu = fcp->inv_mu, mu_off = fcp->mu_off, g_mu0 = fcp->g_mu0;
     const int hs = fcp->hstride;
     const CfSmem L = cf_smem(nbins, max_pix1, nwarps);
@@ -378,10 +388,17 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
     if (lane == 0) visited[warp] = 0ull;
 
     for (;;) {
-        const int item = next_item(scratch, &item_slot, &max_rho_bits);
-        if (item >= num_work) break;
+        const int unit = next_item(scratch, &item_slot, &max_rho_bits);
+        if (unit >= num_work * slices) break;
+        const int item = unit / slices, slice = unit - item * slices;
         const int64_t f1 = work_order ? work_order[item] : item;
         const int32_t row = s1.row[f1];
+        // this slice's neighbours: a slice keeps every warp busy for at
+        // least two of them
+        const int64_t k0 = nbr_offsets[f1], nk = nbr_offsets[f1 + 1] - k0;
+        const int cut = (int)max((int64_t)1, min((int64_t)slices, nk / (2 * nwarps)));
+        if (slice >= cut) continue;
+        const int64_t k_lo = k0 + nk * slice / cut, k1 = k0 + nk * (slice + 1) / cut;
         const int64_t a0 = s1.pix_offset[f1];
         const int64_t n1_64 = s1.pix_offset[f1 + 1] - a0;
         if (n1_64 > max_pix1 || n1_64 > 65535 || n1_64 < 1) {
@@ -395,16 +412,19 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
             f1_geom[0] = s1.x_cart[f1]; f1_geom[1] = s1.y_cart[f1]; f1_geom[2] = s1.z_cart[f1];
             f1_geom[3] = s1.ra[f1]; f1_geom[4] = s1.dec[f1]; f1_geom[5] = s1.cos_dec[f1];
             f1_geom[6] = s1.z_qso[f1];
-            nbr_next = nbr_offsets[f1];
+            nbr_next = k_lo;
         }
         const bool sorted1 = stage_forest1(s1, a0, n1, r_ref, const_cast<float4 *>(p1),
                                            const_cast<float4 *>(p1x), &max_rho_bits);
+        // every pixel has a weight and a distance that is not negative
+        bool plain1 = true;
+        for (int i = lane; i < n1; i += 32) plain1 &= (p1[i].w != 0.f) & (p1[i].y >= 0.f);
+        plain1 = __all_sync(0xffffffffu, plain1);
         const ParGuard pg = par_guard(fcp, __uint_as_float(max_rho_bits));
         const float h_par = pg.h_par, low_clamp = pg.low_clamp;
         // r-mu: r carries the errors of both staged coordinates
         const float g_pp = pg.guard_v;
         const float h_r = h_tr - g_pp;
-        const int64_t k1 = nbr_offsets[f1 + 1];
         int head = 0, tail = 0;  // run ring of this warp (warp-uniform)
         int qn = 0;              // FP64 re-decision queue of this warp
         for (;;) {
@@ -485,7 +505,7 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
                 // stage the chunk: nB = -cp rho2, t = st d2 - 1/2; a pixel
                 // without weight or vetoed against quasar 1 gets w = 0 (and
                 // t = kFar), which removes its pairs in the sweep
-                bool ordered2 = true, valid2 = true;
+                bool valid2 = true, plain2 = true;
                 __syncwarp();
                 for (int jl = lane; jl < jn; jl += 32) {
                     const int64_t jj = b0 + jc + jl;
@@ -493,25 +513,34 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
                     bool ok = w2 != 0;
                     if (EXTRA && zerr_pair && ok)
                         ok = !zerr_veto(s2.z[jj], f1_geom[6], b.zerr_kms);
+                    // conversions on the FP64 pipe, which has room here: the
+                    // kernel is bound by issue
                     const double rho2_d = s2.r_comov[jj] - r_ref;
-                    const float rho2 = (float)rho2_d;
-                    const float d2 = (float)s2.dist_m[jj];
-                    // nB = -cp rho2 as hi + lo (exact to 2^-48): hi decides,
-                    // hi + lo enters the summed r_par
-                    const double nb_d = -((double)cp * rho2_d);
+                    const float rho2 = (float)rho2_d, d2 = (float)s2.dist_m[jj];
+                    // nB = -cp rho2 as hi + lo (the product's rounding error
+                    // and the low part): hi decides, hi + lo enters the
+                    // summed r_par
                     const float nb_h = -__fmul_rn(cp, rho2);
+                    const float nb_l = __fmaf_rn(-cp, (float)(rho2_d - (double)rho2),
+                                                 -__fmaf_rn(cp, rho2, nb_h));
                     buf[jl] = make_float4(nb_h, ok ? __fmaf_rn(st, d2, RMU ? 0.f : -0.5f) : kFar,
                                           (float)s2.z[jj], ok ? weight32(w2) : 0.f);
                     const float2 dw = split2(s2.delta[jj] * w2);
-                    bufx[jl] = make_float4(dw.x, dw.y, (float)(nb_d - (double)nb_h), 0.f);
+                    bufx[jl] = make_float4(dw.x, dw.y, nb_l, 0.f);
                     valid2 &= ok;
-                    if (jl + 1 < jn)
-                        ordered2 &= (float)(s2.r_comov[jj + 1] - r_ref) >= rho2 &&
-                                    (float)s2.dist_m[jj + 1] >= d2;
+                    plain2 &= d2 >= 0.f;
+                }
+                __syncwarp();
+                // the order that the searches below rely on
+                bool ordered2 = true, ordered_t = true;
+                for (int jl = lane; jl + 1 < jn; jl += 32) {
+                    ordered2 &= buf[jl + 1].x <= buf[jl].x;
+                    ordered_t &= buf[jl + 1].y >= buf[jl].y;
                 }
                 ordered2 = __all_sync(0xffffffffu, ordered2);
+                ordered_t = __all_sync(0xffffffffu, ordered_t);
                 valid2 = __all_sync(0xffffffffu, valid2);
-                __syncwarp();
+                plain2 = __all_sync(0xffffffffu, plain2);
                 // the band of diagonals [d_lo, d_hi) holding every pair within
                 // one bin of the accepted r_par range
                 int d_lo = jc - (n1 - 1), d_hi = jc + jn;
@@ -535,7 +564,10 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
                     d_hi = hi;
                 }
                 // along a diagonal x_tr' is non-decreasing: trim at t_end
-                const bool t_trim = sorted1 && ordered2 && valid2 && st > 0.f;
+                const bool t_trim = sorted1 && ordered_t && valid2 && st > 0.f;
+                // no pixel without weight on either side and no negative
+                // r_trans: no test for them per pair
+                const bool plain = plain1 && plain2 && valid2 && st >= 0.f;
                 for (int d0 = d_lo; d0 < d_hi; d0 += 32) {
                     const int d = d0 + lane;
                     // this lane's pairs: j = i + d in the chunk, i in forest 1
@@ -576,7 +608,7 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
                         const int pos = (tail + __popc(m & lt_mask)) & (kAccQ - 1);
                         if (flag) {
                             acc0[pos] = make_float4(r_xi, r_xil, r_w, r_pw);
-                            acc1[pos] = make_float4(r_tw, r_zw, __uint_as_float(run_bin),
+                            acc1[pos] = make_float4(r_tw, r_zw, __uint_as_float(run_bin - bin_off),
                                                     __uint_as_float((unsigned)run_n));
                         }
                         tail += __popc(m);
@@ -586,47 +618,62 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
                     // pairs is evaluated before either enters the run, so
                     // that their dependency chains overlap)
                     struct PairEval {
-                        unsigned bin;
-                        int i;
+                        unsigned bin;  // offset by bin_off
                         float pp, xt, zs, w12;
                         bool acc, near;
                     };
-                    auto eval = [&](int js, PairEval &e) {
-                        bool in = (js >= sa) & (js < sb);
-                        const int i = in ? js - joff : 0;
+                    const unsigned len = ia < ib ? (unsigned)(ib - ia) : 0u;
+                    auto eval = [&](int js, PairEval &e, auto checked) {
+                        bool in = (unsigned)(js - sa) < len;
+                        const int i = js - joff;
                         if (EXTRA && zerr_pair && in) in = ((veto1[i >> 5] >> (i & 31)) & 1u) == 0u;
-                        // js <= g_hi <= jn: the clamp keeps the (unused) read
-                        // one past the group's range inside the chunk
+                        // a lane outside its range reads padding or a
+                        // neighbouring array: not accepted, not queued
                         const float4 q1 = p1[i];
-                        const float4 q2 = buf[min(js, jn - 1)];
+                        const float4 q2 = buf[js];
                         const float pp = __fmaf_rn(cp, q1.x, q2.x);
                         const float v = fabsf(pp);
                         const float pv = AUTO ? v : pp;
                         const float xt = __fmaf_rn(st, q1.y, q2.y);
-                        float fp, ft;
-                        unsigned ip, it;
+                        // coordinates xc (r_par or mu) and yc (r_trans or r):
+                        // bins are the integers they round to. Nothing lies
+                        // below 0 in yc (r_trans, r >= 0; else checked) and,
+                        // with LOWX, in xc; an edge is inside the guard band
+                        float xc, yc, rx, ry;
                         bool near;
+                        unsigned bx, by;
+                        auto round_at = [](float x, float &rem) {
+                            const float y = x + kMagic;
+                            rem = x - (y - kMagic);
+                            return __float_as_uint(y);
+                        };
                         if (RMU) {
                             const float r2 = __fmaf_rn(pp, pp, xt * xt);
                             const float sinv = rsqrtf(r2);
                             const float ru = r2 * sinv;
                             const float mu = pv * sinv;
-                            float xm = __fmaf_rn(mu, inv_mu, -mu_off);
-                            if (LOWX) xm = fmaxf(xm, low_clamp);
-                            ip = round_rem(xm, fp);
-                            it = round_rem(ru - 0.5f, ft);
+                            xc = __fmaf_rn(mu, inv_mu, -mu_off);
+                            if (LOWX) xc = fmaxf(xc, low_clamp);
+                            yc = ru - 0.5f;
+                            bx = round_at(xc, rx);
+                            by = round_at(yc, ry);
                             const float gm = __fmaf_rn(g_pp * sinv, inv_mu, g_mu0);
-                            near = !(gm < 0.25f) | (fabsf(fp) > 0.5f - gm) | (fabsf(ft) > h_r);
+                            near = !(gm < 0.25f) | (fabsf(rx) > 0.5f - gm) | (fabsf(ry) > h_r);
                         } else {
-                            const float xp = LOWX ? fmaxf(pv - pc, low_clamp) : pv - pc;
-                            ip = round_rem(xp, fp);
-                            it = round_rem(xt, ft);
-                            near = (fabsf(fp) > h_par) | (fabsf(ft) > h_tr);
+                            xc = LOWX ? fmaxf(pv - pc, low_clamp) : pv - pc;
+                            yc = xt;
+                            bx = round_at(xc, rx);
+                            by = round_at(yc, ry);
+                            near = (fabsf(rx) > h_par) | (fabsf(ry) > h_tr);
                         }
                         // a pixel without weight or vetoed (w staged as 0) pairs
                         // with nothing: neither accepted nor queued
-                        in &= (q1.w != 0.f) & (q2.w != 0.f);
-                        bool ok = (ip < np) & (it < nt);
+                        bool ok = (xc < x_end) & (yc < y_end);
+                        if (decltype(checked)::value) {
+                            in &= (q1.w != 0.f) & (q2.w != 0.f);
+                            ok &= yc > -0.5f;
+                        }
+                        if (!LOWX) ok &= xc > -0.5f;
                         const float zs = q1.z + q2.z;
                         if (EXTRA) {
                             if (shp) {
@@ -645,8 +692,7 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
                         near &= in;
                         e.acc = in & ok & !near;
                         e.near = near;
-                        e.bin = ip * nt + it;
-                        e.i = i;
+                        e.bin = bx * nt + by;
                         e.pp = pp;
                         e.xt = xt;
                         e.zs = zs;
@@ -670,7 +716,7 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
                         }
                         if (brk) run_bin = e.bin;
                         if (e.acc) {
-                            const float4 x1 = p1x[e.i];
+                            const float4 x1 = p1x[js - joff];
                             const float4 x2 = bufx[js];
                             const float w12 = e.w12;
                             float th, tl;
@@ -697,31 +743,36 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
                             ++run_n;
                         }
                     };
-                    for (int js = g_lo; js < g_hi; js += 2) {
-                        PairEval ea, eb;
-                        eval(js, ea);
-                        eval(js + 1, eb);  // js + 1 = g_hi: outside every lane's range
-                        take(ea, js);
-                        take(eb, js + 1);
-                        if (__any_sync(0xffffffffu, ea.near | eb.near)) {
-                            // rare path: queue the pairs near an edge for FP64 re-decision
-                            if (qn > kCfQueue - 64) {
-                                cf_drain(b, fcp, s1, s2, ctx, queue, qn, h, scratch);
-                                if (lane == 0) atomicAdd(&scratch->recheck_overflows, 1ull);
-                                qn = 0;
+                    auto sweep = [&](auto checked) {
+                        for (int js = g_lo; js < g_hi; js += 2) {
+                            PairEval ea, eb;
+                            eval(js, ea, checked);
+                            eval(js + 1, eb, checked);  // js + 1 = g_hi: outside every range
+                            take(ea, js);
+                            take(eb, js + 1);
+                            if (__any_sync(0xffffffffu, ea.near | eb.near)) {
+                                // rare path: queue the pairs near an edge for
+                                // FP64 re-decision
+                                if (qn > kCfQueue - 64) {
+                                    cf_drain(b, fcp, s1, s2, ctx, queue, qn, h, scratch);
+                                    if (lane == 0) atomicAdd(&scratch->recheck_overflows, 1ull);
+                                    qn = 0;
+                                }
+                                unsigned nmask = __ballot_sync(0xffffffffu, ea.near);
+                                if (ea.near)
+                                    queue[qn + __popc(nmask & lt_mask)] =
+                                        ((uint32_t)(js - joff) << 16) | (uint32_t)(js + jc);
+                                qn += __popc(nmask);
+                                nmask = __ballot_sync(0xffffffffu, eb.near);
+                                if (eb.near)
+                                    queue[qn + __popc(nmask & lt_mask)] =
+                                        ((uint32_t)(js + 1 - joff) << 16) | (uint32_t)(js + 1 + jc);
+                                qn += __popc(nmask);
                             }
-                            unsigned nmask = __ballot_sync(0xffffffffu, ea.near);
-                            if (ea.near)
-                                queue[qn + __popc(nmask & lt_mask)] =
-                                    ((uint32_t)ea.i << 16) | (uint32_t)(ea.i + d);
-                            qn += __popc(nmask);
-                            nmask = __ballot_sync(0xffffffffu, eb.near);
-                            if (eb.near)
-                                queue[qn + __popc(nmask & lt_mask)] =
-                                    ((uint32_t)eb.i << 16) | (uint32_t)(eb.i + d);
-                            qn += __popc(nmask);
                         }
-                    }
+                    };
+                    if (plain) sweep(std::false_type{});
+                    else sweep(std::true_type{});
                     store_runs(run_n > 0);
                     while (tail - head >= 32) {
                         apply_runs<true>(acc0, acc1, head, 32, h, hs);
@@ -734,7 +785,7 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
         if (tail != head) apply_runs<false>(acc0, acc1, head, tail - head, h, hs);
         __syncthreads();
         flush_rows(h, *fcp, out, row);
-        if (threadIdx.x == 0) atomicAdd(&scratch->work_items, 1ull);
+        if (threadIdx.x == 0 && slice == 0) atomicAdd(&scratch->work_items, 1ull);
     }
     if (lane == 0) atomicAdd(&scratch->visited_pairs, visited[warp]);
 }
@@ -778,7 +829,7 @@ __device__ __forceinline__ void xcf_drain(const Binning &b, const FastConst *__r
         const double w1 = fs.weights[ia], wq = objs.obj_weight[g];
         const float w12 = weight32(w1) * weight32(wq);
         // delta1[i] * weights1[i] * weights2[j] (py/picca/xcf.py:308)
-        const float2 dw = split2(fs.delta[ia] * w1 * wq);
+        const float2 dw = split_near(fs.delta[ia] * w1 * wq);
         const float pv = (float)(r_par * inv_p);
         const float tv = (float)(r_trans * inv_t);
         const float zs = (float)z1 + (float)zq;
@@ -867,8 +918,8 @@ __global__ void __launch_bounds__(kXcfBlock, 1) xcf_xi_fast_kernel(
             for (int e = threadIdx.x; e < kXcfBuckets; e += blockDim.x) buckets[e] = 0;
             __syncthreads();
             auto bucket_of = [&](int k) {
-                const double rq = objs.obj_r_comov[nbr_index[ctx.k0 + k]] - r_ref;
-                const int e = __float2int_rd((float)rq * (1.f / kXcfBucketMpc)) + kXcfBuckets / 2;
+                const float rq = f64_to_f32(objs.obj_r_comov[nbr_index[ctx.k0 + k]] - r_ref);
+                const int e = __float2int_rd(rq * (1.f / kXcfBucketMpc)) + kXcfBuckets / 2;
                 return e < 0 ? 0 : (e >= kXcfBuckets ? kXcfBuckets - 1 : e);
             };
             for (int k = threadIdx.x; k < nq; k += blockDim.x) atomicAdd(&buckets[bucket_of(k)], 1);
@@ -930,14 +981,14 @@ __global__ void __launch_bounds__(kXcfBlock, 1) xcf_xi_fast_kernel(
                     }
                     cp = (float)(chalf * inv_p);
                     st = (float)(shalf * inv_t);
-                    const double rho_d = objs.obj_r_comov[g] - r_ref;
-                    const float rho_q = (float)rho_d;
-                    nb = -__fmul_rn(cp, rho_q);
-                    nbl = (float)(-((double)cp * rho_d) - (double)nb);
-                    t = __fmaf_rn(st, (float)objs.obj_dist_m[g], -0.5f);
-                    zv = (float)objs.z_qso[g];
+                    const float2 rho_q = split_near(objs.obj_r_comov[g] - r_ref);
+                    nb = -__fmul_rn(cp, rho_q.x);
+                    nbl = __fmaf_rn(-cp, rho_q.y, -__fmaf_rn(cp, rho_q.x, nb));
+                    t = __fmaf_rn(st, f64_to_f32(objs.obj_dist_m[g]), -0.5f);
+                    zv = f64_to_f32(objs.z_qso[g]);
+                    const float2 wv = split_near(wq);
                     wvh = weight32(wq);
-                    wvl = (float)(wq - (double)wvh);
+                    wvl = wvh == wv.x ? wv.y : (float)(wq - (double)wvh);
                 }
             }
             // this lane's pixels [ia, ib): p and x_tr' are non-decreasing
@@ -1147,10 +1198,10 @@ int launch_cf_xi_fast(const Binning &b, double ang_max, const pg_forest_set &s1,
     // memory leaves room for
     int nwarps = kCfBlock / 32;
     if (tuning.warps > 0 && tuning.warps < nwarps) nwarps = tuning.warps;
-    while (nwarps > 1 && cf_smem(b.nbins, max_pix1, nwarps).total > 227 * 1024) --nwarps;
+    while (nwarps > 1 && cf_smem(b.nbins, max_pix1, nwarps).total > kMaxDynSmem) --nwarps;
     const int block = nwarps * 32;
     const size_t smem = cf_smem(b.nbins, max_pix1, nwarps).total;
-    if (smem > 227 * 1024) return PG_ERR_UNSUPPORTED;
+    if (smem > kMaxDynSmem) return PG_ERR_UNSUPPORTED;
     (void)ang_max;
     int rc = prepare_fast(b, fc, stream);
     if (rc) return rc;
@@ -1159,14 +1210,19 @@ int launch_cf_xi_fast(const Binning &b, double ang_max, const pg_forest_set &s1,
     const bool autoc = !b.x_correlation;
     const bool lowx = autoc && b.r_par_min == 0.0;
     int grid = 0;
+    // few forests: several CTAs share one, each with a slice of its
+    // neighbours, of at least two per warp (a slice costs a staging and a
+    // flush). 150 forests: 1.32 ms for the kernel with whole forests, 0.98 ms so;
+    // eight slices without that minimum left warps idle (1.85 ms)
+    int slices = 1;
+    while (slices < 4 && num_work * slices < 4 * (int64_t)num_sms) slices *= 2;
 #define PG_LAUNCH_CF(A, E, L, R)                                                               \
-    rc = persistent_grid(cf_xi_diag_kernel<A, E, L, R>, block, smem, num_sms, num_work, &grid, \
-                         tuning.blocks_per_sm);                                                \
+    rc = persistent_grid(cf_xi_diag_kernel<A, E, L, R>, block, smem, num_sms,                  \
+                         num_work * slices, &grid, tuning.blocks_per_sm);                      \
     if (rc) return rc;                                                                         \
-    cf_xi_diag_kernel<A, E, L, R><<<grid, block, smem, stream>>>(b, fc, s1, s2, nbr_offsets,   \
-                                                                 nbr_index, nbr_angle,         \
-                                                                 work_order, num_work, out,    \
-                                                                 scratch, max_pix1);
+    cf_xi_diag_kernel<A, E, L, R><<<grid, block, smem, stream>>>(                              \
+        b, fc, s1, s2, nbr_offsets, nbr_index, nbr_angle, work_order, num_work, slices, out,   \
+        scratch, max_pix1);
     if (b.rmu) {
         if (autoc && lowx) { PG_LAUNCH_CF(true, false, true, true) }
         else if (autoc) { PG_LAUNCH_CF(true, false, false, true) }
@@ -1195,10 +1251,10 @@ int launch_xcf_xi_fast(const Binning &b, double ang_max, const pg_forest_set &fo
     // memory leaves room for (histograms, forest, per-warp rings and queues)
     int nwarps = kXcfBlock / 32;
     if (tuning.warps > 0 && tuning.warps < nwarps) nwarps = tuning.warps;
-    while (nwarps > 1 && smem_layout(b.nbins, max_pix1, nwarps, true).total > 227 * 1024) --nwarps;
+    while (nwarps > 1 && smem_layout(b.nbins, max_pix1, nwarps, true).total > kMaxDynSmem) --nwarps;
     const int block = nwarps * 32;
     const size_t smem = smem_layout(b.nbins, max_pix1, nwarps, true).total;
-    if (smem > 227 * 1024) return PG_ERR_UNSUPPORTED;
+    if (smem > kMaxDynSmem) return PG_ERR_UNSUPPORTED;
     (void)ang_max;
     int rc = prepare_fast(b, fc, stream);
     if (rc) return rc;

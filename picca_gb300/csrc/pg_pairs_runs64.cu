@@ -460,7 +460,7 @@ int launch_runs64(const Binning &b, const pg_forest_set &s1, const pg_forest_set
 bool runs64_covers(const Binning &b, const pg_forest_set &s1, const pg_forest_set &s2,
                    int64_t num_work) {
     return !b.rmu && !b.ang_corr && s1.max_pixels <= 65535 && s2.max_pixels <= 65535 &&
-           r64_smem(s1.max_pixels).total <= 227 * 1024 && num_work < (INT32_MAX >> 5);
+           r64_smem(s1.max_pixels).total <= kMaxDynSmem && num_work < (INT32_MAX >> 5);
 }
 
 int launch_cf_xi_runs64(const Binning &b, const pg_forest_set &s1, const pg_forest_set &s2,

@@ -36,7 +36,7 @@ constexpr int kWsBlock = 256;
 constexpr int kWsLanes = 32;       // bins P of a row swept together, a lane each
 constexpr int kWsPitch = 33;       // doubles between the V of consecutive pixels
 constexpr unsigned kWsEnd = 0x80000000u;  // last segment of its bin
-constexpr size_t kWsMaxSmem = 227 * 1024;
+constexpr size_t kWsMaxSmem = kMaxDynSmem;
 constexpr uint64_t kWsBatchBytes = 256ull << 20;  // lists of a batch of pairs
 
 // The lists of one forest pair in the work buffer: nonempty-bin index (or
