@@ -112,6 +112,21 @@ def cubic_ppoly(x, y):
     return breaks, np.ascontiguousarray(pp.c[:, keep])
 
 
+def cubic_ppolys(x, ys):
+    """cubic_ppoly of several functions on the same points (the same bits):
+    breakpoints and one (4, m) coefficient array per function, from one
+    spline solve with a right-hand side each."""
+    splines = make_interp_spline(np.asarray(x, float),
+                                 np.stack([np.asarray(y, float) for y in ys], axis=1), k=3)
+    out = []
+    for k in range(len(ys)):
+        pp = PPoly.from_spline((splines.t, np.ascontiguousarray(splines.c[:, k]), 3))
+        out.append(pp.c)
+    keep = np.diff(pp.x) > 0
+    breaks = np.concatenate([pp.x[:-1][keep], [pp.x[1:][keep][-1]]])
+    return breaks, [np.ascontiguousarray(c[:, keep]) for c in out]
+
+
 def find_bins_log(values, grid):
     """find_bins_log (py/picca/delta_extraction/utils.py:163-186)."""
     step = grid[1] - grid[0]
@@ -197,6 +212,7 @@ class Dr16Gpu:
         self.history = []
         self.refined = []  # forests finished in two-float per counted mixed fit
         self._model_cache = {}
+        self._ppoly_cache = None
 
     # -- model -------------------------------------------------------------
     def _model_key(self, with_stack):
@@ -223,34 +239,35 @@ class Dr16Gpu:
         return model, keep
 
     def _build_model(self, with_stack=False):
-        dev = self.device
-        keep = {}
-        keep["mcx"] = torch.as_tensor(self.mean_cont_x, dtype=torch.float64).to(dev)
-        keep["mcy"] = torch.as_tensor(self.mean_cont_y, dtype=torch.float64).to(dev)
-        coefs = []
-        for vals in (self.eta, self.var_lss, self.fudge):
-            breaks, coef = cubic_ppoly(self.var_x, vals)
-            coefs.append(coef)
-        keep["brk"] = torch.as_tensor(breaks).to(dev)
-        keep["eta"] = torch.as_tensor(coefs[0]).to(dev)
-        keep["vlss"] = torch.as_tensor(coefs[1]).to(dev)
-        keep["fudge"] = torch.as_tensor(coefs[2]).to(dev)
+        # every table in one upload
+        key = (self.var_x.tobytes(), self.eta.tobytes(), self.var_lss.tobytes(),
+               self.fudge.tobytes())
+        if self._ppoly_cache is None or self._ppoly_cache[0] != key:
+            self._ppoly_cache = (key, cubic_ppolys(self.var_x, (self.eta, self.var_lss,
+                                                                self.fudge)))
+        breaks, coefs = self._ppoly_cache[1]
+        parts = {"mcx": self.mean_cont_x, "mcy": self.mean_cont_y, "brk": breaks,
+                 "eta": coefs[0], "vlss": coefs[1], "fudge": coefs[2]}
+        has_stack = with_stack and self.stack_x is not None
+        if has_stack:
+            parts.update(sx=self.stack_x, sy=self.stack_y)
+        flat = np.concatenate([np.asarray(v, dtype=np.float64).ravel() for v in parts.values()])
+        keep = {"tables": torch.from_numpy(flat).to(self.device)}
+        at, address = {}, keep["tables"].data_ptr()
+        for name, v in parts.items():
+            at[name] = address
+            address += 8 * np.size(v)
         rest = self.grid.log_lambda_rest_frame_grid
         model = ContModelC()
         model.num_mean_cont = len(self.mean_cont_x)
-        model.mean_cont_x = keep["mcx"].data_ptr()
-        model.mean_cont_y = keep["mcy"].data_ptr()
+        model.mean_cont_x, model.mean_cont_y = at["mcx"], at["mcy"]
         model.num_var_intervals = coefs[0].shape[1]
-        model.var_breaks = keep["brk"].data_ptr()
-        model.eta_coef = keep["eta"].data_ptr()
-        model.var_lss_coef = keep["vlss"].data_ptr()
-        model.fudge_coef = keep["fudge"].data_ptr()
-        if with_stack and self.stack_x is not None:
-            keep["sx"] = torch.as_tensor(self.stack_x).to(dev)
-            keep["sy"] = torch.as_tensor(self.stack_y).to(dev)
+        model.var_breaks = at["brk"]
+        model.eta_coef, model.var_lss_coef = at["eta"], at["vlss"]
+        model.fudge_coef = at["fudge"]
+        if has_stack:
             model.num_stack = len(self.stack_x)
-            model.stack_x = keep["sx"].data_ptr()
-            model.stack_y = keep["sy"].data_ptr()
+            model.stack_x, model.stack_y = at["sx"], at["sy"]
         model.log_lambda_rest_min = float(rest[0])
         model.log_lambda_rest_max = float(rest[-1])
         model.var_lss_mod = float(self.var_lss_mod)
@@ -334,10 +351,13 @@ class Dr16Gpu:
         grid = self.grid
         rest, obs = grid.log_lambda_rest_frame_grid, grid.log_lambda_grid
         nvar = self.num_bins_variance * NUM_VAR_BINS
-        bufs = {k: torch.zeros(n, dtype=torch.float64, device=dev) for k, n in (
-            ("mc_num", len(rest)), ("mc_w", len(rest)), ("v_mean", nvar), ("v_d2", nvar),
-            ("v_d4", nvar), ("v_np", nvar), ("v_nq", nvar), ("s_num", len(obs)),
-            ("s_w", len(obs)))}
+        # one buffer: cleared and read back in one piece
+        sizes = {"mc_num": len(rest), "mc_w": len(rest), "v_mean": nvar, "v_d2": nvar,
+                 "v_d4": nvar, "v_np": nvar, "v_nq": nvar, "s_num": len(obs), "s_w": len(obs)}
+        flat = torch.zeros(sum(sizes.values()), dtype=torch.float64, device=dev)
+        ends = np.cumsum(list(sizes.values()))
+        address = {k: flat.data_ptr() + 8 * int(end - n)
+                   for (k, n), end in zip(sizes.items(), ends)}
         st = ContStacksC()
         lin = getattr(grid, "wave_solution", "log") == "lin"
         st.wave_lin = int(lin)
@@ -351,21 +371,21 @@ class Dr16Gpu:
         st.rest_bins = len(rest)
         st.rest_grid0, st.rest_step = origin_step(rest)
         if mean_cont:
-            st.mean_cont_num = bufs["mc_num"].data_ptr()
-            st.mean_cont_weight = bufs["mc_w"].data_ptr()
+            st.mean_cont_num = address["mc_num"]
+            st.mean_cont_weight = address["mc_w"]
         st.var_lambda_bins = self.num_bins_variance
         st.var_grid0, st.var_step = origin_step(self.log_lambda_var_func_grid)
         if var_stats:
-            st.var_mean = bufs["v_mean"].data_ptr()
-            st.var_delta2 = bufs["v_d2"].data_ptr()
-            st.var_delta4 = bufs["v_d4"].data_ptr()
-            st.var_npix = bufs["v_np"].data_ptr()
-            st.var_nqso = bufs["v_nq"].data_ptr()
+            st.var_mean = address["v_mean"]
+            st.var_delta2 = address["v_d2"]
+            st.var_delta4 = address["v_d4"]
+            st.var_npix = address["v_np"]
+            st.var_nqso = address["v_nq"]
         st.obs_bins = len(obs)
         st.obs_grid0, st.obs_step = origin_step(obs)
         if delta_stack:
-            st.stack_num = bufs["s_num"].data_ptr()
-            st.stack_weight = bufs["s_w"].data_ptr()
+            st.stack_num = address["s_num"]
+            st.stack_weight = address["s_w"]
         model, keep = self._model()
         fit_c = fit["_keep"][2]
         with torch.cuda.device(dev):
@@ -376,7 +396,7 @@ class Dr16Gpu:
         if stats.status != 0:
             raise _native.NativeError(f"stack accumulation: device status {stats.status}")
         del keep
-        return {k: v.cpu().numpy() for k, v in bufs.items()}
+        return dict(zip(sizes, np.split(flat.cpu().numpy(), ends[:-1])))
 
     def update_mean_cont(self, sums):
         """_compute_mean_cont normalisation (expected_flux.py:291-308)."""
@@ -400,18 +420,19 @@ class Dr16Gpu:
         num_pixels, num_qso = stats["num_pixels"], stats["num_qso"]
         var_pipe_values = 10**(VAR_PIPE_MIN + ((np.arange(NUM_VAR_BINS) + .5) *
                                                (VAR_PIPE_MAX - VAR_PIPE_MIN) / NUM_VAR_BINS))
-        eta = interp1d(self.var_x, self.eta, kind="cubic", fill_value="extrapolate")(
-            self.log_lambda_var_func_grid)
-        vlss = interp1d(self.var_x, self.var_lss, kind="cubic", fill_value="extrapolate")(
-            self.log_lambda_var_func_grid)
-        fudge = interp1d(self.var_x, self.fudge, kind="cubic", fill_value="extrapolate")(
-            self.log_lambda_var_func_grid)
+
+        def start():
+            # the current functions on the grid (only bins without an exact
+            # solution start from them)
+            return np.stack([interp1d(self.var_x, y, kind="cubic", fill_value="extrapolate")(
+                self.log_lambda_var_func_grid) for y in
+                (self.eta, self.var_lss, self.fudge / FUDGE_REF)], axis=1)
+
         shape = (nvb, NUM_VAR_BINS)
         npix_bin = num_pixels.reshape(shape).sum(axis=1)
         sols, failed = fit_var_bins(
             var_delta.reshape(shape), var2_delta.reshape(shape), num_qso.reshape(shape),
-            var_pipe_values, self.min_num_qso_in_fit, self.limit_eta, self.limit_var_lss,
-            np.stack([eta, vlss, fudge / FUDGE_REF], axis=1))
+            var_pipe_values, self.min_num_qso_in_fit, self.limit_eta, self.limit_var_lss, start)
         eta, vlss, fudge = sols[:, 0].copy(), sols[:, 1].copy(), sols[:, 2].copy()
         eta[failed], vlss[failed], fudge[failed] = ETA_DEFAULT, VAR_LSS_DEFAULT, FUDGE_DEFAULT
         valid = ~failed
@@ -527,33 +548,38 @@ def box_lsq3_gram(gram, mty, limit_eta, limit_var_lss):
     nb = gram.shape[0]
     lo = np.array([limit_eta[0], limit_var_lss[0], 0.0])
     hi = np.array([limit_eta[1], limit_var_lss[1], np.inf])
-    best = np.zeros((nb, 3))
-    best_val = np.full(nb, np.inf)
+    faces = _faces(limit_eta, limit_var_lss)
+    x = np.empty((len(faces), nb, 3))
     ok = np.ones(nb, bool)
-    for face in _faces(limit_eta, limit_var_lss):
-        x = np.tile(np.array([0.0 if b is None else b for b in face]), (nb, 1))
-        free = [k for k in range(3) if face[k] is None]
-        feasible = np.ones(nb, bool)
-        if free:
-            fixed = [k for k in range(3) if face[k] is not None]
-            sub = gram[:, free][:, :, free]
-            eig = np.linalg.eigvalsh(sub)
-            # numpy.linalg.matrix_rank's tolerance on the (symmetric) Gram block
-            rank = (eig > eig.max(axis=1, keepdims=True) * len(free) *
-                    np.finfo(np.float64).eps).sum(axis=1)
-            ok &= rank == len(free)
-            r = mty[:, free]
-            if fixed:
-                r = r - np.einsum("bij,j->bi", gram[:, free][:, :, fixed], x[0, fixed])
-            safe = np.where((rank == len(free))[:, None, None], sub, np.eye(len(free)))
-            x[:, free] = np.linalg.solve(safe, r[..., None])[..., 0]
-            feasible = (np.all(x[:, free] >= lo[free] - 1e-15, axis=1) &
-                        np.all(x[:, free] <= hi[free] + 1e-15, axis=1))
-        val = np.einsum("bi,bij,bj->b", x, gram, x) - 2 * np.einsum("bi,bi->b", x, mty)
-        take = feasible & (val < best_val)
-        best[take] = x[take]
-        best_val[take] = val[take]
-    return best, ok
+    groups = {}  # faces with the same free variables share a factorisation
+    for k, face in enumerate(faces):
+        groups.setdefault(tuple(v is None for v in face), []).append(k)
+    for mask, members in groups.items():
+        free = [k for k in range(3) if mask[k]]
+        fixed = [k for k in range(3) if not mask[k]]
+        held = np.array([[faces[k][v] for v in fixed] for k in members])  # [faces, fixed]
+        x[np.ix_(members, range(nb), fixed)] = held[:, None, :]
+        if not free:
+            continue
+        sub = gram[:, free][:, :, free]
+        eig = np.linalg.eigvalsh(sub)
+        # numpy.linalg.matrix_rank's tolerance on the (symmetric) Gram block
+        full = (eig > eig.max(axis=1, keepdims=True) * len(free) *
+                np.finfo(np.float64).eps).sum(axis=1) == len(free)
+        ok &= full
+        r = np.repeat(mty[:, free, None], len(members), axis=2)  # [problem, free, face]
+        if fixed:
+            r = r - np.einsum("bij,kj->bik", gram[:, free][:, :, fixed], held)
+        safe = np.where(full[:, None, None], sub, np.eye(len(free)))
+        x[np.ix_(members, range(nb), free)] = np.linalg.solve(safe, r).transpose(2, 0, 1)
+    # a face's solution counts where its free variables are inside the box
+    # (the held ones sit on it)
+    inside = np.all((x >= lo - 1e-15) & (x <= hi + 1e-15), axis=2)
+    val = np.einsum("kbi,bij,kbj->kb", x, gram, x) - 2 * np.einsum("kbi,bi->kb", x, mty)
+    val = np.where(inside & ~np.isnan(val), val, np.inf)
+    best = np.argmin(val, axis=0)
+    found = val[best, np.arange(nb)] < np.inf
+    return np.where(found[:, None], x[best, np.arange(nb)], 0.0), ok
 
 
 def box_lsq3(mat, rhs, limit_eta, limit_var_lss):
@@ -566,8 +592,8 @@ def box_lsq3(mat, rhs, limit_eta, limit_var_lss):
 def fit_var_bins(var_delta, var2_delta, num_qso, var_pipe_values, min_num_qso, limit_eta,
                  limit_var_lss, start):
     """(eta, var_lss, fudge) of every wavelength bin at once (arrays
-    [bins, NUM_VAR_BINS]; start [bins, 3] with fudge / FUDGE_REF): the
-    batched form of fit_var_bin. Returns [bins, 3] (fudge in its own units)
+    [bins, NUM_VAR_BINS]; start [bins, 3] with fudge / FUDGE_REF, or a
+    function that returns it): the batched form of fit_var_bin. Returns [bins, 3] (fudge in its own units)
     and a mask of the bins whose fit failed."""
     sel = (num_qso > min_num_qso) & (var2_delta > 0)
     wsq = np.where(sel, 1.0 / np.where(sel, var2_delta, 1.0), 0.0)  # wgt^2
@@ -578,8 +604,12 @@ def fit_var_bins(var_delta, var2_delta, num_qso, var_pipe_values, min_num_qso, l
     x, ok = box_lsq3_gram(gram, mty, limit_eta, limit_var_lss)
     out = np.array(x)
     failed = np.zeros(len(out), bool)
-    for b in range(len(out)):
-        if not sel[b].any():
+    some = sel.any(axis=1)
+    todo = np.nonzero(~(some & ok))[0]
+    if todo.size and callable(start):
+        start = start()
+    for b in todo:
+        if not some[b]:
             # flat chi2: the minimiser stays at its starting point
             out[b] = start[b]
         elif not ok[b]:
