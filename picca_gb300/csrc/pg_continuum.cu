@@ -3,17 +3,16 @@
 // py/picca), the per-iteration histograms of Dr16ExpectedFlux and the final
 // delta extraction.
 //
-// One warp fits one forest: every lane holds up to K pixels in registers as
-// the coefficients of
+// One warp fits one forest with
 //     C = (a + b x) mc,      x = (L - Lmin)/(Lmax - Lmin),
 //     D = eta/ivar + var_lss C^2 + fudge ivar C^4,
 //     chi2 = sum (f - C)^2 / D + sum log D
-// (the reference's chi2 - sum log w with w = 1/D), evaluates chi2, its
-// gradient and Hessian in (a, b) in one pass, reduces them in FP64 with warp
-// shuffles and takes a damped Newton step solved in FP64 (backtracking
-// Armijo line search). The per-pixel terms are FP64 (PG_FIT_FP64) or FP32
-// (PG_FIT_MIXED); the reported chi2 is always re-evaluated in FP64.
-// The reference minimises the same function with iminuit's MIGRAD.
+// (the reference's chi2 - sum log w with w = 1/D): chi2, its gradient and
+// Hessian in (a, b) in one pass over the pixels, warp sums, damped Newton
+// steps (backtracking Armijo line search). The per-pixel terms are FP64
+// (cont_fit64_kernel, PG_FIT_FP64, and forests too long for the mixed form) or
+// FP32 (PG_FIT_MIXED). The reference minimises the same function with
+// iminuit's MIGRAD.
 #include <cuda_bf16.h>
 
 #include "pg_cont_common.cuh"
@@ -35,13 +34,15 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // scipy interp1d(kind="linear", fill_value="extrapolate"): searchsorted
-// (left) clipped to [1, n-1], then slope * (v - x_lo) + y_lo.
-__device__ double interp_linear(const double *__restrict__ x, const double *__restrict__ y, int n,
-                                double v) {
+// (left) clipped to [1, n-1], then slope * (v - x_lo) + y_lo. The search
+// compares keys that order like the doubles (integer pipe).
+__device__ __forceinline__ double interp_linear(const double *__restrict__ x,
+                                                const double *__restrict__ y, int n, double v) {
+    const unsigned long long key = order_key(v);
     int lo = 0, hi = n;
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        if (x[mid] < v) lo = mid + 1;
+        if (order_key(x[mid]) < key) lo = mid + 1;
         else hi = mid;
     }
     int idx = lo < 1 ? 1 : (lo > n - 1 ? n - 1 : lo);
@@ -50,18 +51,23 @@ __device__ double interp_linear(const double *__restrict__ x, const double *__re
     return __dadd_rn(__dmul_rn(slope, __dsub_rn(v, xl)), yl);
 }
 
-// Piecewise cubic (highest power first), extrapolated with the end pieces.
-__device__ double eval_ppoly(const double *__restrict__ brk, const double *__restrict__ coef, int m,
-                             double v) {
-    int lo = 0, hi = m + 1;  // searchsorted right over the m + 1 breakpoints
+// Piece of the variance functions that holds v (searchsorted right over the
+// m + 1 breakpoints, the end pieces extrapolated).
+__device__ __forceinline__ int ppoly_piece(const double *__restrict__ brk, int m, double v) {
+    const unsigned long long key = order_key(v);
+    int lo = 0, hi = m + 1;
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
-        if (brk[mid] <= v) lo = mid + 1;
+        if (order_key(brk[mid]) <= key) lo = mid + 1;
         else hi = mid;
     }
-    int i = lo - 1;
-    i = i < 0 ? 0 : (i > m - 1 ? m - 1 : i);
-    const double dx = v - brk[i];
+    const int i = lo - 1;
+    return i < 0 ? 0 : (i > m - 1 ? m - 1 : i);
+}
+
+// Cubic i of a coefficient array (highest power first) at dx.
+__device__ __forceinline__ double ppoly_at(const double *__restrict__ coef, int m, int i,
+                                           double dx) {
     return ((coef[i] * dx + coef[m + i]) * dx + coef[2 * m + i]) * dx + coef[3 * m + i];
 }
 
@@ -78,79 +84,228 @@ __device__ __forceinline__ ModelEval eval_model(const pg_cont_model &m, double l
         e.var_lss = 1.;
         e.fudge = 0.;
     } else {
-        e.eta = eval_ppoly(m.var_breaks, m.eta_coef, m.num_var_intervals, ll);
-        e.var_lss = eval_ppoly(m.var_breaks, m.var_lss_coef, m.num_var_intervals, ll);
-        e.fudge = eval_ppoly(m.var_breaks, m.fudge_coef, m.num_var_intervals, ll);
+        const int mi = m.num_var_intervals, i = ppoly_piece(m.var_breaks, mi, ll);
+        const double dx = ll - m.var_breaks[i];
+        e.eta = ppoly_at(m.eta_coef, mi, i, dx);
+        e.var_lss = ppoly_at(m.var_lss_coef, mi, i, dx);
+        e.fudge = ppoly_at(m.fudge_coef, mi, i, dx);
     }
     return e;
 }
 
-template <typename T>
-struct PixelTerms {
-    T ja[kContK], jb[kContK], f[kContK], q[kContK], vl[kContK], fi[kContK];
-    unsigned valid;
+// ---------------------------------------------------------------------------
+// The FP64 fit
+// ---------------------------------------------------------------------------
+// Bound: the FP64 pipe (16 cycles a warp operation and SM). The line search
+// near the optimum compares rounding noise, so the number of steps a forest
+// takes follows the last bit of every term: all of the below gives the bits of
+// the plain evaluation of the formulas.
+//  * The derivatives are summed as halves: scaling by a power of two commutes
+//    with rounding, and an addition of a scaled term is one FMA (exact
+//    product, one rounding). The terms of fudge are skipped where it is 0 for
+//    the whole forest (they add exact zeros).
+//  * A backtracking trial forms chi2 only, the derivatives when it is taken.
+//    The values at the last accepted point are those of the solution: no
+//    evaluation after the loop.
+//  * The six warp sums share the levels of one butterfly (8 additions instead
+//    of 30; a + b = b + a).
+//  * Searches compare integer keys; the mean continuum of a pixel is kept for
+//    the continuum that is written.
+//  * Pixel terms are in shared memory (slot k of lane l at k * 32 + l) rather
+//    than 224 registers a thread, two pixels are evaluated at a time, and warps
+//    draw forests from a counter.
+// 20,011 forests of 160 pixels: 7.7 ms with terms in registers and static
+// forests, 4.7 ms now; 5,000 forests of 600 pixels (a warp per 32 consecutive
+// forests before, 40 CTAs): 24.7 ms, 5.0 ms.
+constexpr int kLongK = 32;  // pixels per lane of the long form (up to 1,024)
+
+template <int K>
+constexpr int fit64_warps() { return K == kContK ? 16 : 4; }
+
+// One forest's terms: mc, x mc, flux, eta / ivar, var_lss, fudge ivar.
+struct FitTerms64 {
+    const double *ja, *jb, *f, *q, *vl, *fi;
 };
 
-// chi2 / 2 and its derivatives of one lane's pixels (accumulated in T,
-// returned in FP64); constant weights use q = 1, vl = fi = 0 with no log.
-// U is the arithmetic type of the per-pixel terms (T or FP64).
-template <typename U, typename T, typename O, typename A>
-__device__ __forceinline__ void lane_terms(const PixelTerms<T> &px, A a, A b, bool const_w,
-                                           O s[6]) {
-    U val = 0, ga = 0, gb = 0, haa = 0, hab = 0, hbb = 0;
-    const U ua = (U)a, ub = (U)b;
-#pragma unroll
-    for (int k = 0; k < kContK; ++k) {
-        if (!((px.valid >> k) & 1u)) continue;
-        const U ja = (U)px.ja[k], jb = (U)px.jb[k];
-        const U q = (U)px.q[k], vl = (U)px.vl[k], fi = (U)px.fi[k];
-        const U c = ua * ja + ub * jb;
-        const U c2 = c * c;
-        const U d = q + vl * c2 + fi * c2 * c2;
-        const U dd = (U)2 * vl * c + (U)4 * fi * c2 * c;
-        const U d2d = (U)2 * vl + (U)12 * fi * c2;
-        const U r = (U)px.f[k] - c;
-        const U id = (U)1 / d;
-        const U rid = r * id;
-        const U ddid = dd * id;
-        val += r * rid + (const_w ? (U)0 : log(d));
-        const U g = (U)-2 * rid - rid * rid * dd + ddid;
-        const U h = (U)2 * id + (U)4 * rid * ddid + (U)2 * rid * rid * dd * ddid - rid * rid * d2d
-                    + d2d * id - ddid * ddid;
-        ga += g * ja;
-        gb += g * jb;
-        haa += h * ja * ja;
-        hab += h * ja * jb;
-        hbb += h * jb * jb;
+struct PixelTerms64 {
+    double val, gh, hh;  // chi2 term, half derivatives in C
+};
+
+template <bool DERIVATIVES, bool FUDGE>
+__device__ __forceinline__ PixelTerms64 pixel_terms64(const FitTerms64 &t, int e, double a,
+                                                      double b, bool const_w) {
+    PixelTerms64 o;
+    const double c = a * t.ja[e] + b * t.jb[e];
+    const double c2 = c * c;
+    const double vl = t.vl[e];
+    double d = t.q[e] + vl * c2, fc = 0.;
+    if (FUDGE) {
+        fc = t.fi[e] * c2;
+        d = d + fc * c2;
     }
-    s[0] = (O)val; s[1] = (O)ga; s[2] = (O)gb;
-    s[3] = (O)haa; s[4] = (O)hab; s[5] = (O)hbb;
+    const double r = t.f[e] - c;
+    const double id = __drcp_rn(d);
+    const double rid = r * id;
+    o.val = r * rid + (const_w ? 0. : log(d));
+    if (DERIVATIVES) {
+        // hd = (dD/dC) / 2, h2 = (d2D/dC2) / 2
+        double hd = vl * c, h2 = vl;
+        if (FUDGE) {
+            hd = fma(2., fc * c, hd);
+            h2 = vl + (6. * t.fi[e]) * c2;
+        }
+        const double w = hd * id;
+        const double r2 = rid * rid;
+        const double p = r2 * hd;
+        o.gh = (-rid - p) + w;
+        double hh = fma(4., rid * w, id);
+        hh = fma(4., p * w, hh);
+        hh = hh - r2 * h2;
+        hh = hh + h2 * id;
+        o.hh = fma(-2., w * w, hh);
+    }
+    return o;
 }
 
-template <typename U, typename T>
-__device__ __forceinline__ void eval_all(const PixelTerms<T> &px, double a, double b, bool const_w,
-                                         double s[6]) {
-    lane_terms<U, T, double, double>(px, a, b, const_w, s);
+// Sums of one lane's pixels: chi2 and the half derivatives.
+template <bool DERIVATIVES, bool FUDGE>
+__device__ __forceinline__ void lane_sums64(const FitTerms64 &t, unsigned valid, int nk, double a,
+                                            double b, bool const_w, double s[6]) {
+    const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) s[k] = warp_sum(s[k]);
+    for (int q = 0; q < 6; ++q) s[q] = 0.;
+    auto add = [&](const PixelTerms64 &o, int e) {
+        s[0] += o.val;
+        if (DERIVATIVES) {
+            const double ja = t.ja[e], jb = t.jb[e];
+            s[1] += o.gh * ja;
+            s[2] += o.gh * jb;
+            const double ha = o.hh * ja;
+            s[3] += ha * ja;
+            s[4] += ha * jb;
+            s[5] += (o.hh * jb) * jb;
+        }
+    };
+    int k = 0;
+#pragma unroll 1
+    for (; k + 1 < nk; k += 2) {
+        const int e = k * 32 + lane;
+        const PixelTerms64 o0 = pixel_terms64<DERIVATIVES, FUDGE>(t, e, a, b, const_w);
+        const PixelTerms64 o1 = pixel_terms64<DERIVATIVES, FUDGE>(t, e + 32, a, b, const_w);
+        if ((valid >> k) & 1u) add(o0, e);
+        if ((valid >> k) & 2u) add(o1, e + 32);
+    }
+    if (k < nk && ((valid >> k) & 1u)) {
+        const int e = k * 32 + lane;
+        add(pixel_terms64<DERIVATIVES, FUDGE>(t, e, a, b, const_w), e);
+    }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kContBlock) cont_fit_kernel(
+// warp_sum of six values, in every lane: level by level of the same
+// butterfly, each lane carrying only the values it is to deliver.
+__device__ __forceinline__ void warp_sum6(double s[6]) {
+    const int lane = threadIdx.x & 31;
+    const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
+    double v[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        const double keep = b4 ? s[q + 3] : s[q], give = b4 ? s[q] : s[q + 3];
+        v[q] = keep + __shfl_xor_sync(0xffffffffu, give, 16);
+    }
+    // lanes without bit 3: v[0], v[1]; with it: v[2]
+    const double k0 = b3 ? v[2] : v[0], g0 = b3 ? v[0] : v[2];
+    double u0 = k0 + __shfl_xor_sync(0xffffffffu, g0, 8);
+    const double u1 = v[1] + __shfl_xor_sync(0xffffffffu, v[1], 8);
+    // lanes with bit 2 deliver v[1] (of the lanes without bit 3)
+    const double k1 = b2 && !b3 ? u1 : u0, g1 = b2 ? u0 : (b3 ? u0 : u1);
+    u0 = k1 + __shfl_xor_sync(0xffffffffu, g1, 4);
+    u0 += __shfl_xor_sync(0xffffffffu, u0, 2);
+    u0 += __shfl_xor_sync(0xffffffffu, u0, 1);
+#pragma unroll
+    for (int q = 0; q < 6; ++q)
+        s[q] = __shfl_sync(0xffffffffu, u0, (q >= 3 ? 16 : 0) + (q % 3 == 2 ? 8 : 0) +
+                                                (q % 3 == 1 ? 4 : 0));
+}
+
+template <bool DERIVATIVES>
+__device__ __noinline__ void fit_sums64(const FitTerms64 &t, unsigned valid, int nk, double a,
+                                        double b, bool const_w, bool fudge, double s[6]) {
+    if (fudge) lane_sums64<DERIVATIVES, true>(t, valid, nk, a, b, const_w, s);
+    else lane_sums64<DERIVATIVES, false>(t, valid, nk, a, b, const_w, s);
+    if (!DERIVATIVES) {
+        s[0] = warp_sum(s[0]);
+        return;
+    }
+    warp_sum6(s);
+#pragma unroll
+    for (int q = 1; q < 6; ++q) s[q] *= 2.;
+}
+
+// Forests of at most 32 * kContK pixels (K = kContK; a warp draws `group`
+// forests at a time) or of more, up to 32 * K (K = kLongK; draws
+// of half a warp's share of what is left, down to one forest, whose lengths are
+// looked at 32 at a time: a set without long forests is passed over in some
+// thousand draws, and long ones are shared out singly at the end).
+template <int K>
+__global__ void __launch_bounds__(fit64_warps<K>() * 32) cont_fit64_kernel(
     const __grid_constant__ pg_spectra sp, const __grid_constant__ pg_cont_model m,
     const double *__restrict__ start, const int32_t *__restrict__ index, int64_t count,
-    int max_iter, double tol, const __grid_constant__ pg_cont_fit out, Scratch *scratch) {
+    int max_iter, double tol, const __grid_constant__ pg_cont_fit out, int32_t *counter,
+    int group, Scratch *scratch) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int S = 32 * K;
     const int lane = threadIdx.x & 31;
-    const int64_t warp_global = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    double *slab = reinterpret_cast<double *>(smem) + (size_t)(threadIdx.x >> 5) * 6 * S;
+    const FitTerms64 t = {slab, slab + S, slab + 2 * S, slab + 3 * S, slab + 4 * S, slab + 5 * S};
     const bool const_w = m.use_constant_weight != 0;
-    for (int64_t w = warp_global; w < count; w += nwarps) {
+    const int nwarps = gridDim.x * (blockDim.x >> 5);
+    int64_t w_next = 0, w_end = 0;
+    unsigned todo = 0;
+    for (;;) {
+        int64_t w;
+        if (K == kContK) {
+            if (w_next == w_end) {
+                int g = 0;
+                if (lane == 0) g = atomicAdd(counter, 1);
+                w_next = (int64_t)__shfl_sync(0xffffffffu, g, 0) * group;
+                if (w_next >= count) break;
+                w_end = min(count, w_next + group);
+            }
+            w = w_next++;
+        } else {
+            while (!todo) {
+                if (w_next >= w_end) {
+                    int t = 0;
+                    if (lane == 0) t = atomicAdd(counter, 1);
+                    t = __shfl_sync(0xffffffffu, t, 0);
+                    unsigned left = (unsigned)count, size = max(1u, left / (2u * nwarps));
+                    for (; t >= nwarps && left > size * nwarps; t -= nwarps) {
+                        left -= size * nwarps;
+                        size = max(1u, left / (2u * nwarps));
+                    }
+                    w_next = count - left + (int64_t)t * size;
+                    if (w_next >= count) break;
+                    w_end = min(count, w_next + size);
+                }
+                bool is_long = false;
+                if (w_next + lane < w_end) {
+                    const int64_t g = index ? (int64_t)index[w_next + lane] : w_next + lane;
+                    is_long = sp.pix_offset[g + 1] - sp.pix_offset[g] > 32 * kContK;
+                }
+                todo = __ballot_sync(0xffffffffu, is_long);
+                w_next += 32;
+            }
+            if (!todo) break;
+            w = w_next - 32 + (__ffs(todo) - 1);
+            todo &= todo - 1;
+        }
         const int64_t f = index ? (int64_t)index[w] : w;
         const int64_t off = sp.pix_offset[f];
         const int64_t n64 = sp.pix_offset[f + 1] - off;
-        if (n64 > 32 * kContK) continue;  // a long forest: cont_fit_long_kernel
-        if (n64 <= 0) {
+        if (K == kContK && n64 > S) continue;  // the other form's forest
+        if (n64 <= 0 || n64 > S) {
             if (lane == 0) {
+                if (n64 > 0) report_error(scratch, PG_ERR_UNSUPPORTED, (int32_t)f);
                 out.zero_point[f] = NAN;
                 out.slope[f] = NAN;
                 out.chi2[f] = NAN;
@@ -161,59 +316,63 @@ __global__ void __launch_bounds__(kContBlock) cont_fit_kernel(
             continue;
         }
         const int n = (int)n64;
+        const int nk = (n + 31) >> 5;
         const double zp1 = log10(1 + sp.z_qso[f]);
         const double ll_min = m.log_lambda_rest_min + zp1;
         const double ll_max = m.log_lambda_rest_max + zp1;
-        PixelTerms<T> px;
-        px.valid = 0;
+        unsigned valid = 0;
+        bool fudge = false;
         double sfi = 0., si = 0.;
-#pragma unroll
-        for (int k = 0; k < kContK; ++k) {
-            const int p = lane + 32 * k;
-            px.ja[k] = px.jb[k] = px.f[k] = px.q[k] = px.vl[k] = px.fi[k] = (T)0;
+        __syncwarp();
+        for (int k = 0; k < nk; ++k) {
+            const int p = lane + 32 * k, e = k * 32 + lane;
+            double ja = 0., jb = 0., fl = 0., q = 1., vl = 0., fi = 0.;
             if (p < n) {
-                const double ll = sp.log_lambda[off + p], fl = sp.flux[off + p];
+                const double ll = sp.log_lambda[off + p];
                 const double iv = sp.ivar[off + p];
+                fl = sp.flux[off + p];
                 sfi += fl * iv;
                 si += iv;
                 if (iv > 0) {
-                    const ModelEval e = eval_model(m, ll, zp1, sp.transmission_correction[off + p]);
+                    const ModelEval ev = eval_model(m, ll, zp1, sp.transmission_correction[off + p]);
                     const double x = (ll - ll_min) / (ll_max - ll_min);
-                    px.ja[k] = (T)e.mc;
-                    px.jb[k] = (T)(x * e.mc);
-                    px.f[k] = (T)fl;
-                    px.q[k] = (T)(const_w ? 1. : e.eta / iv);
-                    px.vl[k] = (T)(const_w ? 0. : e.var_lss);
-                    px.fi[k] = (T)(const_w ? 0. : e.fudge * iv);
-                    px.valid |= 1u << k;
+                    ja = ev.mc;
+                    jb = x * ev.mc;
+                    if (!const_w) {
+                        q = ev.eta / iv;
+                        vl = ev.var_lss;
+                        fi = ev.fudge * iv;
+                    }
+                    valid |= 1u << k;
+                    fudge |= fi != 0.;
                 }
             }
+            slab[e] = ja; slab[S + e] = jb; slab[2 * S + e] = fl;
+            slab[3 * S + e] = q; slab[4 * S + e] = vl; slab[5 * S + e] = fi;
         }
+        fudge = __any_sync(0xffffffffu, fudge);
         sfi = warp_sum(sfi);
         si = warp_sum(si);
         const double a0 = sfi / si;  // utils.py:92
         // ndata: pixels with a positive weight at the reference's starting
         // point (a0, 0) (cont_model.py:88-92)
         int nd = 0;
-#pragma unroll
-        for (int k = 0; k < kContK; ++k) {
-            if ((px.valid >> k) & 1u) {
-                const double c = a0 * (double)px.ja[k];
-                const double d = (double)px.q[k] + (double)px.vl[k] * c * c +
-                                 (double)px.fi[k] * c * c * c * c;
+        for (int k = 0; k < nk; ++k) {
+            if ((valid >> k) & 1u) {
+                const int e = k * 32 + lane;
+                const double c = a0 * t.ja[e];
+                const double d = t.q[e] + t.vl[e] * c * c + t.fi[e] * c * c * c * c;
                 nd += (d > 0.) ? 1 : 0;
             }
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) nd += __shfl_xor_sync(0xffffffffu, nd, o);
+        nd = __reduce_add_sync(0xffffffffu, nd);
         double a = a0, b = 0.;
         if (start) {
             a = start[2 * f];
             b = m.order == 0 ? 0. : start[2 * f + 1];
         }
-
         double s[6];
-        eval_all<T>(px, a, b, const_w, s);
+        fit_sums64<true>(t, valid, nk, a, b, const_w, fudge, s);
         int it = 0;
         // max_iter == 0 with a start: evaluate the model at the given (a, b)
         bool converged = max_iter == 0 && start != nullptr;
@@ -239,41 +398,46 @@ __global__ void __launch_bounds__(kContBlock) cont_fit_kernel(
                 }
             }
             const double slope_dir = da * s[1] + db * s[2];
-            double t = 1.;
+            double step = 1.;
             double trial[6];
             bool accepted = false;
             for (int ls = 0; ls < 40; ++ls) {
-                eval_all<T>(px, a + t * da, b + t * db, const_w, trial);
-                if (isfinite(trial[0]) && trial[0] <= s[0] + 1e-4 * t * slope_dir) {
+                const double at = a + step * da, bt = b + step * db;
+                if (ls == 0) fit_sums64<true>(t, valid, nk, at, bt, const_w, fudge, trial);
+                else fit_sums64<false>(t, valid, nk, at, bt, const_w, fudge, trial);
+                if (isfinite(trial[0]) && trial[0] <= s[0] + 1e-4 * step * slope_dir) {
+                    if (ls > 0) fit_sums64<true>(t, valid, nk, at, bt, const_w, fudge, trial);
                     accepted = true;
                     break;
                 }
-                t *= 0.5;
+                step *= 0.5;
             }
             if (!accepted) {
                 converged = fabs(s[1]) + fabs(s[2]) < 1e-6 * fmax(1., fabs(s[0]));
                 break;
             }
-            a += t * da;
-            b += t * db;
+            a += step * da;
+            b += step * db;
 #pragma unroll
             for (int k = 0; k < 6; ++k) s[k] = trial[k];
-            if (fabs(t * da) < tol * fmax(1., fmax(fabs(a), fabs(b))) &&
-                fabs(t * db) < tol * fmax(1., fmax(fabs(a), fabs(b)))) {
+            if (fabs(step * da) < tol * fmax(1., fmax(fabs(a), fabs(b))) &&
+                fabs(step * db) < tol * fmax(1., fmax(fabs(a), fabs(b)))) {
                 converged = true;
                 ++it;
                 break;
             }
         }
-        // chi2 at the solution in FP64, and the continuum with the
-        // reference's operation order (cont_model.py:138-144)
-        double fin[6];
-        eval_all<double>(px, a, b, const_w, fin);
+        // the continuum with the reference's operation order
+        // (cont_model.py:138-144); s holds chi2 at (a, b)
         bool negative = false, all_zero = true;
-        for (int p = lane; p < n; p += 32) {
+        for (int k = 0; k < nk; ++k) {
+            const int p = lane + 32 * k;
+            if (p >= n) continue;
             const double ll = sp.log_lambda[off + p];
-            const double mc = interp_linear(m.mean_cont_x, m.mean_cont_y, m.num_mean_cont,
-                                            ll - zp1) * sp.transmission_correction[off + p];
+            const double mc = ((valid >> k) & 1u)
+                                  ? t.ja[k * 32 + lane]
+                                  : interp_linear(m.mean_cont_x, m.mean_cont_y, m.num_mean_cont,
+                                                  ll - zp1) * sp.transmission_correction[off + p];
             const double line = b * (ll - ll_min) / (ll_max - ll_min) + a;
             const double c = line * mc;
             if (out.continuum) out.continuum[off + p] = c;
@@ -288,7 +452,7 @@ __global__ void __launch_bounds__(kContBlock) cont_fit_kernel(
             if (all_zero) status = 3;
             out.zero_point[f] = status == 0 ? a : NAN;
             out.slope[f] = status == 0 ? b : NAN;
-            out.chi2[f] = status == 0 ? fin[0] : NAN;
+            out.chi2[f] = status == 0 ? s[0] : NAN;
             out.ndata[f] = nd;
             out.status[f] = status;
             out.iterations[f] = it;
@@ -296,223 +460,25 @@ __global__ void __launch_bounds__(kContBlock) cont_fit_kernel(
     }
 }
 
-// ---------------------------------------------------------------------------
-// Long forests (more than 32 * kContK pixels, up to 32 * kLongK: the linear
-// 0.8 Angstrom grid reaches about 1,000 pixels). Same fit as cont_fit_kernel
-// in FP64 (damped Newton with Armijo backtracking, the same status codes),
-// with the per-pixel terms in the warp's shared-memory slab instead of
-// registers: term t of pixel k*32 + lane at slab[t * 32 * kLongK + k * 32 +
-// lane] (consecutive lanes, consecutive banks). Forests of at most
-// 32 * kContK pixels are left to the register kernels.
-// ---------------------------------------------------------------------------
-constexpr int kLongK = 32;
-constexpr int kLongWarps = 4;  // 4 x 48 KB slabs per block
-
-__device__ __forceinline__ void long_terms(const double *slab, unsigned valid, int nk, double a,
-                                           double b, bool const_w, double s[6]) {
-    const int lane = threadIdx.x & 31;
-    double val = 0, ga = 0, gb = 0, haa = 0, hab = 0, hbb = 0;
-    constexpr int S = 32 * kLongK;
-    for (int k = 0; k < nk; ++k) {
-        if (!((valid >> k) & 1u)) continue;
-        const int e = k * 32 + lane;
-        const double ja = slab[e], jb = slab[S + e], fl = slab[2 * S + e];
-        const double q = slab[3 * S + e], vl = slab[4 * S + e], fi = slab[5 * S + e];
-        const double c = a * ja + b * jb;
-        const double c2 = c * c;
-        const double d = q + vl * c2 + fi * c2 * c2;
-        const double dd = 2. * vl * c + 4. * fi * c2 * c;
-        const double d2d = 2. * vl + 12. * fi * c2;
-        const double r = fl - c;
-        const double id = 1. / d;
-        const double rid = r * id;
-        const double ddid = dd * id;
-        val += r * rid + (const_w ? 0. : log(d));
-        const double g = -2. * rid - rid * rid * dd + ddid;
-        const double h = 2. * id + 4. * rid * ddid + 2. * rid * rid * dd * ddid - rid * rid * d2d +
-                         d2d * id - ddid * ddid;
-        ga += g * ja;
-        gb += g * jb;
-        haa += h * ja * ja;
-        hab += h * ja * jb;
-        hbb += h * jb * jb;
-    }
-    s[0] = warp_sum(val); s[1] = warp_sum(ga); s[2] = warp_sum(gb);
-    s[3] = warp_sum(haa); s[4] = warp_sum(hab); s[5] = warp_sum(hbb);
-}
-
-__global__ void __launch_bounds__(32 * kLongWarps) cont_fit_long_kernel(
-    const __grid_constant__ pg_spectra sp, const __grid_constant__ pg_cont_model m,
-    const double *__restrict__ start, const int32_t *__restrict__ index, int64_t count,
-    int max_iter, double tol, const __grid_constant__ pg_cont_fit out, Scratch *scratch) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int lane = threadIdx.x & 31;
-    double *slab = reinterpret_cast<double *>(smem) + (size_t)(threadIdx.x >> 5) * 6 * 32 * kLongK;
-    constexpr int S = 32 * kLongK;
-    const int64_t warp_global = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const bool const_w = m.use_constant_weight != 0;
-    // lanes test 32 forests at a time; the warp fits the long ones among them
-    for (int64_t base = warp_global * 32; base < count; base += nwarps * 32) {
-        int64_t lane_f = -1;
-        bool is_long = false;
-        if (base + lane < count) {
-            lane_f = index ? (int64_t)index[base + lane] : base + lane;
-            is_long = sp.pix_offset[lane_f + 1] - sp.pix_offset[lane_f] > 32 * kContK;
-        }
-        unsigned todo = __ballot_sync(0xffffffffu, is_long);
-        while (todo) {
-            const int src = __ffs(todo) - 1;
-            todo &= todo - 1;
-            const int64_t f = __shfl_sync(0xffffffffu, lane_f, src);
-            const int64_t off = sp.pix_offset[f];
-            const int64_t n64 = sp.pix_offset[f + 1] - off;
-            if (n64 <= 32 * kContK) continue;  // the register kernels' forests
-            if (n64 > 32 * kLongK) {
-                if (lane == 0) {
-                    report_error(scratch, PG_ERR_UNSUPPORTED, (int32_t)f);
-                    out.zero_point[f] = NAN;
-                    out.slope[f] = NAN;
-                    out.chi2[f] = NAN;
-                    out.ndata[f] = 0;
-                    out.status[f] = 1;
-                    out.iterations[f] = 0;
-                }
-                continue;
-            }
-            const int n = (int)n64;
-            const int nk = (n + 31) / 32;
-            const double zp1 = log10(1 + sp.z_qso[f]);
-            const double ll_min = m.log_lambda_rest_min + zp1;
-            const double ll_max = m.log_lambda_rest_max + zp1;
-            unsigned valid = 0;
-            double sfi = 0., si = 0.;
-            __syncwarp();
-            for (int k = 0; k < nk; ++k) {
-                const int p = lane + 32 * k;
-                const int e = k * 32 + lane;
-                double ja = 0, jb = 0, fl = 0, q = 0, vl = 0, fi = 0;
-                if (p < n) {
-                    const double ll = sp.log_lambda[off + p];
-                    fl = sp.flux[off + p];
-                    const double iv = sp.ivar[off + p];
-                    sfi += fl * iv;
-                    si += iv;
-                    if (iv > 0) {
-                        const ModelEval ev = eval_model(m, ll, zp1, sp.transmission_correction[off + p]);
-                        const double x = (ll - ll_min) / (ll_max - ll_min);
-                        ja = ev.mc;
-                        jb = x * ev.mc;
-                        q = const_w ? 1. : ev.eta / iv;
-                        vl = const_w ? 0. : ev.var_lss;
-                        fi = const_w ? 0. : ev.fudge * iv;
-                        valid |= 1u << k;
-                    }
-                }
-                slab[e] = ja; slab[S + e] = jb; slab[2 * S + e] = fl;
-                slab[3 * S + e] = q; slab[4 * S + e] = vl; slab[5 * S + e] = fi;
-            }
-            __syncwarp();
-            sfi = warp_sum(sfi);
-            si = warp_sum(si);
-            const double a0 = sfi / si;  // utils.py:92
-            int nd = 0;
-            for (int k = 0; k < nk; ++k) {
-                if ((valid >> k) & 1u) {
-                    const int e = k * 32 + lane;
-                    const double c = a0 * slab[e];
-                    const double d = slab[3 * S + e] + slab[4 * S + e] * c * c +
-                                     slab[5 * S + e] * c * c * c * c;
-                    nd += (d > 0.) ? 1 : 0;
-                }
-            }
-    #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) nd += __shfl_xor_sync(0xffffffffu, nd, o);
-            double a = a0, b = 0.;
-            if (start) {
-                a = start[2 * f];
-                b = m.order == 0 ? 0. : start[2 * f + 1];
-            }
-            double s[6];
-            long_terms(slab, valid, nk, a, b, const_w, s);
-            int it = 0;
-            bool converged = max_iter == 0 && start != nullptr;
-            for (; it < max_iter; ++it) {
-                double da, db;
-                if (m.order == 0) {
-                    da = s[3] > 0 ? -s[1] / s[3] : -s[1];
-                    db = 0.;
-                } else {
-                    const double det = s[3] * s[5] - s[4] * s[4];
-                    if (det > 0 && s[3] > 0) {
-                        da = -(s[5] * s[1] - s[4] * s[2]) / det;
-                        db = -(s[3] * s[2] - s[4] * s[1]) / det;
-                    } else {
-                        const double scale = fmax(fabs(s[3]), fabs(s[5]));
-                        da = -s[1] / (scale > 0 ? scale : 1.);
-                        db = -s[2] / (scale > 0 ? scale : 1.);
-                    }
-                    if (da * s[1] + db * s[2] >= 0) {  // not a descent direction
-                        const double scale = fmax(fabs(s[3]), fabs(s[5]));
-                        da = -s[1] / (scale > 0 ? scale : 1.);
-                        db = -s[2] / (scale > 0 ? scale : 1.);
-                    }
-                }
-                const double slope_dir = da * s[1] + db * s[2];
-                double t = 1.;
-                double trial[6];
-                bool accepted = false;
-                for (int ls = 0; ls < 40; ++ls) {
-                    long_terms(slab, valid, nk, a + t * da, b + t * db, const_w, trial);
-                    if (isfinite(trial[0]) && trial[0] <= s[0] + 1e-4 * t * slope_dir) {
-                        accepted = true;
-                        break;
-                    }
-                    t *= 0.5;
-                }
-                if (!accepted) {
-                    converged = fabs(s[1]) + fabs(s[2]) < 1e-6 * fmax(1., fabs(s[0]));
-                    break;
-                }
-                a += t * da;
-                b += t * db;
-    #pragma unroll
-                for (int k = 0; k < 6; ++k) s[k] = trial[k];
-                if (fabs(t * da) < tol * fmax(1., fmax(fabs(a), fabs(b))) &&
-                    fabs(t * db) < tol * fmax(1., fmax(fabs(a), fabs(b)))) {
-                    converged = true;
-                    ++it;
-                    break;
-                }
-            }
-            double fin[6];
-            long_terms(slab, valid, nk, a, b, const_w, fin);
-            bool negative = false, all_zero = true;
-            for (int p = lane; p < n; p += 32) {
-                const double ll = sp.log_lambda[off + p];
-                const double mc = interp_linear(m.mean_cont_x, m.mean_cont_y, m.num_mean_cont,
-                                                ll - zp1) * sp.transmission_correction[off + p];
-                const double line = b * (ll - ll_min) / (ll_max - ll_min) + a;
-                const double c = line * mc;
-                if (out.continuum) out.continuum[off + p] = c;
-                negative |= c < 0;
-                all_zero &= c == 0;
-            }
-            negative = __any_sync(0xffffffffu, negative);
-            all_zero = __all_sync(0xffffffffu, all_zero);
-            if (lane == 0) {
-                int status = converged ? 0 : 1;
-                if (negative) status = 2;
-                if (all_zero) status = 3;
-                out.zero_point[f] = status == 0 ? a : NAN;
-                out.slope[f] = status == 0 ? b : NAN;
-                out.chi2[f] = status == 0 ? fin[0] : NAN;
-                out.ndata[f] = nd;
-                out.status[f] = status;
-                out.iterations[f] = it;
-            }
-        }
-    }
+template <int K>
+int launch_fit64(const pg_spectra &sp, const pg_cont_model &m, const double *start,
+                 const int32_t *index, int64_t count, int max_iter, double tol,
+                 const pg_cont_fit &out, int32_t *counter, Scratch *scratch, int num_sms,
+                 cudaStream_t stream) {
+    constexpr int warps = fit64_warps<K>();
+    const size_t smem = (size_t)warps * 6 * 32 * K * sizeof(double);
+    cudaError_t err = cudaFuncSetAttribute(
+        cont_fit64_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess) return check_cuda(err);
+    int64_t blocks = (count + warps - 1) / warps;
+    if (blocks > num_sms) blocks = num_sms;
+    // forests drawn one at a time, several where there are many (a draw by
+    // every warp for each of them would queue at the counter)
+    int64_t group = count / (blocks * warps * 16);
+    group = group < 1 ? 1 : (group > 32 ? 32 : group);
+    cont_fit64_kernel<K><<<(unsigned)blocks, warps * 32, smem, stream>>>(
+        sp, m, start, index, count, max_iter, tol, out, counter, (int)group, scratch);
+    return check_cuda(cudaGetLastError());
 }
 
 // ---------------------------------------------------------------------------
@@ -685,7 +651,7 @@ __global__ void __launch_bounds__(kContBlock, 4) cont_fit_mixed_kernel(
             if (f < 0) break;
             const int64_t off = slots[j].off;
             const int n = slots[j].n;
-            if (n > 32 * kContK) continue;  // a long forest: cont_fit_long_kernel
+            if (n > 32 * kContK) continue;  // a long forest: cont_fit64_kernel<kLongK>
             if (lane == j) slots[j].write = 1;
             if (n <= 0) continue;           // empty: the defaults (status 1, NaN)
             const float lmh = slots[j].lm_hi;
@@ -989,27 +955,14 @@ __device__ __forceinline__ int64_t find_bin(double x, double grid0, double step,
     return (int64_t)((x - grid0) / step + 0.5);
 }
 
-// eta, var_lss and fudge at v in FP64 from the model's coefficient arrays:
-// one search (searchsorted right, the end pieces extrapolated) and the three
-// cubics as eval_ppoly evaluates them.
+// eta, var_lss and fudge at v in FP64 from the model's coefficient arrays.
 __device__ void var_funcs_f64(const pg_cont_model &m, double v, double &eta, double &vlss,
                               double &fudge) {
-    const int mi = m.num_var_intervals;
-    int lo = 0, hi = mi + 1;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (m.var_breaks[mid] <= v) lo = mid + 1;
-        else hi = mid;
-    }
-    int i = lo - 1;
-    i = i < 0 ? 0 : (i > mi - 1 ? mi - 1 : i);
+    const int mi = m.num_var_intervals, i = ppoly_piece(m.var_breaks, mi, v);
     const double dx = v - m.var_breaks[i];
-    const double *c = m.eta_coef;
-    eta = ((c[i] * dx + c[mi + i]) * dx + c[2 * mi + i]) * dx + c[3 * mi + i];
-    c = m.var_lss_coef;
-    vlss = ((c[i] * dx + c[mi + i]) * dx + c[2 * mi + i]) * dx + c[3 * mi + i];
-    c = m.fudge_coef;
-    fudge = ((c[i] * dx + c[mi + i]) * dx + c[2 * mi + i]) * dx + c[3 * mi + i];
+    eta = ppoly_at(m.eta_coef, mi, i, dx);
+    vlss = ppoly_at(m.var_lss_coef, mi, i, dx);
+    fudge = ppoly_at(m.fudge_coef, mi, i, dx);
 }
 
 // ---- two-float (double-float) arithmetic -----------------------------------
@@ -1715,13 +1668,9 @@ __global__ void __launch_bounds__(kContBlock) cont_deltas_kernel(
                         int i = count_keys<true>(brk, mi + 1, key) - 1;
                         i = i < 0 ? 0 : (i > mi - 1 ? mi - 1 : i);
                         const double dx = ll - m.var_breaks[i];
-                        const double *c = m.eta_coef;
-                        eta = ((c[i] * dx + c[mi + i]) * dx + c[2 * mi + i]) * dx + c[3 * mi + i];
-                        c = m.var_lss_coef;
-                        vlss = ((c[i] * dx + c[mi + i]) * dx + c[2 * mi + i]) * dx + c[3 * mi + i];
-                        c = m.fudge_coef;
-                        fudge = ((c[i] * dx + c[mi + i]) * dx + c[2 * mi + i]) * dx +
-                                c[3 * mi + i];
+                        eta = ppoly_at(m.eta_coef, mi, i, dx);
+                        vlss = ppoly_at(m.var_lss_coef, mi, i, dx);
+                        fudge = ppoly_at(m.fudge_coef, mi, i, dx);
                     }
                     const double inv_pipe = iv * (expected * expected);
                     w = 1.0 / (eta * (1.0 / inv_pipe) + m.var_lss_mod * vlss + fudge * inv_pipe);
@@ -1790,7 +1739,6 @@ int launch_cont_fit(const pg_spectra &sp, const pg_cont_model &m, const double *
                     const pg_cont_fit &out, Scratch *scratch, int num_sms, cudaStream_t stream,
                     float cert_chi2, float cert_ab) {
     if (count <= 0) return PG_OK;
-    const unsigned blocks = blocks_for(count, num_sms);
     if (mode == PG_FIT_MIXED) {
         const size_t smem = kFitSlabBytes * (kContBlock / 32) +
                             fit_smem_bytes(m.num_mean_cont, m.num_var_intervals);
@@ -1810,26 +1758,20 @@ int launch_cont_fit(const pg_spectra &sp, const pg_cont_model &m, const double *
         cont_fit_mixed_kernel<<<(unsigned)mixed_blocks, kContBlock, smem, stream>>>(
             sp, m, start, index, count, max_iter, tol, out, scratch, cert_chi2, cert_ab);
     } else {
-        cont_fit_kernel<double><<<blocks, kContBlock, 0, stream>>>(sp, m, start, index, count,
-                                                                    max_iter, tol, out, scratch);
+        const int rc = launch_fit64<kContK>(sp, m, start, index, count, max_iter, tol, out,
+                                            &scratch->work_counter, scratch, num_sms, stream);
+        if (rc) return rc;
     }
     cudaError_t err = cudaGetLastError();
     if (err != cudaSuccess) return check_cuda(err);
-    // forests longer than the register kernels hold (the linear grid), in FP64
-    const size_t long_smem = (size_t)kLongWarps * 6 * 32 * kLongK * sizeof(double);
-    err = cudaFuncSetAttribute(cont_fit_long_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)long_smem);
-    if (err != cudaSuccess) return check_cuda(err);
-    // the long kernel has no certificate: under it the warm-started fit of a
-    // long forest runs to convergence with the plain fit's iteration limit
-    const int long_iter = cert_chi2 > 0.f && max_iter < 100 ? 100 : max_iter;
-    int64_t long_blocks = (count + 32 * kLongWarps - 1) / (32 * kLongWarps);
-    if (long_blocks > (int64_t)num_sms * 8) long_blocks = (int64_t)num_sms * 8;
-    cont_fit_long_kernel<<<(unsigned)(long_blocks < 1 ? 1 : long_blocks), 32 * kLongWarps,
-                           long_smem, stream>>>(sp, m, start, index, count, long_iter,
-                                                cert_chi2 > 0.f ? 1e-10 : tol, out, scratch);
-    err = cudaGetLastError();
-    if (err != cudaSuccess) return check_cuda(err);
+    // forests longer than those hold (the linear grid), in FP64; the long form
+    // has no certificate: under it the warm-started fit of a long forest runs
+    // to convergence with the plain fit's iteration limit
+    const int rc = launch_fit64<kLongK>(sp, m, start, index, count,
+                                        cert_chi2 > 0.f && max_iter < 100 ? 100 : max_iter,
+                                        cert_chi2 > 0.f ? 1e-10 : tol, out, &scratch->long_counter, scratch,
+                                        num_sms, stream);
+    if (rc) return rc;
     if (mode == PG_FIT_MIXED && max_iter > 0 && !(cert_chi2 > 0.f)) {
         // the two-float finish of the forests flagged status 4, same stream
         const size_t rsmem = refine_smem_bytes(m.num_mean_cont, m.num_var_intervals);

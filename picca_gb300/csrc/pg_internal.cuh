@@ -27,7 +27,7 @@ struct Scratch {
     int32_t work_counter;      // persistent-kernel work queue head
     int32_t status;            // first device-side error (0 = none)
     int32_t error_detail;
-    int32_t pad;
+    int32_t long_counter;      // queue head of the long continuum fits
     unsigned long long rechecked_pairs;
     unsigned long long recheck_overflows;
     unsigned long long work_items;
