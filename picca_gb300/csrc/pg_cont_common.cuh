@@ -34,12 +34,16 @@ __device__ __forceinline__ float diff_prod(float a, float b, float c, float d) {
 // last bit); variance functions as FP32 cubics, the three functions of an
 // interval interleaved (eta, var_lss, fudge: c3 c2 c1 c0 each). Uniformly
 // spaced nodes or breaks (the usual case) are found by one multiply and a
-// correction step, others by bisection.
+// correction step, others by bisection. The quotients of the model's scalars
+// are formed by four lanes of one warp: a division is some 25 operations of
+// the FP64 pipe, which the CTA's other warps would queue for (7 us of the
+// mixed fit's 353 us for 40,000 forests).
 struct FitTables {
     const float *mc_off, *mc_y, *mc_slope, *brk;
     const float4 *coef;
     int nmc, m;
     float mc_off0, mc_inv_step, brk0, brk_inv_step;
+    float inv_span;  // 1 / (rest-frame range in log lambda)
     bool mc_uniform, brk_uniform;
 };
 
@@ -49,6 +53,8 @@ __host__ __device__ inline size_t fit_smem_bytes(int nmc, int m) {
 
 __device__ FitTables load_fit_tables(const pg_cont_model &m, unsigned char *smem) {
     __shared__ int s_uniform[2];
+    __shared__ double s_step[2];
+    __shared__ float s_inv[4];
     FitTables t;
     const int nmc = m.num_mean_cont, mi = m.use_constant_weight ? 0 : m.num_var_intervals;
     float4 *coef = reinterpret_cast<float4 *>(smem);
@@ -56,10 +62,29 @@ __device__ FitTables load_fit_tables(const pg_cont_model &m, unsigned char *smem
     float *mc_y = mc_off + nmc;
     float *mc_slope = mc_y + nmc;
     float *brk = mc_slope + nmc;
-    if (threadIdx.x == 0) s_uniform[0] = s_uniform[1] = 1;
+    // steps of the nodes (lane 0) and the breaks (1), then their reciprocals
+    // and that of the rest-frame range (2)
+    if (threadIdx.x < 4) {
+        double num = 1., den = 1.;
+        if (threadIdx.x == 0 && nmc > 1) {
+            num = m.mean_cont_x[nmc - 1] - m.mean_cont_x[0];
+            den = nmc - 1;
+        } else if (threadIdx.x == 1 && mi > 0) {
+            num = m.var_breaks[mi] - m.var_breaks[0];
+            den = mi;
+        } else if (threadIdx.x == 2) {
+            num = m.log_lambda_rest_max - m.log_lambda_rest_min;
+        }
+        const double step = num / den;
+        if (threadIdx.x < 2) {
+            s_step[threadIdx.x] = step;
+            s_uniform[threadIdx.x] = 1;
+        }
+        s_inv[threadIdx.x] = (float)(1.0 / step);
+    }
     __syncthreads();
     const double rest_min = m.log_lambda_rest_min;
-    const double mc_step = nmc > 1 ? (m.mean_cont_x[nmc - 1] - m.mean_cont_x[0]) / (nmc - 1) : 1.;
+    const double mc_step = s_step[0], brk_step = s_step[1];
     for (int i = threadIdx.x; i < nmc; i += blockDim.x) {
         const double x = m.mean_cont_x[i], y = m.mean_cont_y[i];
         mc_off[i] = (float)(x - rest_min);
@@ -68,7 +93,6 @@ __device__ FitTables load_fit_tables(const pg_cont_model &m, unsigned char *smem
                                   : 0.f;
         if (fabs(x - m.mean_cont_x[0] - i * mc_step) > 1e-3 * mc_step) s_uniform[0] = 0;
     }
-    const double brk_step = mi > 0 ? (m.var_breaks[mi] - m.var_breaks[0]) / mi : 1.;
     for (int i = threadIdx.x; i <= mi; i += blockDim.x) {
         brk[i] = (float)m.var_breaks[i];
         if (fabs(m.var_breaks[i] - m.var_breaks[0] - i * brk_step) > 1e-3 * brk_step)
@@ -88,10 +112,11 @@ __device__ FitTables load_fit_tables(const pg_cont_model &m, unsigned char *smem
     t.mc_off = mc_off; t.mc_y = mc_y; t.mc_slope = mc_slope; t.brk = brk; t.coef = coef;
     t.nmc = nmc; t.m = mi;
     t.mc_off0 = nmc > 0 ? mc_off[0] : 0.f;
-    t.mc_inv_step = (float)(1.0 / mc_step);
+    t.mc_inv_step = s_inv[0];
     t.mc_uniform = s_uniform[0] != 0 && nmc > 2;
     t.brk0 = mi > 0 ? brk[0] : 0.f;
-    t.brk_inv_step = (float)(1.0 / brk_step);
+    t.brk_inv_step = s_inv[1];
+    t.inv_span = s_inv[2];
     t.brk_uniform = s_uniform[1] != 0 && mi > 1;
     return t;
 }
@@ -162,63 +187,80 @@ __device__ __forceinline__ float2 forest_lmin(const pg_spectra &sp, const pg_con
     return split_f64(m.log_lambda_rest_min + log10(1. + sp.z_qso[f]));
 }
 
-// Sums of forest f's rest-frame bins into sums[0][bin] (sum f/mc ivar) and
+// Sums of a forest's rest-frame bins into sums[0][bin] (sum f/mc ivar) and
 // sums[1][bin] (sum ivar), zeroed here, and its scalar inputs; the whole warp
-// calls it. Consecutive pixels fall in runs of one bin across the lanes: a
-// segmented scan over the maximal runs of equal bins leaves each run's sum
-// at its last lane, which alone adds it to the bin.
-__device__ FeatScalars forest_feature_sums(const pg_spectra &sp, const FitTables &tab, int64_t f,
-                                           float lmh, float lml, float bins_per_span,
-                                           float (*sums)[kFeatBins], int lane) {
+// calls it with the forest's first pixel and length. The inputs of kFeatBatch
+// chunks of 32 pixels are asked for together, so that a forest waits for
+// memory once or twice. Consecutive pixels fall in runs of one bin across the
+// lanes: a segmented scan over the maximal runs of equal bins (as many steps
+// as the longest run asks for) leaves each run's sum at its last lane, which
+// alone adds it to the bin.
+constexpr int kFeatBatch = 3;
+
+__device__ FeatScalars forest_feature_sums(const pg_spectra &sp, const FitTables &tab, int64_t off,
+                                           int64_t n, double z_qso, float lmh, float lml,
+                                           float bins_per_span, float (*sums)[kFeatBins],
+                                           int lane) {
     for (int k = lane; k < kFeatBins; k += 32) {
         sums[0][k] = 0.f;
         sums[1][k] = 0.f;
     }
     __syncwarp();
-    const int64_t off = sp.pix_offset[f];
-    const int64_t n = sp.pix_offset[f + 1] - off;
     float sfi = 0.f, si = 0.f, snr = 0.f, cnt = 0.f;
-    for (int64_t base = 0; base < n; base += 32) {
-        const int64_t p = base + lane;
-        int bin = -1;
-        float num = 0.f, den = 0.f;
-        if (p < n) {
-            const float fl = f64_to_f32(sp.flux[off + p]);
-            const float iv = f64_to_f32(sp.ivar[off + p]);
-            sfi = fmaf(fl, iv, sfi);
-            si += iv;
-            if (iv > 0.f) {
-                snr = fmaf(fl, sqrtf(iv), snr);
-                cnt += 1.f;
-                const float2 ll = split_f64(sp.log_lambda[off + p]);
-                const float u = (ll.x - lmh) + (ll.y - lml);  // L - Lmin
-                const float mc =
-                    fit_mean_cont(tab, u) * f64_to_f32(sp.transmission_correction[off + p]);
-                if (mc != 0.f) {
-                    bin = __float2int_rd(u * bins_per_span);
-                    bin = bin < 0 ? 0 : (bin >= kFeatBins ? kFeatBins - 1 : bin);
-                    num = __fdividef(fl, mc) * iv;
-                    den = iv;
+    for (int64_t base = 0; base < n; base += 32 * kFeatBatch) {
+        double d_fl[kFeatBatch], d_iv[kFeatBatch], d_ll[kFeatBatch], d_tc[kFeatBatch];
+#pragma unroll
+        for (int c = 0; c < kFeatBatch; ++c) {
+            const int64_t p = base + 32 * c + lane;
+            d_fl[c] = d_iv[c] = d_ll[c] = d_tc[c] = 0.;
+            if (p < n) {
+                d_fl[c] = sp.flux[off + p];
+                d_iv[c] = sp.ivar[off + p];
+                d_ll[c] = sp.log_lambda[off + p];
+                d_tc[c] = sp.transmission_correction[off + p];
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < kFeatBatch; ++c) {
+            if (base + 32 * c >= n) break;
+            int bin = -1;
+            float num = 0.f, den = 0.f;
+            const float fl = f64_to_f32(d_fl[c]);
+            const float iv = f64_to_f32(d_iv[c]);
+            if (base + 32 * c + lane < n) {
+                sfi = fmaf(fl, iv, sfi);
+                si += iv;
+                if (iv > 0.f) {
+                    snr = fmaf(fl, sqrtf(iv), snr);
+                    cnt += 1.f;
+                    const float2 ll = split_f64(d_ll[c]);
+                    const float u = (ll.x - lmh) + (ll.y - lml);  // L - Lmin
+                    const float mc = fit_mean_cont(tab, u) * f64_to_f32(d_tc[c]);
+                    if (mc != 0.f) {
+                        bin = __float2int_rd(u * bins_per_span);
+                        bin = bin < 0 ? 0 : (bin >= kFeatBins ? kFeatBins - 1 : bin);
+                        num = __fdividef(fl, mc) * iv;
+                        den = iv;
+                    }
                 }
             }
-        }
-        const int prev = __shfl_up_sync(0xffffffffu, bin, 1);
-        const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || prev != bin);
-        const unsigned upto = lane == 31 ? 0xffffffffu : ((2u << lane) - 1u);
-        const int start = 31 - __clz(heads & upto);  // first lane of this run
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const float tn = __shfl_up_sync(0xffffffffu, num, o);
-            const float td = __shfl_up_sync(0xffffffffu, den, o);
-            if (lane - o >= start) {
-                num += tn;
-                den += td;
+            const int prev = __shfl_up_sync(0xffffffffu, bin, 1);
+            const unsigned heads = __ballot_sync(0xffffffffu, lane == 0 || prev != bin);
+            const unsigned upto = lane == 31 ? 0xffffffffu : ((2u << lane) - 1u);
+            const int before = lane - (31 - __clz(heads & upto));  // lanes of this run before
+            for (int o = 1; __any_sync(0xffffffffu, before >= o); o <<= 1) {
+                const float tn = __shfl_up_sync(0xffffffffu, num, o);
+                const float td = __shfl_up_sync(0xffffffffu, den, o);
+                if (before >= o) {
+                    num += tn;
+                    den += td;
+                }
             }
-        }
-        const int next = __shfl_down_sync(0xffffffffu, bin, 1);
-        if (bin >= 0 && (lane == 31 || next != bin)) {
-            atomicAdd(&sums[0][bin], num);
-            atomicAdd(&sums[1][bin], den);
+            const int next = __shfl_down_sync(0xffffffffu, bin, 1);
+            if (bin >= 0 && (lane == 31 || next != bin)) {
+                atomicAdd(&sums[0][bin], num);
+                atomicAdd(&sums[1][bin], den);
+            }
         }
     }
     sfi = warp_sum_f(sfi);
@@ -228,7 +270,7 @@ __device__ FeatScalars forest_feature_sums(const pg_spectra &sp, const FitTables
     __syncwarp();
     FeatScalars fs;
     fs.a0 = si > 0.f ? sfi / si : 0.f;
-    fs.zfeat = f64_to_f32(sp.z_qso[f]) - 3.f;
+    fs.zfeat = f64_to_f32(z_qso) - 3.f;
     fs.snrfeat = logf(fmaxf(cnt > 0.f ? snr / cnt : 0.f, 1e-3f));
     return fs;
 }

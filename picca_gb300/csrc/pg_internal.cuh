@@ -344,7 +344,6 @@ int launch_mlp_warm_start_tc(const pg_spectra &sp, const pg_cont_model &model,
                              const uint16_t *packed, const float *params, float *y, double *a0,
                              Scratch *scratch, int num_sms, cudaStream_t stream);
 int launch_mlp_features(const pg_spectra &sp, const pg_cont_model &m, uint16_t *features,
-                        int stride, double *a0, Scratch *scratch, int num_sms,
-                        cudaStream_t stream);
+                        int stride, double *a0, int num_sms, cudaStream_t stream);
 
 }  // namespace pg

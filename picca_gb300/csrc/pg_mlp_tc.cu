@@ -252,8 +252,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_forward_tc_kernel(
             return;
         }
         // the warp's 8 forests of the tile, features formed in place
-        const float bins_per_span =
-            (float)(kFeatBins / (model.log_lambda_rest_max - model.log_lambda_rest_min));
+        const float bins_per_span = kFeatBins * tab.inv_span;
         const int r0 = warp * 8;
         if (lane < 8 && row0 + r0 + lane < m) {
             const float2 lm = forest_lmin(sp, model, row0 + r0 + lane);
@@ -266,8 +265,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) mlp_forward_tc_kernel(
             const int64_t f = row0 + r;
             FeatScalars fs{0.f, 0.f, 0.f};
             if (f < m) {
-                fs = forest_feature_sums(sp, tab, f, s_lm[warp][j][0], s_lm[warp][j][1],
-                                         bins_per_span, s_feat_sums[warp], lane);
+                const int64_t off = sp.pix_offset[f];
+                fs = forest_feature_sums(sp, tab, off, sp.pix_offset[f + 1] - off, sp.z_qso[f],
+                                         s_lm[warp][j][0], s_lm[warp][j][1], bins_per_span,
+                                         s_feat_sums[warp], lane);
                 if (lane == 0) a0_out[f] = f32_to_f64(fs.a0);
             }
             if (lane < kInPad / 8) {
