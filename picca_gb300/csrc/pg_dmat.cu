@@ -75,6 +75,7 @@ struct DmatConst {
     int64_t cta_doubles;     // list_doubles + work_doubles (+ digits and exponents)
     int32_t split;           // 1: tensor-core product (PG_DMAT_SPLIT_BF16)
     int32_t xcf;             // 1: delta x quasar layout (forest, quasar slots)
+    int32_t key_rows, key_pitch;  // rows of bins in shared memory (cf_dmat_same_kernel)
 };
 
 // Shared-memory layout (bytes), identical on host and device.
@@ -1059,6 +1060,634 @@ __global__ void __launch_bounds__(kDmBlock, 2)
 }
 
 // ---------------------------------------------------------------------------
+// Equal data and model binning in (r_par, r_trans), the usual matrix: every
+// pixel pair is decided once, in FP32, and its bin kept in shared memory; the
+// few pairs inside a guard band wait in a queue and are decided in FP64 32 at
+// a time. The sweeps read those bins along each row's and column's window of
+// accepted pixels and add four (row: and r_par) FP64 numbers a pair, and the
+// effective sums come from U: with U_i and X_j a bin's sums of w12 over row i
+// and column j,
+//   weights = sum_i U_i,  2 z_eff = sum_i z1_i U_i + sum_j z2_j X_j,
+//   r_trans_eff = sin (sum_i m1_i U_i + sum_j m2_j X_j),
+// and where every pair of the forest pair is selected the Kronecker term of a
+// bin is sum(w1) sum(w2) eta5. U and X are stored with their z factor
+// (w zf sum w'), E and its kin as plain sums (-sum a'), so that a run costs
+// two products, and the factors 1 / zf are in the pixel arrays of stage 3.
+//
+// Bound: the FP64 pipe (10 operations an accepted pair, 12 a stored element
+// in stage 3). The form below it (cf_dmat_kernel) decides every pair three
+// times, with FP64 decisions in divergence, and adds 16 numbers a pair in
+// runs whose ends cost 16 more. 6,200 pairs of 160-pixel forests, 50 x 50 bins:
+// 36.4 ms in the general form, 27.8 ms here (sweeps 8 ms of it, they were 25).
+//
+// Forests whose bins do not fit in shared memory at once go through in strips
+// of rows, decided once more for each strip.
+constexpr int kDsQueue = 512;         // guard-band pairs waiting; more are decided in place
+constexpr int kDsMaxBins = 0x7FFF;
+constexpr uint16_t kDsNone = 0xFFFF;  // outside the binning
+constexpr uint16_t kDsVeto = 0x8000;  // in the model range only
+
+// Pixel arrays in shared memory. While the forests are staged iz, diz, ziz and
+// miz hold zf, log lambda (then minus its mean), z and dist_m.
+struct DsPix {
+    double *r, *w;
+    double *wd;   // w dll
+    double *a;    // zf w / sum(w)
+    double *b;    // zf w dll / sum(w dll^2)
+    double *wzf;  // w zf
+    double *iz, *diz, *ziz, *miz;  // 1, dll, z / 2 and dist_m, each over zf
+    float *rh, *rl, *mf;
+};
+
+constexpr size_t kDsPixBytes = sizeof(double) * 10 + sizeof(float) * 3;
+
+__device__ __forceinline__ DsPix ds_pix(unsigned char *base, int p) {
+    double *d = reinterpret_cast<double *>(base);
+    float *f = reinterpret_cast<float *>(d + 10 * p);
+    return {d, d + p, d + 2 * p, d + 3 * p, d + 4 * p, d + 5 * p, d + 6 * p, d + 7 * p,
+            d + 8 * p, d + 9 * p, f, f + p, f + 2 * p};
+}
+
+// Shared-memory layout (bytes). The bins share their place with the product's
+// tiles.
+struct DsSmem {
+    size_t f1, f2, flags1, flags2, win1, win2, mbits, mpref, dbits, dpref, list, queue, keys, total;
+};
+
+__host__ __device__ inline size_t dm_tile_bytes(int split) {
+    return split ? 4 * sizeof(uint16_t) * kSlices * kTcM * kTcRow
+                 : 2 * sizeof(double) * kSlab * kTilePad;
+}
+
+__host__ __device__ inline DsSmem ds_smem(int p1, int p2, int words, size_t key_bytes) {
+    DsSmem s;
+    size_t o = 0;
+    s.f1 = o; o = dm_align(o + kDsPixBytes * (size_t)p1, 16);
+    s.f2 = o; o = dm_align(o + kDsPixBytes * (size_t)p2, 16);
+    s.flags1 = o; o += (size_t)p1;
+    s.flags2 = o; o = dm_align(o + (size_t)p2, 8);
+    s.win1 = o; o += 8 * (size_t)p1;
+    s.win2 = o; o += 8 * (size_t)p2;
+    s.mbits = o; o += 4 * (size_t)words;
+    s.mpref = o; o += 4 * (size_t)words;
+    s.dbits = o; o += 4 * (size_t)words;
+    s.dpref = o; o += 4 * (size_t)words;
+    s.list = o; o += 2 * 32 * (size_t)words;
+    s.queue = o; o += 4 * kDsQueue;
+    o = dm_align(o, 16);
+    s.keys = o;
+    s.total = o + key_bytes;
+    return s;
+}
+
+// Bins of a row: lanes that walk neighbouring rows (or columns) at one
+// distance from the diagonal are pitch + 1 apart; an odd number of words keeps
+// them on different banks.
+__host__ __device__ inline int ds_pitch(int p2) { return ((p2 + 1) / 4) * 4 + 1 >= p2
+                                                      ? ((p2 + 1) / 4) * 4 + 1
+                                                      : ((p2 + 1) / 4) * 4 + 5; }
+
+// dm_pair_f32 for equal binnings.
+__device__ __forceinline__ int ds_pair_f32(const DmatConst &c, const DmGuard &g, float r1h,
+                                           float r1l, float m1, float r2h, float r2l, float m2,
+                                           bool shp, int &bin, bool &counted) {
+    const float d = __fadd_rn(__fsub_rn(r1h, r2h), __fsub_rn(r1l, r2l));
+    float rp = __fmul_rn(d, g.cc);
+    if (!c.b.x_correlation) rp = fabsf(rp);
+    const float rt = __fmul_rn(__fadd_rn(m1, m2), g.ss);
+    if (rp >= c.f_rpmax + g.gp || rt >= c.f_rtmax + g.gt || rp < c.f_rpmin - g.gp) return 0;
+    if (rp > c.f_rpmax - g.gp || rt > c.f_rtmax - g.gt || rp < c.f_rpmin + g.gp) return 2;
+    counted = true;
+    if (c.b.remove_shp && shp) {
+        const float a = fabsf(rp);
+        if (fabsf(__fsub_rn(a, c.f_hpc)) <= g.gp) return 2;
+        counted = a >= c.f_hpc;
+    }
+    const float yp = __fmul_rn(__fsub_rn(rp, c.f_rpmin), c.f_sp), yt = __fmul_rn(rt, c.f_st);
+    const float bp = floorf(yp), bt = floorf(yt);
+    if (yp - bp <= g.gyp || bp + 1.f - yp <= g.gyp || yt - bt <= g.gyt || bt + 1.f - yt <= g.gyt)
+        return 2;
+    bin = (int32_t)bt + c.b.nt * (int32_t)bp;
+    return 1;
+}
+
+__global__ void __launch_bounds__(kDmBlock, 2)
+    cf_dmat_same_kernel(DmatConst c, pg_forest_set s1, pg_forest_set s2, const double *ll1,
+                        const double *ll2, const int32_t *order1g, const int32_t *order2g,
+                        const int32_t *pair_first, const int32_t *pair_second,
+                        const double *pair_angle, int64_t num_pairs, pg_dmat_sums out,
+                        double *work, Scratch *scratch) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const DsSmem L = ds_smem(c.p1, c.p2, c.mwords, 0);
+    const DsPix P1 = ds_pix(smem + L.f1, c.p1);
+    const DsPix P2 = ds_pix(smem + L.f2, c.p2);
+    unsigned char *sel1 = smem + L.flags1, *sel2 = smem + L.flags2;
+    int2 *win1 = reinterpret_cast<int2 *>(smem + L.win1);  // first and last + 1 accepted j
+    int2 *win2 = reinterpret_cast<int2 *>(smem + L.win2);  // and i (of the strip)
+    uint32_t *mbits = reinterpret_cast<uint32_t *>(smem + L.mbits);
+    int32_t *mpref = reinterpret_cast<int32_t *>(smem + L.mpref);
+    uint32_t *dbits = reinterpret_cast<uint32_t *>(smem + L.dbits);
+    int32_t *dpref = reinterpret_cast<int32_t *>(smem + L.dpref);
+    uint16_t *list = reinterpret_cast<uint16_t *>(smem + L.list);  // bin of a model rank
+    uint32_t *queue = reinterpret_cast<uint32_t *>(smem + L.queue);
+    uint16_t *keys = reinterpret_cast<uint16_t *>(smem + L.keys);
+    double (*ta)[kTilePad] = reinterpret_cast<double (*)[kTilePad]>(smem + L.keys);
+    double (*tb)[kTilePad] = ta + kSlab;
+    uint16_t *ta_raw = reinterpret_cast<uint16_t *>(smem + L.keys);
+    uint16_t *tb_raw = ta_raw + 2 * kSlices * kTcM * kTcRow;
+    __shared__ double red[kDmWarps];
+    __shared__ int red_int[kDmWarps];
+    __shared__ int s_item, s_count, s_veto, s_queue;
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int nb = c.b.nbins;
+    double *cta = work + (int64_t)blockIdx.x * c.cta_doubles;
+    int32_t *dlist = reinterpret_cast<int32_t *>(cta);  // [nb]
+    int32_t *mlist = dlist + nb;                         // [nb]
+    double *rows = cta + c.list_doubles;
+    uint16_t *digits = reinterpret_cast<uint16_t *>(rows + c.work_doubles);
+    int32_t *rexp = reinterpret_cast<int32_t *>(digits + (c.work_doubles * kSlices));
+    const int pitch = c.key_pitch;
+
+    for (;;) {
+        if (tid == 0) s_item = atomicAdd(&scratch->work_counter, 1);
+        __syncthreads();
+        const int64_t q = s_item;
+        if (q >= num_pairs) break;
+        const int f = pair_first[q], g = pair_second[q];
+        const int64_t o1 = s1.pix_offset[f], o2 = s2.pix_offset[g];
+        const int n1 = (int)(s1.pix_offset[f + 1] - o1);
+        const int n2 = (int)(s2.pix_offset[g + 1] - o2);
+        if (n1 > c.p1 || n2 > c.p2) {
+            if (tid == 0) report_error(scratch, PG_ERR_UNSUPPORTED, (int32_t)q);
+            __syncthreads();
+            continue;
+        }
+        const double ang = pair_angle ? pair_angle[q]
+                                      : angle_between(s1.x_cart[f], s1.y_cart[f], s1.z_cart[f],
+                                                      s1.ra[f], s1.dec[f], s1.cos_dec[f],
+                                                      s2.x_cart[g], s2.y_cart[g], s2.z_cart[g],
+                                                      s2.ra[g], s2.dec[g]);
+        const double cc = cos(ang / 2), ss = sin(ang / 2);
+        const bool ord1 = order1g[f] == 1, ord2 = order2g[g] == 1;
+        bool shp = false;
+        if (c.b.remove_shp && s1.plate[f] == s2.plate[g]) {
+            const int64_t a = s1.fiberid[f], b2 = s2.fiberid[g];
+            shp = (a <= 500 && b2 <= 500) || (a > 500 && b2 > 500);
+        }
+        const bool zerr_on = c.b.zerr_on && ang < c.b.zerr_ang;
+        const double zq1 = s1.z_qso[f], zq2 = s2.z_qso[g];
+
+        // stage the pixels; flags: bit 0 a weight, bit 1 passes the redshift veto
+        float lmax = 0.f, lmmax = 0.f;
+        auto stage = [&](const DsPix &P, const pg_forest_set &s, int64_t o, int n,
+                         const double *ll, unsigned char *sel, double zq) {
+            for (int t = tid; t < n; t += kDmBlock) {
+                const double r = s.r_comov[o + t], m = s.dist_m[o + t], z = s.z[o + t];
+                const double w = s.weights[o + t];
+                P.r[t] = r;
+                P.w[t] = w;
+                P.ziz[t] = z;
+                P.miz[t] = m;
+                P.diz[t] = ll[o + t];
+                const float rh = (float)r, mf = (float)m;
+                P.rh[t] = rh;
+                P.rl[t] = (float)__dsub_rn(r, (double)rh);
+                P.mf[t] = mf;
+                lmax = fmaxf(lmax, fabsf(rh));
+                lmmax = fmaxf(lmmax, fabsf(mf));
+                sel[t] = (w != 0. ? 1 : 0) | (zerr_on && zerr_veto(z, zq, c.b.zerr_kms) ? 0 : 2);
+            }
+        };
+        stage(P1, s1, o1, n1, ll1, sel1, zq2);
+        stage(P2, s2, o2, n2, ll2, sel2, zq1);
+        for (int t = tid; t < c.mwords; t += kDmBlock) mbits[t] = dbits[t] = 0u;
+        // guard bands as in cf_dmat_kernel (the maxima rounded to FP32: one
+        // part in 2^24 of a bound that is doubled)
+        for (int o = 16; o > 0; o >>= 1) {
+            lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
+            lmmax = fmaxf(lmmax, __shfl_xor_sync(0xffffffffu, lmmax, o));
+        }
+        if (lane == 0) red[warp] = __hiloint2double(__float_as_int(lmax), __float_as_int(lmmax));
+        if (tid == 0) s_count = s_veto = 0;
+        __syncthreads();
+        float rmax = 0.f, mmax = 0.f;
+        for (int k = 0; k < kDmWarps; ++k) {
+            rmax = fmaxf(rmax, __int_as_float(__double2hiint(red[k])));
+            mmax = fmaxf(mmax, __int_as_float(__double2loint(red[k])));
+        }
+        DmGuard gd;
+        {
+            // in FP32, each factor rounded up by the last term
+            constexpr float u = 5.9604645e-8f, up = 1.00001f;  // 2^-24
+            gd.cc = (float)cc;
+            gd.ss = (float)ss;
+            const float rlim = fmaxf(fabsf(c.f_rpmax), fabsf(c.f_rpmin));
+            gd.gp = up * 2.f * (2.f * u * rmax + 3.f * u * (rlim + 1.f) / fmaxf(gd.cc, 1e-6f));
+            gd.gt = up * 2.f * (4.f * u * mmax * gd.ss + 2.f * u * c.f_rtmax);
+            gd.gyp = up * (gd.gp * c.f_sp + 8.f * u * (c.b.np + 1));
+            gd.gyt = up * (gd.gt * c.f_st + 8.f * u * (c.b.nt + 1));
+            gd.gymp = gd.gyp;
+            gd.gymt = gd.gyt;
+        }
+        __syncthreads();
+
+        // 1. bins of the pairs of rows [i0, i1): as bins with the bitmaps of
+        // the touched model bins and of the data bins of selected pairs, or
+        // (the bitmaps known) as ranks of model bins
+        auto decide_strip = [&](int i0, int i1, bool ranked) {
+            for (int t = tid; t < n1; t += kDmBlock) win1[t] = make_int2(n2, 0);
+            for (int t = tid; t < n2; t += kDmBlock) win2[t] = make_int2(n1, 0);
+            if (tid == 0) s_queue = 0;
+            __syncthreads();
+            int counted = 0, veto = 0;
+            auto settle = [&](int i, int j, int bin, bool cnt) {
+                if (bin < 0 || bin >= nb) {
+                    report_error(scratch, PG_ERR_BIN_RANGE, bin);
+                    return kDsNone;
+                }
+                bool sel = cnt && (sel1[i] & sel2[j] & 2);
+                if (sel && (c.b.zmin_on || c.b.zmax_on)) {
+                    const double z = __dadd_rn(s1.z[o1 + i], s2.z[o2 + j]) / 2;
+                    sel = !((c.b.zmin_on && z < c.b.z_min) || (c.b.zmax_on && z > c.b.z_max));
+                }
+                const uint16_t mark = sel ? 0 : kDsVeto;
+                if (ranked) return (uint16_t)(dm_rank(mbits, mpref, bin) | mark);
+                counted += cnt;
+                veto |= !sel;
+                const uint32_t bit = 1u << (bin & 31);
+                if (!(mbits[bin >> 5] & bit)) atomicOr(&mbits[bin >> 5], bit);
+                if (sel && !(dbits[bin >> 5] & bit)) atomicOr(&dbits[bin >> 5], bit);
+                return (uint16_t)(bin | mark);
+            };
+            auto decide64 = [&](int i, int j) {
+                DmPair o;
+                if (!dm_pair(c, P1.r[i], s1.dist_m[o1 + i], s1.z[o1 + i], P2.r[j],
+                             s2.dist_m[o2 + j], s2.z[o2 + j], cc, ss, shp, o))
+                    return kDsNone;
+                return settle(i, j, o.db, o.counted);
+            };
+            const int chunks = (n2 + 31) >> 5;
+            const int part = (i1 - i0 + 3) >> 2;  // four warp tasks a chunk of columns
+            for (int t = warp; t < 4 * chunks; t += kDmWarps) {
+                const int j = (t >> 2) * 32 + lane;
+                const int a0 = i0 + (t & 3) * part, a1 = min(i1, a0 + part);
+                const bool live = j < n2 && (sel2[j] & 1);
+                const float rh = live ? P2.rh[j] : 0.f, rl = live ? P2.rl[j] : 0.f;
+                const float mf = live ? P2.mf[j] : 0.f;
+                int lo = n1, hi = 0;
+                for (int i = a0; i < a1; ++i) {
+                    int st = 0, bin = 0;
+                    bool cnt = false;
+                    if (live && (sel1[i] & 1))
+                        st = ds_pair_f32(c, gd, P1.rh[i], P1.rl[i], P1.mf[i], rh, rl, mf, shp,
+                                         bin, cnt);
+                    uint16_t key = kDsNone;
+                    if (st == 1) key = settle(i, j, bin, cnt);
+                    if (st == 2) {
+                        const int at = atomicAdd(&s_queue, 1);
+                        if (at < kDsQueue) queue[at] = (uint32_t)i << 16 | (uint32_t)j;
+                        else key = decide64(i, j);
+                    }
+                    if (j < n2) keys[(i - i0) * pitch + j] = key;
+                    const unsigned in = __ballot_sync(0xffffffffu, key != kDsNone);
+                    if (key != kDsNone) {
+                        lo = min(lo, i);
+                        hi = i + 1;
+                    }
+                    if (in && lane == 0) {
+                        atomicMin(&win1[i].x, j + __ffs(in) - 1);
+                        atomicMax(&win1[i].y, j + 32 - __clz(in));
+                    }
+                }
+                if (hi) {
+                    atomicMin(&win2[j].x, lo);
+                    atomicMax(&win2[j].y, hi);
+                }
+            }
+            __syncthreads();
+            const int waiting = min(s_queue, kDsQueue);
+            for (int e = tid; e < waiting; e += kDmBlock) {
+                const int i = queue[e] >> 16, j = queue[e] & 0xFFFF;
+                const uint16_t key = decide64(i, j);
+                if (key == kDsNone) continue;
+                keys[(i - i0) * pitch + j] = key;
+                atomicMin(&win1[i].x, j);
+                atomicMax(&win1[i].y, j + 1);
+                atomicMin(&win2[j].x, i);
+                atomicMax(&win2[j].y, i + 1);
+            }
+            if (!ranked) {
+                counted = __reduce_add_sync(0xffffffffu, counted);
+                if (lane == 0 && counted) atomicAdd(&s_count, counted);
+                if (veto) s_veto = 1;
+            }
+            __syncthreads();
+        };
+        const int strips = (n1 + c.key_rows - 1) / c.key_rows;
+        const int strip = max(1, (n1 + strips - 1) / max(1, strips));
+        const bool one_strip = strip >= n1;
+        for (int i0 = 0; i0 < n1; i0 += strip) decide_strip(i0, min(n1, i0 + strip), false);
+        if (s_count == 0) {
+            __syncthreads();
+            continue;
+        }
+        const bool veto = s_veto != 0;
+        const int nmt = dm_scan_bits(mbits, mpref, c.mwords, red_int);
+        const int nbt = dm_scan_bits(dbits, dpref, c.mwords, red_int);
+        if (nbt == 0) {  // no selected pair: nothing reaches the matrix
+            __syncthreads();
+            continue;
+        }
+        if (tid == 0) atomicAdd(&scratch->work_items, 1ull);
+        for (int w = tid; w < c.mwords; w += kDmBlock) {
+            int k = mpref[w];
+            for (uint32_t bits = mbits[w]; bits; bits &= bits - 1u) {
+                const int bin = w * 32 + __ffs(bits) - 1;
+                list[k] = (uint16_t)bin;
+                mlist[k++] = bin;
+            }
+            k = dpref[w];
+            for (uint32_t bits = dbits[w]; bits; bits &= bits - 1u)
+                dlist[k++] = w * 32 + __ffs(bits) - 1;
+        }
+        if (one_strip)  // bins -> ranks
+            for (int i = warp; i < n1; i += kDmWarps) {
+                const int2 win = win1[i];
+                for (int j = win.x + lane; j < win.y; j += 32) {
+                    const uint16_t key = keys[i * pitch + j];
+                    if (key != kDsNone)
+                        keys[i * pitch + j] = (uint16_t)(
+                            dm_rank(mbits, mpref, key & ~kDsVeto) | (key & kDsVeto));
+                }
+            }
+
+        // auxiliary sums (py/picca/cf.py:573-595) and per-pixel factors
+        auto weigh = [&](const DsPix &P, int n, double alpha, double &sw, double &sq) {
+            double lw = 0., lsw = 0.;
+            for (int t = tid; t < n; t += kDmBlock) {
+                lw += P.w[t];
+                lsw += __dmul_rn(P.diz[t], P.w[t]);
+            }
+            sw = dm_block_sum(lw, red);
+            const double mean = dm_block_sum(lsw, red) / sw;
+            double lq = 0.;
+            for (int t = tid; t < n; t += kDmBlock) {
+                const double d = __dsub_rn(P.diz[t], mean);
+                P.diz[t] = d;
+                lq += __dmul_rn(P.w[t], __dmul_rn(d, d));
+                P.iz[t] = c.redshift_evolution
+                              ? pow(__dadd_rn(1., P.ziz[t]) / __dadd_rn(1., c.z_ref),
+                                    __dsub_rn(alpha, 1.))
+                              : 1.;
+            }
+            sq = dm_block_sum(lq, red);
+            const double inv_sw = 1. / sw, inv_q = 1. / sq;
+            for (int t = tid; t < n; t += kDmBlock) {
+                const double w = P.w[t], zf = P.iz[t], d = P.diz[t];
+                const double wz = __dmul_rn(w, zf), iz = 1. / zf;
+                P.wzf[t] = wz;
+                P.a[t] = __dmul_rn(wz, inv_sw);
+                P.b[t] = __dmul_rn(__dmul_rn(wz, d), inv_q);
+                P.wd[t] = __dmul_rn(w, d);
+                P.iz[t] = iz;
+                P.diz[t] = __dmul_rn(d, iz);
+                P.ziz[t] = __dmul_rn(0.5 * P.ziz[t], iz);
+                P.miz[t] = __dmul_rn(P.miz[t], iz);
+            }
+        };
+        double sw1, sw2, sq1, sq2;
+        weigh(P1, n1, c.alpha, sw1, sq1);
+        weigh(P2, n2, c.alpha2, sw2, sq2);
+        if ((ord1 && !(sq1 != 0.)) || (ord2 && !(sq2 != 0.))) {
+            // the reference divides by zero here (a forest without spread in
+            // log lambda); the pair is reported and skipped
+            if (tid == 0) report_error(scratch, PG_ERR_INVALID_ARGUMENT, (int32_t)q);
+            __syncthreads();
+            continue;
+        }
+
+        // kappa layout of the U and E rows
+        const int kU = 0, kX = n1, kV = n1 + n2;
+        const int kY = kV + (ord2 ? n1 : 0);
+        const int kR = kY + (ord1 ? n2 : 0);
+        const int kst = (int)dm_align((size_t)kR + 4, kSlab);
+        const int64_t cap = c.work_doubles / kst;
+        int dc = nbt, mc = nmt;
+        if ((int64_t)nbt + nmt > cap) {
+            dc = (int)min((int64_t)nbt, cap / 2);
+            mc = (int)(cap - dc);
+        }
+        const bool one_chunk = dc == nbt && mc == nmt;
+        __syncthreads();
+
+        for (int d0 = 0; d0 < nbt; d0 += dc) {
+            const int dcc = min(dc, nbt - d0);
+            for (int m0 = 0; m0 < nmt; m0 += mc) {
+                const int mcc = min(mc, nmt - m0);
+                const bool first = d0 == 0 && m0 == 0;
+                double *U = rows;
+                double *E = rows + (int64_t)dcc * kst;
+                {
+                    const int64_t n = (int64_t)(dcc + mcc) * kst / 2;
+                    double2 *p = reinterpret_cast<double2 *>(rows);
+                    for (int64_t t = tid; t < n; t += kDmBlock) p[t] = make_double2(0., 0.);
+                }
+                // 2. sweeps over the windows, half a row's or column's a lane:
+                // an entry belongs to one pixel (its two halves and, where
+                // |r_par| falls and rises again, two runs may share it), added
+                // with atomics that return nothing and read back through L2
+                for (int i0 = 0; i0 < n1; i0 += strip) {
+                    const int i1 = min(n1, i0 + strip);
+                    if (!(one_strip && one_chunk)) decide_strip(i0, i1, true);
+                    __syncthreads();
+                    const int rtasks = 2 * ((i1 - i0 + 31) >> 5);
+                    const int ctasks = 2 * ((n2 + 31) >> 5);
+                    for (int t = warp; t < rtasks + ctasks; t += kDmWarps) {
+                        if (t < rtasks) {
+                            const int i = i0 + (t >> 1) * 32 + lane;
+                            if (i >= i1) continue;
+                            const int2 win = win1[i];
+                            const int mid = (win.x + win.y) >> 1;
+                            const int jb = (t & 1) ? mid : win.x, je = (t & 1) ? win.y : mid;
+                            const double r1 = P1.r[i], wzf = P1.wzf[i], w1cc = P1.w[i] * cc;
+                            const double kron = sw2 * wzf;
+                            const uint16_t *row = keys + (i - i0) * pitch;
+                            uint16_t run = kDsNone;
+                            double e1 = 0., e3 = 0., u = 0., v = 0., rp = 0.;
+                            auto flush = [&]() {
+                                const int mr = run & ~kDsVeto, ml = mr - m0;
+                                if (ml >= 0 && ml < mcc) {
+                                    double *e = E + (int64_t)ml * kst + i;
+                                    atomicAdd(e + kU, e1);
+                                    if (ord2) atomicAdd(e + kV, e3);
+                                }
+                                if (run & kDsVeto) return;
+                                const int bin = list[mr];
+                                const int dl = (veto ? dm_rank(dbits, dpref, bin) : mr) - d0;
+                                if (dl >= 0 && dl < dcc) {
+                                    double *p = U + (int64_t)dl * kst + i;
+                                    atomicAdd(p + kU, wzf * u);
+                                    if (ord2) atomicAdd(p + kV, wzf * v);
+                                }
+                                if (first) {
+                                    atomicAdd(&out.r_par_eff[bin], w1cc * rp);
+                                    if (veto)
+                                        atomicAdd(&out.dmat[(int64_t)bin * nb + bin], -kron * e1);
+                                }
+                            };
+                            for (int j = jb; j < je; ++j) {
+                                const uint16_t key = row[j];
+                                if (key != run) {
+                                    if (run != kDsNone) flush();
+                                    run = key;
+                                    e1 = e3 = u = v = rp = 0.;
+                                }
+                                if (key == kDsNone) continue;
+                                const double w2 = P2.w[j];
+                                double d = __dsub_rn(r1, P2.r[j]);
+                                if (!c.b.x_correlation) d = fabs(d);
+                                e1 -= P2.a[j];
+                                u += w2;
+                                rp = __fma_rn(w2, d, rp);
+                                if (ord2) {
+                                    e3 -= P2.b[j];
+                                    v += P2.wd[j];
+                                }
+                            }
+                            if (run != kDsNone) flush();
+                        } else {
+                            const int j = ((t - rtasks) >> 1) * 32 + lane;
+                            if (j >= n2) continue;
+                            const int2 win = win2[j];
+                            const int mid = (win.x + win.y) >> 1;
+                            const int ib = (t & 1) ? mid : win.x, ie = (t & 1) ? win.y : mid;
+                            const double wzf = P2.wzf[j];
+                            const uint16_t *col = keys + j - i0 * pitch;
+                            uint16_t run = kDsNone;
+                            double e2 = 0., e4 = 0., x = 0., y = 0.;
+                            auto flush = [&]() {
+                                const int mr = run & ~kDsVeto, ml = mr - m0;
+                                if (ml >= 0 && ml < mcc) {
+                                    double *e = E + (int64_t)ml * kst + j;
+                                    atomicAdd(e + kX, e2);
+                                    if (ord1) atomicAdd(e + kY, e4);
+                                }
+                                if (run & kDsVeto) return;
+                                const int dl = (veto ? dm_rank(dbits, dpref, list[mr]) : mr) - d0;
+                                if (dl >= 0 && dl < dcc) {
+                                    double *p = U + (int64_t)dl * kst + j;
+                                    atomicAdd(p + kX, wzf * x);
+                                    if (ord1) atomicAdd(p + kY, wzf * y);
+                                }
+                            };
+                            for (int i = ib; i < ie; ++i) {
+                                const uint16_t key = col[i * pitch];
+                                if (key != run) {
+                                    if (run != kDsNone) flush();
+                                    run = key;
+                                    e2 = e4 = x = y = 0.;
+                                }
+                                if (key == kDsNone) continue;
+                                e2 -= P1.a[i];
+                                x += P1.w[i];
+                                if (ord1) {
+                                    e4 -= P1.b[i];
+                                    y += P1.wd[i];
+                                }
+                            }
+                            if (run != kDsNone) flush();
+                        }
+                    }
+                    __syncthreads();
+                }
+
+                // 3. rank rows and effective sums; blocks of zeros are passed over
+                for (int r = warp; r < dcc + mcc; r += kDmWarps) {
+                    double *row = rows + (int64_t)r * kst;
+                    double s0 = 0., s1v = 0., s2v = 0., s3 = 0., sz = 0., sm = 0.;
+                    if (r < dcc) {
+                        for (int b = 0; b < n1; b += 32) {
+                            const int i = b + lane;
+                            const double x = i < n1 ? __ldcg(row + kU + i) : 0.;
+                            const double y = ord1 && ord2 && i < n1 ? __ldcg(row + kV + i) : 0.;
+                            if (!__any_sync(0xffffffffu, x != 0. || y != 0.) || i >= n1) continue;
+                            s0 = __fma_rn(P1.iz[i], x, s0);
+                            s2v = __fma_rn(P1.diz[i], x, s2v);
+                            if (ord1 && ord2) s3 = __fma_rn(P1.diz[i], y, s3);
+                            if (m0 == 0) {
+                                sz = __fma_rn(P1.ziz[i], x, sz);
+                                sm = __fma_rn(P1.miz[i], x, sm);
+                            }
+                        }
+                        for (int b = 0; b < n2; b += 32) {
+                            const int j = b + lane;
+                            const double x = j < n2 ? __ldcg(row + kX + j) : 0.;
+                            if (!__any_sync(0xffffffffu, x != 0.) || j >= n2) continue;
+                            s1v = __fma_rn(P2.diz[j], x, s1v);
+                            if (m0 == 0) {
+                                sz = __fma_rn(P2.ziz[j], x, sz);
+                                sm = __fma_rn(P2.miz[j], x, sm);
+                            }
+                        }
+                        if (m0 == 0) {
+                            sz = warp_sum(sz);
+                            sm = warp_sum(sm);
+                        }
+                    } else {
+                        for (int b = 0; b < n1; b += 32) {
+                            const int i = b + lane;
+                            const double x = i < n1 ? __ldcg(row + kU + i) : 0.;
+                            const double y = ord2 && i < n1 ? __ldcg(row + kV + i) : 0.;
+                            if (!__any_sync(0xffffffffu, x != 0. || y != 0.) || i >= n1) continue;
+                            s0 = __fma_rn(-P1.a[i], x, s0);
+                            if (ord2) s1v = __fma_rn(-P1.a[i], y, s1v);
+                            if (ord1) {
+                                s2v = __fma_rn(-P1.b[i], x, s2v);
+                                if (ord2) s3 = __fma_rn(-P1.b[i], y, s3);
+                            }
+                        }
+                    }
+                    s0 = warp_sum(s0);
+                    s1v = warp_sum(s1v);
+                    s2v = warp_sum(s2v);
+                    s3 = warp_sum(s3);
+                    if (lane == 0) {
+                        row[kR + 0] = s0;
+                        row[kR + 1] = s1v;
+                        row[kR + 2] = s2v;
+                        row[kR + 3] = s3;
+                        if (r < dcc && m0 == 0) {
+                            const int bin = dlist[d0 + r];
+                            atomicAdd(&out.weights_dmat[bin], s0);
+                            atomicAdd(&out.weight_eff[bin], s0);
+                            atomicAdd(&out.z_eff[bin], sz);
+                            atomicAdd(&out.r_trans_eff[bin], sm * ss);
+                        } else if (r >= dcc && d0 == 0 && !veto) {
+                            const int bin = list[m0 + r - dcc];
+                            atomicAdd(&out.dmat[(int64_t)bin * nb + bin], sw1 * sw2 * s0);
+                        }
+                    }
+                }
+                __syncthreads();
+
+                // 4. D = U E^T, added to the global matrix
+                if (tid == 0)
+                    atomicAdd(&scratch->gemm_macs,
+                              (unsigned long long)dcc * (unsigned long long)mcc * (kR + 4));
+                if (c.split)
+                    dm_product_split(U, E, dcc, mcc, kst, digits, rexp, ta_raw, tb_raw,
+                                     dlist + d0, mlist + m0, nb, out.dmat);
+                else
+                    dm_product_fp64(U, E, dcc, mcc, kst, ta, tb, dlist + d0, mlist + m0, nb,
+                                    out.dmat);
+                __syncthreads();
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Delta x quasar distortion matrix: xcf.compute_dmat (py/picca/xcf.py:325-424)
 // and xcf.compute_dmat_forest_pairs_fast (py/picca/xcf.py:427-675). A work
 // item is one forest with up to kXdObjects of its kept quasars. Only the
@@ -1486,8 +2115,28 @@ int dmat_config(const pg_corr_params &p, const pg_dmat_params &d, int p1, int p2
     if (d.product != PG_DMAT_FP64 && d.product != PG_DMAT_SPLIT_BF16) return PG_ERR_INVALID_ARGUMENT;
     const int split = d.product == PG_DMAT_SPLIT_BF16;
     const DmSmem s = dm_smem(p1, p2, mwords, dwords, split, xcf);
-    if (s.total > 220 * 1024) return PG_ERR_UNSUPPORTED;
-    h.smem = s.total;
+    // equal binnings in (r_par, r_trans): cf_dmat_same_kernel, with as many
+    // rows of bins as let two CTAs share an SM or, for long forests, one
+    // (fewer than 32 rows would leave lanes idle: the general form)
+    h.key_rows = h.key_pitch = 0;
+    if (!xcf && !p.rmu_binning && d.num_model_bins_r_par == p.num_bins_r_par &&
+        d.num_model_bins_r_trans == p.num_bins_r_trans && nb <= kDsMaxBins && p1 <= 0xFFFF &&
+        p2 <= 0xFFFF) {
+        const int pitch = ds_pitch(p2);
+        const size_t base = ds_smem(p1, p2, mwords, 0).total, tiles = dm_tile_bytes(split);
+        for (const size_t limit : {kMaxDynSmem / 2, kMaxDynSmem}) {
+            if (base + tiles > limit || h.key_rows) continue;
+            const int64_t rows = std::min<int64_t>(p1, (int64_t)((limit - base) / (2 * pitch)));
+            if (rows < std::min(p1, 32)) continue;
+            h.key_rows = (int)rows;
+            h.key_pitch = pitch;
+            h.smem = base + std::max(tiles, dm_align((size_t)rows * pitch * 2, 16));
+        }
+    }
+    if (!h.key_rows) {
+        if (s.total > 220 * 1024) return PG_ERR_UNSUPPORTED;
+        h.smem = s.total;
+    }
     h.p1 = p1;
     h.p2 = p2;
     h.mwords = mwords;
@@ -1506,11 +2155,13 @@ int dmat_config(const pg_corr_params &p, const pg_dmat_params &d, int p1, int p2
     h.cta_doubles = (int64_t)dm_align((size_t)(h.list_doubles + h.work_doubles + extra), 32);
     h.xcf = xcf;
     int occ = 0;
-    const void *fn = xcf ? (const void *)xcf_dmat_kernel : (const void *)cf_dmat_kernel;
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.total) !=
+    const void *fn = xcf          ? (const void *)xcf_dmat_kernel
+                     : h.key_rows ? (const void *)cf_dmat_same_kernel
+                                  : (const void *)cf_dmat_kernel;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h.smem) !=
         cudaSuccess)
         return PG_ERR_CUDA;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kDmBlock, s.total) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, kDmBlock, h.smem) !=
             cudaSuccess ||
         occ < 1)
         return PG_ERR_CUDA;
@@ -1551,6 +2202,8 @@ static DmatConst dmat_const(const pg_corr_params &p, const pg_dmat_params &d, co
     c.cta_doubles = h.cta_doubles;
     c.split = h.split;
     c.xcf = h.xcf;
+    c.key_rows = h.key_rows;
+    c.key_pitch = h.key_pitch;
     return c;
 }
 
@@ -1562,9 +2215,10 @@ int launch_cf_dmat(const pg_corr_params &p, const pg_dmat_params &d, const DmatC
                    const pg_dmat_sums &out, Scratch *scratch, cudaStream_t stream) {
     if (num_pairs == 0) return PG_OK;
     const DmatConst c = dmat_const(p, d, h);
-    cf_dmat_kernel<<<grid, kDmBlock, h.smem, stream>>>(c, s1, s2, ll1, ll2, order1, order2,
-                                                       pair_first, pair_second, pair_angle,
-                                                       num_pairs, out, work, scratch);
+    const auto kernel = h.key_rows ? cf_dmat_same_kernel : cf_dmat_kernel;
+    kernel<<<grid, kDmBlock, h.smem, stream>>>(c, s1, s2, ll1, ll2, order1, order2, pair_first,
+                                               pair_second, pair_angle, num_pairs, out, work,
+                                               scratch);
     return check_cuda(cudaGetLastError());
 }
 

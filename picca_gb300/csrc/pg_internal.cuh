@@ -246,6 +246,7 @@ struct DmatConstHost {
     int max_grid;
     int split;
     int xcf;
+    int key_rows, key_pitch;  // bins in shared memory (equal binnings), 0: the general form
 };
 // p1 / p2: pixel capacity of the two forests (cross: of the forest; the
 // quasar capacity of a work item is fixed).
