@@ -39,6 +39,7 @@
 #include <algorithm>
 
 #include "pg_internal.cuh"
+#include "pg_tc_common.cuh"
 
 namespace pg {
 namespace {
@@ -76,6 +77,8 @@ struct DmatConst {
     int32_t split;           // 1: tensor-core product (PG_DMAT_SPLIT_BF16)
     int32_t xcf;             // 1: delta x quasar layout (forest, quasar slots)
     int32_t key_rows, key_pitch;  // rows of bins in shared memory (cf_dmat_same_kernel)
+    int32_t key_bytes;            // shared memory of the bins and the product's steps
+    int64_t digit_doubles;        // elements with digits
 };
 
 // Shared-memory layout (bytes), identical on host and device.
@@ -1060,6 +1063,220 @@ __global__ void __launch_bounds__(kDmBlock, 2)
 }
 
 // ---------------------------------------------------------------------------
+// D = U E^T of cf_dmat_same_kernel on the fifth-generation tensor cores: the
+// digits of dm_product_split (six of 8 bits, bf16), exact products of digits
+// summed in FP32 in tensor memory, M = up to 128 model bins, N = up to 32 data
+// bins, six level sums (p + q of the digits) of N columns: 192 of the 256
+// columns of tensor memory that each of an SM's two CTAs holds. A level's sum
+// between two reads (at most 160 steps of six digit pairs of at most 2^14)
+// stays below 2^24 and is an exact integer; it is added to 64-bit integers,
+// level l shifted by 8 (4 - l) bits (of the last level the low 8 bits are
+// rounded away, 2^-10 of what the digit pairs left out can come to), below 2^58
+// for a reduction of 4,096.
+//
+// The digits lie in global memory as the operands' shared-memory image (K-major,
+// 32-byte rows, 32-byte swizzle), per step of 16 and digit, so that one thread
+// brings a step in with a bulk copy per digit, another issues its 21 MMAs, and
+// all read the sums back. Bound: the MMAs' reading of their operands from shared
+// memory (82 cycles of an SM an MMA without the swizzle, about 60 with it; N = 80
+// in two passes of three levels was no faster). 6,200 pairs of 160-pixel forests,
+// 50 x 50 bins: 33 of 53 million cycles a CTA with dm_product_split, 15 of 40
+// here; 27.8 -> 18.6 ms together with the digits formed in stage 3.
+constexpr int kDtCols = 256;     // tensor memory columns of a CTA
+constexpr int kDtGroupsM = 16;   // 8-row groups of an M tile (the MMA's 128 rows)
+constexpr int kDtGroupsN = 4;    // and of an N tile
+constexpr int kDtBlock = 10;     // steps between reads of the sums: 10 x 16 x 6 x 2^14 < 2^24
+constexpr int kDtStages = 4;
+constexpr size_t kDtGroup = 256; // bytes of a group in one digit's image
+constexpr int kDtPadRows = 16;   // rows of digits beyond U and E (two part groups)
+// least shared memory: two steps of the largest tile, from a multiple of 256
+// bytes on (the swizzle goes by the address)
+constexpr size_t kDtMinBytes = 2 * kSlices * (kDtGroupsM + kDtGroupsN) * kDtGroup + 256;
+static_assert(kSlices * kDtGroupsN * 8 <= kDtCols, "tensor memory");
+
+// Operand descriptor: 32-byte swizzle (layout type 6), 256 bytes between groups.
+__device__ __forceinline__ uint64_t dt_desc(uint32_t saddr) {
+    return tc_desc(saddr, 16u, (uint32_t)kDtGroup) | (6ull << 61);
+}
+
+// Byte of element (row, k) in a group's image: the 16-byte halves of rows 4..7
+// are exchanged.
+__device__ __forceinline__ uint32_t dt_offset(int row, int k) {
+    return (uint32_t)(row * 32 + ((((k >> 3) ^ (row >> 2)) & 1) << 4) + (k & 7) * 2);
+}
+
+struct DtSync {
+    uint64_t full[kDtStages], empty[kDtStages], drain;
+    uint32_t tmem;
+};
+
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t r[8]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+          "=r"(r[7])
+        : "r"(taddr));
+}
+
+// Digits of two neighbouring elements with |x| < 2^(ex - 1), as bf16 pairs.
+__device__ __forceinline__ void dt_digits(double x, double y, int ex, uint32_t out[kSlices]) {
+    // bytes of m + 128 in every byte but the top one: digit + 128
+    const long long tx = dm_fixed48(x, ex) + 0x8080808080LL;
+    const long long ty = dm_fixed48(y, ex) + 0x8080808080LL;
+    const uint32_t xl = (uint32_t)tx, yl = (uint32_t)ty;
+    const int xh = (int)(tx >> 32), yh = (int)(ty >> 32);
+    out[0] = dm_bf16_small(xh >> 8) | dm_bf16_small(yh >> 8) << 16;
+#pragma unroll
+    for (int p = 1; p < kSlices; ++p) {
+        const uint32_t sx = p == 1 ? (uint32_t)xh : xl >> (8 * (kSlices - 1 - p));
+        const uint32_t sy = p == 1 ? (uint32_t)yh : yl >> (8 * (kSlices - 1 - p));
+        const float fx = __uint_as_float(0x4B000000u | (sx & 0xFFu)) - 8388736.f;
+        const float fy = __uint_as_float(0x4B000000u | (sy & 0xFFu)) - 8388736.f;
+        out[p] = __byte_perm(__float_as_uint(fx), __float_as_uint(fy), 0x7632);
+    }
+}
+
+constexpr uint32_t kDtDrainPhase = 1u << 31, kDtFailed = 1u << 30;
+
+// Called by the whole CTA, the digits written and fenced for the asynchronous
+// copies (proxy_fence_all and a barrier). am, an: digit images of E (gm groups
+// of 8 rows) and U (gn groups); region: shared memory for the steps. phase:
+// each thread's record of the barriers' phases, kept from call to call, with
+// kDtFailed once a wait ran out (the copies in flight have then landed, as far
+// as a second bounded wait can tell). Not inlined: the caller's values wait on
+// the stack.
+__device__ __noinline__ uint32_t dt_product(const unsigned char *am, const unsigned char *an,
+                                            int dcc, int mcc, int kst, const int32_t *rexp,
+                                            uint32_t region, int region_bytes, DtSync *sync,
+                                            uint32_t phase, const int32_t *dlist,
+                                            const int32_t *mlist, int nm, double *dmat) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int gm = (mcc + 7) >> 3, gn = (dcc + 7) >> 3;
+    const int steps = kst / 16;
+    const uint32_t drain = smem_u32(&sync->drain), tmem = sync->tmem;
+    for (int m0 = 0; m0 < gm; m0 += kDtGroupsM) {
+        const int mg = min(kDtGroupsM, gm - m0);
+        for (int n0 = 0; n0 < gn; n0 += kDtGroupsN) {
+            const int ng = min(kDtGroupsN, gn - n0);
+            const int np = (ng + 1) >> 1, n = 16 * np;  // N is a multiple of 16
+            const uint32_t a_digit = mg * (uint32_t)kDtGroup, b_digit = 2 * np * (uint32_t)kDtGroup;
+            const uint32_t stage_bytes = kSlices * (a_digit + b_digit);
+            const int stages = min(kDtStages, region_bytes / (int)stage_bytes);
+            const uint32_t idesc = tc_idesc(128, n);
+            long long acc[kDtGroupsN / 2][8];
+#pragma unroll
+            for (int b = 0; b < kDtGroupsN / 2; ++b)
+#pragma unroll
+                for (int k = 0; k < 8; ++k) acc[b][k] = 0;
+            int issued = 0;
+            bool ok = true;
+#pragma unroll 1
+            for (int s0 = 0; s0 < steps; s0 += kDtBlock) {
+                const int s1 = min(steps, s0 + kDtBlock);
+                if (tid == 0) {
+                    // copies of this block's steps and of what its MMAs free
+                    for (; issued < min(steps, s1 + stages); ++issued) {
+                        const int st = issued % stages;
+                        const uint32_t full = smem_u32(&sync->full[st]);
+                        if (issued >= stages) {
+                            ok = mbar_wait(smem_u32(&sync->empty[st]), phase >> st & 1u);
+                            phase ^= 1u << st;
+                            if (!ok) break;
+                        }
+                        const uint32_t base = region + st * stage_bytes;
+                        mbar_expect(full, kSlices * (uint32_t)(mg + ng) * (uint32_t)kDtGroup);
+                        for (int p = 0; p < kSlices; ++p) {
+                            const int64_t at = (int64_t)issued * kSlices + p;
+                            bulk_copy(base + p * a_digit, am + (at * gm + m0) * kDtGroup, a_digit,
+                                      full);
+                            bulk_copy(base + kSlices * a_digit + p * b_digit,
+                                      an + (at * gn + n0) * kDtGroup, ng * (uint32_t)kDtGroup,
+                                      full);
+                        }
+                    }
+                } else if (tid == 32) {
+                    for (int s = s0; s < s1; ++s) {
+                        const int st = s % stages;
+                        ok = mbar_wait(smem_u32(&sync->full[st]), phase >> st & 1u);
+                        phase ^= 1u << st;
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint32_t a = region + st * stage_bytes;
+                        const uint32_t b = a + kSlices * a_digit;
+#pragma unroll 1
+                        for (int p = 0; p < kSlices; ++p)
+                            for (int l = p; l < kSlices; ++l)
+                                tc_mma(tmem + l * n, dt_desc(a + p * a_digit),
+                                       dt_desc(b + (l - p) * b_digit), idesc,
+                                       s > s0 || p > 0 ? 1u : 0u);
+                        tc_commit(smem_u32(&sync->empty[st]));
+                    }
+                    if (ok) tc_commit(drain);
+                }
+                __syncwarp();
+                ok = mbar_wait(drain, phase >> 31) && ok;
+                phase ^= kDtDrainPhase;
+                ok = __syncthreads_and(ok) != 0;
+                if (!ok) break;
+                tc_fence_after();
+                if (m0 * 8 + (warp & 3) * 32 < mcc) {
+                    const uint32_t t = tmem + ((uint32_t)(warp & 3) << 21) + (warp >> 2) * 8 * np;
+#pragma unroll
+                    for (int b = 0; b < kDtGroupsN / 2; ++b) {
+                        if (b >= np) break;
+#pragma unroll
+                        for (int l = 0; l < kSlices; ++l) {
+                            uint32_t r[8];
+                            tmem_ld8(t + l * n + 8 * b, r);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                            for (int k = 0; k < 8; ++k) {
+                                const int v = __float2int_rn(__uint_as_float(r[k]));
+                                acc[b][k] += l < 5 ? v * (1LL << (8 * (4 - l))) : (v + 128) >> 8;
+                            }
+                        }
+                    }
+                }
+                tc_fence_before();
+                __syncthreads();
+            }
+            if (tid == 0) {  // the frees nobody waited for
+                for (int s = max(0, issued - stages); s < issued; ++s) {
+                    const int st = s % stages;
+                    if (ok) mbar_wait(smem_u32(&sync->empty[st]), phase >> st & 1u);
+                    phase ^= 1u << st;
+                }
+            }
+            if (!ok) {
+                if (tid == 32)  // the copies in flight, before the memory is given up
+                    for (int st = 0; st < stages; ++st)
+                        mbar_wait(smem_u32(&sync->full[st]), phase >> st & 1u);
+                __syncthreads();
+                return phase | kDtFailed;
+            }
+            const int ml = m0 * 8 + (warp & 3) * 32 + lane;
+            if (ml < mcc) {
+                const int er = rexp[dcc + ml];
+                const int64_t col = mlist[ml];
+#pragma unroll
+                for (int b = 0; b < kDtGroupsN / 2; ++b) {
+                    if (b >= np) break;
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) {
+                        const int dl = n0 * 8 + (warp >> 2) * 8 * np + 8 * b + k;
+                        if (dl >= dcc || acc[b][k] == 0) continue;
+                        // sum_l lev_l 2^(-8 (l + 2)) of |x| < 1/2 rows
+                        atomicAdd(&dmat[(int64_t)dlist[dl] * nm + col],
+                                  ldexp((double)acc[b][k], er + rexp[dl] - 48));
+                    }
+                }
+            }
+        }
+    }
+    return phase;
+}
+
+// ---------------------------------------------------------------------------
 // Equal data and model binning in (r_par, r_trans), the usual matrix: every
 // pixel pair is decided once, in FP32, and its bin kept in shared memory; the
 // few pairs inside a guard band wait in a queue and are decided in FP64 32 at
@@ -1078,7 +1295,9 @@ __global__ void __launch_bounds__(kDmBlock, 2)
 // in stage 3). The form below it (cf_dmat_kernel) decides every pair three
 // times, with FP64 decisions in divergence, and adds 16 numbers a pair in
 // runs whose ends cost 16 more. 6,200 pairs of 160-pixel forests, 50 x 50 bins:
-// 36.4 ms in the general form, 27.8 ms here (sweeps 8 ms of it, they were 25).
+// 36.4 ms in the general form, 27.8 ms with the same product, 18.6 ms now: a
+// third each in the product, in stage 3 and in the rest (8 of 40 million cycles
+// in the sweeps), with U and E of all CTAs (260 MB) larger than L2.
 //
 // Forests whose bins do not fit in shared memory at once go through in strips
 // of rows, decided once more for each strip.
@@ -1114,9 +1333,8 @@ struct DsSmem {
     size_t f1, f2, flags1, flags2, win1, win2, mbits, mpref, dbits, dpref, list, queue, keys, total;
 };
 
-__host__ __device__ inline size_t dm_tile_bytes(int split) {
-    return split ? 4 * sizeof(uint16_t) * kSlices * kTcM * kTcRow
-                 : 2 * sizeof(double) * kSlab * kTilePad;
+__host__ __device__ inline size_t ds_tile_bytes(int split) {
+    return split ? kDtMinBytes : 2 * sizeof(double) * kSlab * kTilePad;
 }
 
 __host__ __device__ inline DsSmem ds_smem(int p1, int p2, int words, size_t key_bytes) {
@@ -1193,11 +1411,10 @@ __global__ void __launch_bounds__(kDmBlock, 2)
     uint16_t *keys = reinterpret_cast<uint16_t *>(smem + L.keys);
     double (*ta)[kTilePad] = reinterpret_cast<double (*)[kTilePad]>(smem + L.keys);
     double (*tb)[kTilePad] = ta + kSlab;
-    uint16_t *ta_raw = reinterpret_cast<uint16_t *>(smem + L.keys);
-    uint16_t *tb_raw = ta_raw + 2 * kSlices * kTcM * kTcRow;
     __shared__ double red[kDmWarps];
     __shared__ int red_int[kDmWarps];
     __shared__ int s_item, s_count, s_veto, s_queue;
+    __shared__ DtSync s_sync;
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nb = c.b.nbins;
@@ -1206,14 +1423,35 @@ __global__ void __launch_bounds__(kDmBlock, 2)
     int32_t *mlist = dlist + nb;                         // [nb]
     double *rows = cta + c.list_doubles;
     uint16_t *digits = reinterpret_cast<uint16_t *>(rows + c.work_doubles);
-    int32_t *rexp = reinterpret_cast<int32_t *>(digits + (c.work_doubles * kSlices));
+    int32_t *rexp = reinterpret_cast<int32_t *>(digits + (c.digit_doubles * kSlices));
     const int pitch = c.key_pitch;
+    uint32_t phase = 0;
+    if (c.split) {
+        if (tid == 0) {
+            for (int st = 0; st < kDtStages; ++st) {
+                mbar_init(smem_u32(&s_sync.full[st]), 1);
+                mbar_init(smem_u32(&s_sync.empty[st]), 1);
+            }
+            mbar_init(smem_u32(&s_sync.drain), 1);
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        }
+        if (warp == 0) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                             smem_u32(&s_sync.tmem)),
+                         "r"(kDtCols)
+                         : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+    }
 
     for (;;) {
         if (tid == 0) s_item = atomicAdd(&scratch->work_counter, 1);
         __syncthreads();
         const int64_t q = s_item;
-        if (q >= num_pairs) break;
+        if (q >= num_pairs || (phase & kDtFailed)) break;
         const int f = pair_first[q], g = pair_second[q];
         const int64_t o1 = s1.pix_offset[f], o2 = s2.pix_offset[g];
         const int n1 = (int)(s1.pix_offset[f + 1] - o1);
@@ -1602,73 +1840,126 @@ __global__ void __launch_bounds__(kDmBlock, 2)
                     __syncthreads();
                 }
 
-                // 3. rank rows and effective sums; blocks of zeros are passed over
-                for (int r = warp; r < dcc + mcc; r += kDmWarps) {
+                // 3. rank rows, effective sums and (split) the digits: eight rows
+                // a warp, four lanes a row and two elements a lane
+                const int gn = (dcc + 7) >> 3, gm = (mcc + 7) >> 3;
+                unsigned char *img_m = reinterpret_cast<unsigned char *>(digits);
+                unsigned char *img_n = img_m + (size_t)gm * kst / 16 * kSlices * kDtGroup;
+                for (int grp = warp; grp < gn + gm; grp += kDmWarps) {
+                    const bool is_u = grp < gn;
+                    const int g0 = is_u ? grp : grp - gn;
+                    const int rl = g0 * 8 + (lane >> 2), r = is_u ? rl : dcc + rl;
+                    const bool live = rl < (is_u ? dcc : mcc);
                     double *row = rows + (int64_t)r * kst;
+                    const bool extra = m0 == 0;
                     double s0 = 0., s1v = 0., s2v = 0., s3 = 0., sz = 0., sm = 0.;
-                    if (r < dcc) {
-                        for (int b = 0; b < n1; b += 32) {
-                            const int i = b + lane;
-                            const double x = i < n1 ? __ldcg(row + kU + i) : 0.;
-                            const double y = ord1 && ord2 && i < n1 ? __ldcg(row + kV + i) : 0.;
-                            if (!__any_sync(0xffffffffu, x != 0. || y != 0.) || i >= n1) continue;
-                            s0 = __fma_rn(P1.iz[i], x, s0);
-                            s2v = __fma_rn(P1.diz[i], x, s2v);
-                            if (ord1 && ord2) s3 = __fma_rn(P1.diz[i], y, s3);
-                            if (m0 == 0) {
-                                sz = __fma_rn(P1.ziz[i], x, sz);
-                                sm = __fma_rn(P1.miz[i], x, sm);
+                    unsigned mx = 0;
+                    auto add = [&](int k, double x) {
+                        if (is_u) {
+                            if (k < kX) {
+                                s0 = __fma_rn(P1.iz[k], x, s0);
+                                s2v = __fma_rn(P1.diz[k], x, s2v);
+                                if (extra) {
+                                    sz = __fma_rn(P1.ziz[k], x, sz);
+                                    sm = __fma_rn(P1.miz[k], x, sm);
+                                }
+                            } else if (k < kV) {
+                                s1v = __fma_rn(P2.diz[k - kX], x, s1v);
+                                if (extra) {
+                                    sz = __fma_rn(P2.ziz[k - kX], x, sz);
+                                    sm = __fma_rn(P2.miz[k - kX], x, sm);
+                                }
+                            } else if (k < kY && ord1) {
+                                s3 = __fma_rn(P1.diz[k - kV], x, s3);
                             }
+                        } else if (k < kX) {
+                            s0 = __fma_rn(-P1.a[k], x, s0);
+                            if (ord1) s2v = __fma_rn(-P1.b[k], x, s2v);
+                        } else if (k >= kV && k < kY) {
+                            s1v = __fma_rn(-P1.a[k - kV], x, s1v);
+                            if (ord1) s3 = __fma_rn(-P1.b[k - kV], x, s3);
                         }
-                        for (int b = 0; b < n2; b += 32) {
-                            const int j = b + lane;
-                            const double x = j < n2 ? __ldcg(row + kX + j) : 0.;
-                            if (!__any_sync(0xffffffffu, x != 0.) || j >= n2) continue;
-                            s1v = __fma_rn(P2.diz[j], x, s1v);
-                            if (m0 == 0) {
-                                sz = __fma_rn(P2.ziz[j], x, sz);
-                                sm = __fma_rn(P2.miz[j], x, sm);
-                            }
+                    };
+                    constexpr int kBatch = 8;
+                    for (int k0 = 2 * (lane & 3); k0 < kst; k0 += 8 * kBatch) {
+                        double2 v[kBatch];
+#pragma unroll
+                        for (int c8 = 0; c8 < kBatch; ++c8) {
+                            const int k = k0 + 8 * c8;
+                            v[c8] = live && k < kst ? __ldcg(reinterpret_cast<double2 *>(row + k))
+                                                    : make_double2(0., 0.);
                         }
-                        if (m0 == 0) {
-                            sz = warp_sum(sz);
-                            sm = warp_sum(sm);
-                        }
-                    } else {
-                        for (int b = 0; b < n1; b += 32) {
-                            const int i = b + lane;
-                            const double x = i < n1 ? __ldcg(row + kU + i) : 0.;
-                            const double y = ord2 && i < n1 ? __ldcg(row + kV + i) : 0.;
-                            if (!__any_sync(0xffffffffu, x != 0. || y != 0.) || i >= n1) continue;
-                            s0 = __fma_rn(-P1.a[i], x, s0);
-                            if (ord2) s1v = __fma_rn(-P1.a[i], y, s1v);
-                            if (ord1) {
-                                s2v = __fma_rn(-P1.b[i], x, s2v);
-                                if (ord2) s3 = __fma_rn(-P1.b[i], y, s3);
-                            }
+#pragma unroll
+                        for (int c8 = 0; c8 < kBatch; ++c8) {
+                            const unsigned hx = __double2hiint(v[c8].x) & 0x7FFFFFFF;
+                            const unsigned hy = __double2hiint(v[c8].y) & 0x7FFFFFFF;
+                            if ((hx | hy) == 0u) continue;
+                            mx = max(mx, max(hx, hy));
+                            add(k0 + 8 * c8, v[c8].x);
+                            add(k0 + 8 * c8 + 1, v[c8].y);
                         }
                     }
-                    s0 = warp_sum(s0);
-                    s1v = warp_sum(s1v);
-                    s2v = warp_sum(s2v);
-                    s3 = warp_sum(s3);
-                    if (lane == 0) {
+                    __syncwarp();
+#pragma unroll
+                    for (int o = 1; o < 4; o <<= 1) {
+                        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+                        s1v += __shfl_xor_sync(0xffffffffu, s1v, o);
+                        s2v += __shfl_xor_sync(0xffffffffu, s2v, o);
+                        s3 += __shfl_xor_sync(0xffffffffu, s3, o);
+                        sz += __shfl_xor_sync(0xffffffffu, sz, o);
+                        sm += __shfl_xor_sync(0xffffffffu, sm, o);
+                        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+                    }
+                    if (live && (lane & 3) == 0) {
                         row[kR + 0] = s0;
                         row[kR + 1] = s1v;
                         row[kR + 2] = s2v;
                         row[kR + 3] = s3;
-                        if (r < dcc && m0 == 0) {
-                            const int bin = dlist[d0 + r];
+                        if (is_u && m0 == 0) {
+                            const int bin = dlist[d0 + rl];
                             atomicAdd(&out.weights_dmat[bin], s0);
                             atomicAdd(&out.weight_eff[bin], s0);
                             atomicAdd(&out.z_eff[bin], sz);
                             atomicAdd(&out.r_trans_eff[bin], sm * ss);
-                        } else if (r >= dcc && d0 == 0 && !veto) {
-                            const int bin = list[m0 + r - dcc];
+                        } else if (!is_u && d0 == 0 && !veto) {
+                            const int bin = list[m0 + rl];
                             atomicAdd(&out.dmat[(int64_t)bin * nb + bin], sw1 * sw2 * s0);
                         }
                     }
+                    if (!c.split) continue;
+                    mx = max(mx, (unsigned)__double2hiint(s0) & 0x7FFFFFFFu);
+                    mx = max(mx, (unsigned)__double2hiint(s1v) & 0x7FFFFFFFu);
+                    mx = max(mx, (unsigned)__double2hiint(s2v) & 0x7FFFFFFFu);
+                    mx = max(mx, (unsigned)__double2hiint(s3) & 0x7FFFFFFFu);
+                    const int ex = (int)(mx >> 20);
+                    const int e = (ex == 0 ? -1022 : ex - 1022) + 1;  // |x| < 2^(e - 1)
+                    if (live && (lane & 3) == 0) rexp[r] = e;
+                    __syncwarp();
+                    unsigned char *img = (is_u ? img_n : img_m) + g0 * kDtGroup;
+                    const size_t digit = (size_t)(is_u ? gn : gm) * kDtGroup;
+                    for (int k0 = 2 * (lane & 3); k0 < kst; k0 += 8 * kBatch) {
+                        double2 v[kBatch];
+#pragma unroll
+                        for (int c8 = 0; c8 < kBatch; ++c8) {
+                            const int k = k0 + 8 * c8;
+                            v[c8] = live && k < kst ? __ldcg(reinterpret_cast<double2 *>(row + k))
+                                                    : make_double2(0., 0.);
+                        }
+#pragma unroll
+                        for (int c8 = 0; c8 < kBatch; ++c8) {
+                            const int k = k0 + 8 * c8;
+                            if (k >= kst) break;
+                            uint32_t d[kSlices];
+                            dt_digits(v[c8].x, v[c8].y, e, d);
+                            unsigned char *dst = img + (size_t)(k >> 4) * kSlices * digit +
+                                                 dt_offset(lane >> 2, k);
+#pragma unroll
+                            for (int p = 0; p < kSlices; ++p)
+                                *reinterpret_cast<uint32_t *>(dst + p * digit) = d[p];
+                        }
+                    }
                 }
+                proxy_fence_all();
                 __syncthreads();
 
                 // 4. D = U E^T, added to the global matrix
@@ -1676,13 +1967,30 @@ __global__ void __launch_bounds__(kDmBlock, 2)
                     atomicAdd(&scratch->gemm_macs,
                               (unsigned long long)dcc * (unsigned long long)mcc * (kR + 4));
                 if (c.split)
-                    dm_product_split(U, E, dcc, mcc, kst, digits, rexp, ta_raw, tb_raw,
-                                     dlist + d0, mlist + m0, nb, out.dmat);
+                    phase = dt_product(img_m, img_n, dcc, mcc, kst, rexp,
+                                       (smem_u32(keys) + 255u) & ~255u, c.key_bytes - 256,
+                                       &s_sync, phase, dlist + d0, mlist + m0, nb, out.dmat);
                 else
                     dm_product_fp64(U, E, dcc, mcc, kst, ta, tb, dlist + d0, mlist + m0, nb,
                                     out.dmat);
                 __syncthreads();
+                if (phase & kDtFailed) {
+                    if (tid == 0) report_error(scratch, PG_ERR_TIMEOUT, (int32_t)q);
+                    d0 = nbt;
+                    break;
+                }
             }
+        }
+    }
+    if (c.split) {
+        tc_fence_before();
+        __syncthreads();
+        if (warp == 0) {
+            tc_fence_after();
+            asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(
+                             s_sync.tmem),
+                         "r"(kDtCols)
+                         : "memory");
         }
     }
 }
@@ -2118,19 +2426,20 @@ int dmat_config(const pg_corr_params &p, const pg_dmat_params &d, int p1, int p2
     // equal binnings in (r_par, r_trans): cf_dmat_same_kernel, with as many
     // rows of bins as let two CTAs share an SM or, for long forests, one
     // (fewer than 32 rows would leave lanes idle: the general form)
-    h.key_rows = h.key_pitch = 0;
+    h.key_rows = h.key_pitch = h.key_bytes = 0;
     if (!xcf && !p.rmu_binning && d.num_model_bins_r_par == p.num_bins_r_par &&
         d.num_model_bins_r_trans == p.num_bins_r_trans && nb <= kDsMaxBins && p1 <= 0xFFFF &&
         p2 <= 0xFFFF) {
         const int pitch = ds_pitch(p2);
-        const size_t base = ds_smem(p1, p2, mwords, 0).total, tiles = dm_tile_bytes(split);
+        const size_t base = ds_smem(p1, p2, mwords, 0).total, tiles = ds_tile_bytes(split);
         for (const size_t limit : {kMaxDynSmem / 2, kMaxDynSmem}) {
             if (base + tiles > limit || h.key_rows) continue;
             const int64_t rows = std::min<int64_t>(p1, (int64_t)((limit - base) / (2 * pitch)));
             if (rows < std::min(p1, 32)) continue;
             h.key_rows = (int)rows;
             h.key_pitch = pitch;
-            h.smem = base + std::max(tiles, dm_align((size_t)rows * pitch * 2, 16));
+            h.key_bytes = (int)std::max(tiles, dm_align((size_t)rows * pitch * 2, 16));
+            h.smem = base + h.key_bytes;
         }
     }
     if (!h.key_rows) {
@@ -2150,7 +2459,8 @@ int dmat_config(const pg_corr_params &p, const pg_dmat_params &d, int p1, int p2
     h.list_doubles = (int64_t)dm_align((size_t)(nb + nm), 32) / 2;
     h.work_doubles = rows * kcap;
     // tensor-core form: six bf16 digits per element and one exponent per row
-    const int64_t extra = split ? h.work_doubles * kSlices / 4 + h.work_doubles / 32 : 0;
+    h.digit_doubles = h.work_doubles + (h.key_rows ? kDtPadRows * kcap : 0);
+    const int64_t extra = split ? h.digit_doubles * kSlices / 4 + h.work_doubles / 32 : 0;
     h.split = split;
     h.cta_doubles = (int64_t)dm_align((size_t)(h.list_doubles + h.work_doubles + extra), 32);
     h.xcf = xcf;
@@ -2165,6 +2475,9 @@ int dmat_config(const pg_corr_params &p, const pg_dmat_params &d, int p1, int p2
             cudaSuccess ||
         occ < 1)
         return PG_ERR_CUDA;
+    // the occupancy of a kernel with tensor memory is reported as one CTA; two
+    // fit where their shared memory does (kDtCols columns each, 128 registers)
+    if (h.key_rows && split) occ = h.smem <= kMaxDynSmem / 2 ? 512 / kDtCols : 1;
     h.max_grid = num_sms * occ;
     return PG_OK;
 }
@@ -2204,6 +2517,8 @@ static DmatConst dmat_const(const pg_corr_params &p, const pg_dmat_params &d, co
     c.xcf = h.xcf;
     c.key_rows = h.key_rows;
     c.key_pitch = h.key_pitch;
+    c.key_bytes = h.key_bytes;
+    c.digit_doubles = h.digit_doubles;
     return c;
 }
 

@@ -246,7 +246,8 @@ struct DmatConstHost {
     int max_grid;
     int split;
     int xcf;
-    int key_rows, key_pitch;  // bins in shared memory (equal binnings), 0: the general form
+    int key_rows, key_pitch, key_bytes;  // bins in shared memory (equal binnings); 0: general form
+    int64_t digit_doubles;               // elements with digits
 };
 // p1 / p2: pixel capacity of the two forests (cross: of the forest; the
 // quasar capacity of a work item is fixed).

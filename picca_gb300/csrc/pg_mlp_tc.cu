@@ -23,6 +23,7 @@
 
 #include "pg_cont_common.cuh"
 #include "pg_internal.cuh"
+#include "pg_tc_common.cuh"
 
 namespace pg {
 namespace {
@@ -42,50 +43,6 @@ constexpr int64_t kPackW2 = (int64_t)kHidden * kHidden;
 constexpr int64_t kPackW4 = (int64_t)kOutPad * kHidden;
 constexpr int64_t kPackTotal = kPackW1 + 2 * kPackW2 + kPackW4;
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-    return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-// shared-memory matrix descriptor: start, leading and stride byte offsets
-// (16-byte units), descriptor version 1, no swizzle
-__device__ __forceinline__ uint64_t tc_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
-}
-
-// instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both
-// K-major, N >> 3 and M >> 4
-__host__ __device__ constexpr uint32_t tc_idesc(int m, int n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
-           ((uint32_t)(m >> 4) << 24);
-}
-
-__device__ __forceinline__ void tc_mma(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
-                                       uint32_t accumulate) {
-    asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-        "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
-}
-
-__device__ __forceinline__ void tc_commit(uint32_t mbar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::
-                     "r"(mbar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() {
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-
-__device__ __forceinline__ void tc_fence_after() {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-
-__device__ __forceinline__ void proxy_fence() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
 // 16-byte global -> shared copy through the asynchronous copy path;
 // src_bytes = 0 fills the 16 bytes with zeros (nothing is read)
 __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc, uint32_t src_bytes) {
@@ -96,21 +53,6 @@ __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc, uin
 
 __device__ __forceinline__ void cp_async_wait_all() {
     asm volatile("cp.async.wait_all;" ::: "memory");
-}
-
-// bounded wait on an mbarrier phase; false when the bound ran out
-__device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
-    for (int i = 0; i < (1 << 20); ++i) {
-        uint32_t done;
-        asm volatile(
-            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            "selp.u32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(mbar), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
-    return false;
 }
 
 // 32 consecutive FP32 columns of this thread's TMEM lane

@@ -43,3 +43,15 @@ def test_strips(cuda, monkeypatch):
     monkeypatch.setattr(base, "_synthetic", _long)
     assert np.diff(_long().pix_offset).max() > 400
     base.test_synthetic_matches_oracle(cuda, "long")
+
+
+def test_row_counts(cuda, monkeypatch):
+    """Numbers of touched bins around the product's tiles of 32 and 128 rows
+    (row chunks of 17 to 300 for a pair's few hundred bins)."""
+    from picca_gb300 import dmat
+    make = dmat.make_dmat_params
+    for capacity in (34, 66, 130, 258, 600):
+        monkeypatch.setitem(base.CASES, "rows", dict(CASES["fine"], nt=40, reject=0.985))
+        monkeypatch.setattr(dmat, "make_dmat_params", lambda *a, **k: make(
+            *a, **dict(k, row_capacity=capacity, product="split_bf16")))
+        base.test_synthetic_matches_oracle(cuda, "rows")
