@@ -61,13 +61,13 @@
 namespace pg {
 namespace {
 
-constexpr int kQueue = 256;                   // FP64 recheck entries per warp (cross)
+constexpr int kQueue = 96;                    // FP64 recheck entries per warp (cross)
 constexpr int kCfQueue = 96;                  // FP64 recheck entries per warp (auto)
 constexpr int kAccQ = 64;                     // run ring per warp (<= 31 + 32 entries held)
 constexpr int kChunk = 128;                   // forest-2 pixels staged per warp at a time
 constexpr int kRunMax = 64;                   // pairs summed in FP32 registers per run
 constexpr int kCfBlock = 640;
-constexpr int kXcfBlock = 512;
+constexpr int kXcfBlock = 704;
 
 // ---------------------------------------------------------------------------
 // shared-memory histograms: H_COUNT float arrays of stride hstride
@@ -852,6 +852,11 @@ __device__ __forceinline__ void xcf_drain(const Binning &b, const FastConst *__r
 // outside the accepted ranges, so the reference rejects them too. Pairs
 // within the guard band of an edge or a cut are re-decided in FP64
 // (xcf_drain).
+//
+// Bound: issue, a third of it in the runs' adds to shared memory (a run is two
+// pixels long at 2 Mpc/h a pixel). 9,000 forests x 13,500 quasars: 10.3 ms with
+// 16 warps and groups dealt out in turn, 10.1 ms with groups drawn, 9.4 ms with
+// the 22 warps that smaller queues leave room for (20 warps 9.5 ms, 24 no better).
 template <bool EXTRA>
 __global__ void __launch_bounds__(kXcfBlock, 1) xcf_xi_fast_kernel(
     const __grid_constant__ Binning b, const FastConst *__restrict__ fcp,
@@ -862,6 +867,7 @@ __global__ void __launch_bounds__(kXcfBlock, 1) xcf_xi_fast_kernel(
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int item_slot;
     __shared__ unsigned max_rho_bits;
+    __shared__ int next_task;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int nwarps = blockDim.x >> 5;
@@ -872,6 +878,7 @@ __global__ void __launch_bounds__(kXcfBlock, 1) xcf_xi_fast_kernel(
     const float h_tr = fcp->h_tr;
     const unsigned np = fcp->np, nt = fcp->nt;
     const int hs = fcp->hstride;
+    if (threadIdx.x == 0) next_task = 0;  // seen by all after next_item's barrier
     // accepted range of p with one bin of margin each side, and of x_tr'
     const float p_lo = (pc - 0.5f) - 1.f, p_hi = (pc - 0.5f) + (float)np + 1.f;
     const float t_end = (float)nt + 1.f;
@@ -945,7 +952,18 @@ __global__ void __launch_bounds__(kXcfBlock, 1) xcf_xi_fast_kernel(
         }
         int head = 0, tail = 0;  // run ring of this warp (warp-uniform)
         int qn = 0;              // FP64 re-decision queue of this warp
-        for (int kb = warp * 32; kb < nq; kb += nwarps * 32) {
+        // groups of 32 quasars, drawn by the warps; where there are fewer than
+        // warps, each in up to four parts of its pixels (a part repeats the
+        // group's set-up, a sixth of its time)
+        const int groups = (nq + 31) >> 5;
+        int parts = 1;
+        while (parts < 4 && groups * parts < nwarps) parts *= 2;
+        for (;;) {
+            int task = 0;
+            if (lane == 0) task = atomicAdd(&next_task, 1);
+            task = __shfl_sync(0xffffffffu, task, 0);
+            if (task >= groups * parts) break;
+            const int kb = (task / parts) * 32, part = task % parts;
             const int kk = kb + lane < nq ? (by_distance ? (int)qorder[kb + lane] : kb + lane) : nq;
             float cp = 1.f, st = 0.f, nb = kFar, nbl = 0.f, t = kFar, zv = kFar;
             float wvh = 0.f, wvl = 0.f;
@@ -1025,6 +1043,12 @@ __global__ void __launch_bounds__(kXcfBlock, 1) xcf_xi_fast_kernel(
                 g_hi = max(g_hi, __shfl_xor_sync(0xffffffffu, g_hi, o));
             }
             if (g_lo >= g_hi) continue;
+            if (parts > 1) {
+                const int len = (g_hi - g_lo + parts - 1) / parts;
+                g_lo += part * len;
+                g_hi = min(g_hi, g_lo + len);
+                ib = min(ib, g_hi);  // the odd pixel past the part is the next part's
+            }
             unsigned run_bin = 0xFFFFFFFFu;
             int run_n = 0;
             float r_xi = 0.f, r_xil = 0.f, r_w = 0.f, r_pw = 0.f, r_tw = 0.f, r_zw = 0.f;
@@ -1113,7 +1137,7 @@ __global__ void __launch_bounds__(kXcfBlock, 1) xcf_xi_fast_kernel(
             for (int i = g_lo; i < g_hi; i += 2) {
                 PairEval ea, eb;
                 eval(i, ea);
-                eval(i + 1, eb);  // i + 1 = g_hi: outside every lane's range
+                eval(i + 1, eb);
                 take(ea, i);
                 take(eb, i + 1);
                 if (__any_sync(0xffffffffu, ea.near | eb.near)) {
@@ -1148,7 +1172,10 @@ __global__ void __launch_bounds__(kXcfBlock, 1) xcf_xi_fast_kernel(
         if (tail != head) apply_runs<false>(acc0, acc1, head, tail - head, h, hs);
         __syncthreads();
         flush_rows(h, *fcp, out, row);
-        if (threadIdx.x == 0) atomicAdd(&scratch->work_items, 1ull);
+        if (threadIdx.x == 0) {
+            next_task = 0;
+            atomicAdd(&scratch->work_items, 1ull);
+        }
     }
     if (lane == 0) {
         atomicAdd(&scratch->rechecked_pairs, rechecks);
