@@ -209,6 +209,12 @@ int launch_cf_xi_runs64(const Binning &b, const pg_forest_set &s1, const pg_fore
                         const double *nbr_angle, const int32_t *work_order, int64_t num_work,
                         const pg_xi_rows &out, Scratch *scratch, int num_sms,
                         cudaStream_t stream);
+bool xruns64_covers(const Binning &b, const pg_forest_set &fs, int64_t num_work);
+int launch_xcf_xi_runs64(const Binning &b, const pg_forest_set &fs, const pg_forest_set &objs,
+                         const int64_t *nbr_offsets, const int32_t *nbr_index,
+                         const double *nbr_angle, const int32_t *work_order, int64_t num_work,
+                         const pg_xi_rows &out, Scratch *scratch, int num_sms,
+                         cudaStream_t stream);
 int launch_xcf_xi_fp64(const Binning &b, const pg_forest_set &forests, const pg_forest_set &objs,
                        const int64_t *nbr_offsets, const int32_t *nbr_index, const double *nbr_angle,
                        const int32_t *work_order, int64_t num_work, const pg_xi_rows &out,

@@ -1,6 +1,6 @@
 // Plain all-FP64 pair accumulation (the "plain GPU drop-in" form): the
-// angular and r-mu binnings, forests too long for the shared memory of
-// pg_pairs_runs64.cu, and the correlation with quasars.
+// angular and r-mu binnings and forests too long for the shared memory of
+// pg_pairs_runs64.cu.
 //
 // Persistent kernel: each CTA pops a work item (one forest of set 1 with all
 // of its neighbours) from a global counter, accumulates every pixel pair in
@@ -303,6 +303,9 @@ int launch_xcf_xi_fp64(const Binning &b, const pg_forest_set &forests, const pg_
                        const int32_t *work_order, int64_t num_work, const pg_xi_rows &out,
                        Scratch *scratch, int num_sms, cudaStream_t stream) {
     if (num_work <= 0) return PG_OK;
+    if (xruns64_covers(b, forests, num_work))
+        return launch_xcf_xi_runs64(b, forests, objs, nbr_offsets, nbr_index, nbr_angle,
+                                    work_order, num_work, out, scratch, num_sms, stream);
     const size_t smem = hist64_bytes(b.nbins);
     int grid = 0, rc;
     if (smem <= 220 * 1024) {
