@@ -67,6 +67,7 @@ constexpr int kAccQ = 64;                     // run ring per warp (<= 31 + 32 e
 constexpr int kChunk = 128;                   // forest-2 pixels staged per warp at a time
 constexpr int kRunMax = 64;                   // pairs summed in FP32 registers per run
 constexpr int kCfBlock = 640;
+constexpr int kCfParts = 8;                   // parts of a neighbour where there are few (auto)
 constexpr int kXcfBlock = 704;
 
 // ---------------------------------------------------------------------------
@@ -337,7 +338,9 @@ __host__ __device__ inline CfSmem cf_smem(int nbins, int max_pix1, int nwarps) {
 // re-decided in FP64. Runs along diagonals work as before: r and mu change
 // slowly along a diagonal. The r_par histogram sums mu w, the r_trans one
 // r w in r-bin units.
-template <bool AUTO, bool EXTRA, bool LOWX, bool RMU>
+// FEW: few forests, whose neighbours are shared out over `slices` CTAs and, in
+// parts, over the warps.
+template <bool AUTO, bool EXTRA, bool LOWX, bool RMU, bool FEW>
 __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
     const __grid_constant__ Binning b, const FastConst *__restrict__ fcp,
     const __grid_constant__ pg_forest_set s1, const __grid_constant__ pg_forest_set s2,
@@ -389,16 +392,23 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
 
     for (;;) {
         const int unit = next_item(scratch, &item_slot, &max_rho_bits);
-        if (unit >= num_work * slices) break;
-        const int item = unit / slices, slice = unit - item * slices;
+        if (unit >= (FEW ? num_work * slices : num_work)) break;
+        const int item = FEW ? unit / slices : unit, slice = FEW ? unit - item * slices : 0;
         const int64_t f1 = work_order ? work_order[item] : item;
         const int32_t row = s1.row[f1];
-        // this slice's neighbours: a slice keeps every warp busy for at
-        // least two of them
+        // this slice's neighbours, each in up to kCfParts parts of its
+        // diagonals so that a slice has at least two tasks for every warp (a
+        // part stages the neighbour again; the runs stay whole)
         const int64_t k0 = nbr_offsets[f1], nk = nbr_offsets[f1 + 1] - k0;
-        const int cut = (int)max((int64_t)1, min((int64_t)slices, nk / (2 * nwarps)));
-        if (slice >= cut) continue;
-        const int64_t k_lo = k0 + nk * slice / cut, k1 = k0 + nk * (slice + 1) / cut;
+        int64_t k_lo = k0, k1 = k0 + nk;
+        int part_bits = 0;
+        if (FEW) {
+            const int cut = (int)max((int64_t)1, min((int64_t)slices, nk * kCfParts / (2 * nwarps)));
+            if (slice >= cut) continue;
+            k_lo = k0 + nk * slice / cut;
+            k1 = k0 + nk * (slice + 1) / cut;
+            while (1 << part_bits < kCfParts && (k1 - k_lo) << part_bits < 2 * nwarps) ++part_bits;
+        }
         const int64_t a0 = s1.pix_offset[f1];
         const int64_t n1_64 = s1.pix_offset[f1 + 1] - a0;
         if (n1_64 > max_pix1 || n1_64 > 65535 || n1_64 < 1) {
@@ -412,7 +422,7 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
             f1_geom[0] = s1.x_cart[f1]; f1_geom[1] = s1.y_cart[f1]; f1_geom[2] = s1.z_cart[f1];
             f1_geom[3] = s1.ra[f1]; f1_geom[4] = s1.dec[f1]; f1_geom[5] = s1.cos_dec[f1];
             f1_geom[6] = s1.z_qso[f1];
-            nbr_next = k_lo;
+            nbr_next = k_lo << part_bits;
         }
         const bool sorted1 = stage_forest1(s1, a0, n1, r_ref, const_cast<float4 *>(p1),
                                            const_cast<float4 *>(p1x), &max_rho_bits);
@@ -432,7 +442,10 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
             int64_t k = 0;
             if (lane == 0) k = (int64_t)atomicAdd((unsigned long long *)&nbr_next, 1ull);
             k = __shfl_sync(0xffffffffu, k, 0);
-            if (k >= k1) break;
+            if (k >= k1 << part_bits) break;
+            const int d_first = FEW ? 32 * ((int)k & ((1 << part_bits) - 1)) : 0;
+            const int d_step = FEW ? 32 << part_bits : 32;
+            if (FEW) k >>= part_bits;
             const int64_t g = nbr_index[k];
             const int64_t b0 = s2.pix_offset[g];
             const int64_t n2_64 = s2.pix_offset[g + 1] - b0;
@@ -560,15 +573,16 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
                         lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
                         hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
                     }
-                    d_lo = lo;
-                    d_hi = hi;
+                    d_lo = lo < hi ? lo : 0;
+                    d_hi = lo < hi ? hi : 0;
                 }
                 // along a diagonal x_tr' is non-decreasing: trim at t_end
                 const bool t_trim = sorted1 && ordered_t && valid2 && st > 0.f;
                 // no pixel without weight on either side and no negative
                 // r_trans: no test for them per pair
                 const bool plain = plain1 && plain2 && valid2 && st >= 0.f;
-                for (int d0 = d_lo; d0 < d_hi; d0 += 32) {
+                // this part's share of the groups of 32 diagonals
+                for (int d0 = d_lo + d_first; d0 < d_hi; d0 += d_step) {
                     const int d = d0 + lane;
                     // this lane's pairs: j = i + d in the chunk, i in forest 1
                     int ia = max(0, jc - d), ib = min(n1, jc + jn - d);
@@ -1238,18 +1252,24 @@ int launch_cf_xi_fast(const Binning &b, double ang_max, const pg_forest_set &s1,
     const bool lowx = autoc && b.r_par_min == 0.0;
     int grid = 0;
     // few forests: several CTAs share one, each with a slice of its
-    // neighbours, of at least two per warp (a slice costs a staging and a
-    // flush). 150 forests: 1.32 ms for the kernel with whole forests, 0.98 ms so;
-    // eight slices without that minimum left warps idle (1.85 ms)
+    // neighbours (a slice costs a staging and a flush), and few neighbours are
+    // cut into parts for the warps. 150 forests: 1.32 ms for the kernel with whole
+    // forests, 0.96 ms in up to four slices of whole neighbours, 0.86 ms with up
+    // to eight parts (four parts 0.91 ms). Parts of the pixels instead of the
+    // diagonals, 0.83 ms, cut the runs and so round their FP32 sums otherwise.
+    // A kernel of its own (FEW): the parts cost the sweeps of many forests 0.8 %
     int slices = 1;
     while (slices < 4 && num_work * slices < 4 * (int64_t)num_sms) slices *= 2;
-#define PG_LAUNCH_CF(A, E, L, R)                                                               \
-    rc = persistent_grid(cf_xi_diag_kernel<A, E, L, R>, block, smem, num_sms,                  \
+#define PG_LAUNCH_CF_F(A, E, L, R, F)                                                           \
+    rc = persistent_grid(cf_xi_diag_kernel<A, E, L, R, F>, block, smem, num_sms,               \
                          num_work * slices, &grid, tuning.blocks_per_sm);                      \
     if (rc) return rc;                                                                         \
-    cf_xi_diag_kernel<A, E, L, R><<<grid, block, smem, stream>>>(                              \
+    cf_xi_diag_kernel<A, E, L, R, F><<<grid, block, smem, stream>>>(                           \
         b, fc, s1, s2, nbr_offsets, nbr_index, nbr_angle, work_order, num_work, slices, out,   \
         scratch, max_pix1);
+#define PG_LAUNCH_CF(A, E, L, R)                                                               \
+    if (slices > 1) { PG_LAUNCH_CF_F(A, E, L, R, true) }                                       \
+    else { PG_LAUNCH_CF_F(A, E, L, R, false) }
     if (b.rmu) {
         if (autoc && lowx) { PG_LAUNCH_CF(true, false, true, true) }
         else if (autoc) { PG_LAUNCH_CF(true, false, false, true) }
@@ -1262,6 +1282,7 @@ int launch_cf_xi_fast(const Binning &b, double ang_max, const pg_forest_set &s1,
     else if (!extra) { PG_LAUNCH_CF(false, false, false, false) }
     else { PG_LAUNCH_CF(false, true, false, false) }
 #undef PG_LAUNCH_CF
+#undef PG_LAUNCH_CF_F
     return check_cuda(cudaGetLastError());
 }
 
