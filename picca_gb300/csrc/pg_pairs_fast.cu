@@ -68,7 +68,7 @@ constexpr int kChunk = 128;                   // forest-2 pixels staged per warp
 constexpr int kRunMax = 64;                   // pairs summed in FP32 registers per run
 constexpr int kCfBlock = 640;
 constexpr int kCfParts = 8;                   // parts of a neighbour where there are few (auto)
-constexpr int kXcfBlock = 704;
+constexpr int kXcfBlock = 640;
 
 // ---------------------------------------------------------------------------
 // shared-memory histograms: H_COUNT float arrays of stride hstride
@@ -869,8 +869,9 @@ __device__ __forceinline__ void xcf_drain(const Binning &b, const FastConst *__r
 //
 // Bound: issue, a third of it in the runs' adds to shared memory (a run is two
 // pixels long at 2 Mpc/h a pixel). 9,000 forests x 13,500 quasars: 10.3 ms with
-// 16 warps and groups dealt out in turn, 10.1 ms with groups drawn, 9.4 ms with
-// the 22 warps that smaller queues leave room for (20 warps 9.5 ms, 24 no better).
+// 16 warps and groups dealt out in turn, 10.1 ms with groups drawn, 9.8 ms with
+// the 20 warps that smaller queues leave room for (24 warps 9.9 ms; groups drawn
+// from the middle outwards, 10.2 ms, meet in the same bins).
 template <bool EXTRA>
 __global__ void __launch_bounds__(kXcfBlock, 1) xcf_xi_fast_kernel(
     const __grid_constant__ Binning b, const FastConst *__restrict__ fcp,
@@ -966,18 +967,15 @@ __global__ void __launch_bounds__(kXcfBlock, 1) xcf_xi_fast_kernel(
         }
         int head = 0, tail = 0;  // run ring of this warp (warp-uniform)
         int qn = 0;              // FP64 re-decision queue of this warp
-        // groups of 32 quasars, drawn by the warps; where there are fewer than
-        // warps, each in up to four parts of its pixels (a part repeats the
-        // group's set-up, a sixth of its time)
+        // groups of 32 quasars, drawn by the warps; a quasar's pixels stay in one
+        // task, so that its runs do not depend on how the groups fall
         const int groups = (nq + 31) >> 5;
-        int parts = 1;
-        while (parts < 4 && groups * parts < nwarps) parts *= 2;
         for (;;) {
             int task = 0;
             if (lane == 0) task = atomicAdd(&next_task, 1);
             task = __shfl_sync(0xffffffffu, task, 0);
-            if (task >= groups * parts) break;
-            const int kb = (task / parts) * 32, part = task % parts;
+            if (task >= groups) break;
+            const int kb = task * 32;
             const int kk = kb + lane < nq ? (by_distance ? (int)qorder[kb + lane] : kb + lane) : nq;
             float cp = 1.f, st = 0.f, nb = kFar, nbl = 0.f, t = kFar, zv = kFar;
             float wvh = 0.f, wvl = 0.f;
@@ -1057,12 +1055,6 @@ __global__ void __launch_bounds__(kXcfBlock, 1) xcf_xi_fast_kernel(
                 g_hi = max(g_hi, __shfl_xor_sync(0xffffffffu, g_hi, o));
             }
             if (g_lo >= g_hi) continue;
-            if (parts > 1) {
-                const int len = (g_hi - g_lo + parts - 1) / parts;
-                g_lo += part * len;
-                g_hi = min(g_hi, g_lo + len);
-                ib = min(ib, g_hi);  // the odd pixel past the part is the next part's
-            }
             unsigned run_bin = 0xFFFFFFFFu;
             int run_n = 0;
             float r_xi = 0.f, r_xil = 0.f, r_w = 0.f, r_pw = 0.f, r_tw = 0.f, r_zw = 0.f;
@@ -1151,7 +1143,7 @@ __global__ void __launch_bounds__(kXcfBlock, 1) xcf_xi_fast_kernel(
             for (int i = g_lo; i < g_hi; i += 2) {
                 PairEval ea, eb;
                 eval(i, ea);
-                eval(i + 1, eb);
+                eval(i + 1, eb);  // i + 1 = g_hi: outside every lane's range
                 take(ea, i);
                 take(eb, i + 1);
                 if (__any_sync(0xffffffffu, ea.near | eb.near)) {

@@ -1,7 +1,7 @@
 """The delta x quasar correlation for numbers of quasars around its groups of
-32 and the counts where a group is cut into parts (a few to some hundred per
-forest): pair counts are the FP64 kernel's, the other sums within 2e-6 of it
-(FP32 pair terms, the tolerance of test_gpu_pairs)."""
+32, fewer and more groups than warps: pair counts are the FP64 kernel's, the
+other sums within 2e-6 of it (FP32 pair terms, the tolerance of
+test_gpu_pairs)."""
 
 import numpy as np
 import pytest
