@@ -1626,6 +1626,9 @@ __device__ __forceinline__ int count_keys(const unsigned long long *key, int n,
     return lo;
 }
 
+// TABLES: the tables fit in shared memory; else (a stack of more than some
+// 14,000 points) the searches read the model's arrays.
+template <bool TABLES>
 __global__ void __launch_bounds__(kContBlock) cont_deltas_kernel(
     const __grid_constant__ pg_spectra sp, const __grid_constant__ pg_cont_model m,
     const __grid_constant__ pg_cont_fit fit, double *__restrict__ delta,
@@ -1639,13 +1642,23 @@ __global__ void __launch_bounds__(kContBlock) cont_deltas_kernel(
     unsigned long long *brk = reinterpret_cast<unsigned long long *>(smem + L.brk);
     // scipy interp1d(kind="nearest"): x_bds[i] = (x[i] + x[i + 1]) / 2,
     // index = searchsorted(x_bds, v, "left")
-    for (int k = threadIdx.x; k < ns; k += blockDim.x) {
+    for (int k = threadIdx.x; TABLES && k < ns; k += blockDim.x) {
         if (k + 1 < ns) mid[k] = order_key((m.stack_x[k] + m.stack_x[k + 1]) / 2.0);
         stack_y[k] = m.stack_y[k];
     }
-    if (mi > 0)
+    if (TABLES && mi > 0)
         for (int k = threadIdx.x; k <= mi; k += blockDim.x) brk[k] = order_key(m.var_breaks[k]);
     __syncthreads();
+    auto stack_at = [&](unsigned long long v) {
+        if (TABLES) return stack_y[count_keys<false>(mid, ns - 1, v)];
+        int lo = 0, hi = ns - 1;
+        while (lo < hi) {
+            const int i = (lo + hi) >> 1;
+            if (order_key((m.stack_x[i] + m.stack_x[i + 1]) / 2.0) < v) lo = i + 1;
+            else hi = i;
+        }
+        return m.stack_y[lo];
+    };
     const int lane = threadIdx.x & 31;
     const int64_t warp_global = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -1659,13 +1672,14 @@ __global__ void __launch_bounds__(kContBlock) cont_deltas_kernel(
                 const double ll = sp.log_lambda[off + p], iv = sp.ivar[off + p];
                 const unsigned long long key = order_key(ll);
                 double expected = fit.continuum[off + p];
-                if (ns > 0) expected *= stack_y[count_keys<false>(mid, ns - 1, key)];
+                if (ns > 0) expected *= stack_at(key);
                 // compute_forest_weights (dr16_expected_flux.py:466-488) with
                 // 1 / var_pipe = ivar expected^2
                 if (iv > 0) {
                     double eta = 0., vlss = 1., fudge = 0.;
                     if (mi > 0) {
-                        int i = count_keys<true>(brk, mi + 1, key) - 1;
+                        int i = TABLES ? count_keys<true>(brk, mi + 1, key) - 1
+                                       : ppoly_piece(m.var_breaks, mi, ll);
                         i = i < 0 ? 0 : (i > mi - 1 ? mi - 1 : i);
                         const double dx = ll - m.var_breaks[i];
                         eta = ppoly_at(m.eta_coef, mi, i, dx);
@@ -1686,7 +1700,7 @@ __global__ void __launch_bounds__(kContBlock) cont_deltas_kernel(
 // Warm-start network inputs (see pg_mlp_features in include/picca_gb300.h),
 // a warp per forest with forest_feature_sums. A CTA has a range of forests;
 // its threads fetch the offsets and redshifts and form log10(1 + z) (FP64) of
-// up to kFeatBlock of them together. Bound: HBM (32 bytes a pixel). Before, a
+// up to kFeatBlock of them together. Before, a
 // warp took eight forests of five dependent loads each in a row: 209 us
 // for 50,021 forests, 111 us now, at 2.3 TB/s bound by issue (1,700 instructions a
 // forest: conversions, the segmented scan, IEEE roots and quotients).
@@ -1854,13 +1868,16 @@ int launch_cont_deltas(const pg_spectra &sp, const pg_cont_model &m, const pg_co
     if (sp.num <= 0) return PG_OK;
     const size_t smem = delta_smem(m.stack_x ? m.num_stack : 0,
                                    m.use_constant_weight ? 0 : m.num_var_intervals).total;
-    if (smem > kMaxDynSmem) return PG_ERR_UNSUPPORTED;
-    cudaError_t err = cudaFuncSetAttribute(cont_deltas_kernel,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (err != cudaSuccess) return check_cuda(err);
     unsigned blocks = blocks_for(sp.num, num_sms);
     if (blocks > (unsigned)num_sms * 8) blocks = (unsigned)num_sms * 8;
-    cont_deltas_kernel<<<blocks, kContBlock, smem, stream>>>(sp, m, fit, delta, weights);
+    if (smem > kMaxDynSmem) {
+        cont_deltas_kernel<false><<<blocks, kContBlock, 0, stream>>>(sp, m, fit, delta, weights);
+        return check_cuda(cudaGetLastError());
+    }
+    cudaError_t err = cudaFuncSetAttribute(cont_deltas_kernel<true>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (err != cudaSuccess) return check_cuda(err);
+    cont_deltas_kernel<true><<<blocks, kContBlock, smem, stream>>>(sp, m, fit, delta, weights);
     return check_cuda(cudaGetLastError());
 }
 
