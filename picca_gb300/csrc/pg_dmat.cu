@@ -2442,10 +2442,8 @@ int dmat_config(const pg_corr_params &p, const pg_dmat_params &d, int p1, int p2
             h.smem = base + h.key_bytes;
         }
     }
-    if (!h.key_rows) {
-        if (s.total > 220 * 1024) return PG_ERR_UNSUPPORTED;
-        h.smem = s.total;
-    }
+    if (s.total > 220 * 1024) return PG_ERR_UNSUPPORTED;
+    if (!h.key_rows) h.smem = s.total;
     h.p1 = p1;
     h.p2 = p2;
     h.mwords = mwords;
