@@ -747,8 +747,9 @@ def wick_leg(args, fs, params, ang_max):
             "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak,
                          "unit": "TFLOP/s", "frac": achieved / peak,
                          "peak_source": "cuBLAS DGEMM 4096^3 measured in this run",
-                         "achieved_counts": "2 flops (one FMA) per pair of listed pixel pairs"
-                         if qs is None else "2 flops per GEMM multiply-add (U^T X U, W^T cW; "
+                         "achieved_counts": "2 flops (one FMA) per pair of listed pixel pairs, "
+                         "the reference's count (the kernel sums over segments of equal bin and "
+                         "executes fewer)" if qs is None else "2 flops per GEMM multiply-add (U^T X U, W^T cW; "
                          "the direct same-quasar sums and the scatter not counted)"},
             "cpu_baseline": {"value": cpu_units, "unit": unit,
                              "pairs_of_pixel_pairs_per_s": cpu_pairs2, "cores": cores,

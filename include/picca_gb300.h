@@ -464,7 +464,7 @@ int pg_mlp_forward(pg_plan *plan, const uint16_t *packed, const float *params, c
  * current model straight into the tensor-core operand in shared memory
  * (the same values pg_mlp_features writes), then the network runs on them;
  * writes y [num, 2] FP32 and a0 [num] FP64. Measured slower than the two
- * calls (3.2 ms against 1.1 + 0.5 ms for 400k forests on a GB300): the
+ * calls (1.8 ms against 0.75 + 0.45 ms for 400k forests on a GB300): the
  * feature pass is memory-latency bound and gets only the 16 warps per SM
  * that the network's 192 KB of operand buffers leave room for. */
 int pg_mlp_warm_start(pg_plan *plan, const pg_spectra *spectra, const pg_cont_model *model,
