@@ -9,7 +9,7 @@
 struct pg_plan {
     int device;
     int num_sms;
-    void *scratch;      // pg::Scratch followed by the precision-form constants
+    void *scratch;      // pg::Scratch, the precision-form constants, the histograms' exact sums
     cudaStream_t last_stream;
     pg_tuning tuning;   // launch shapes of the precision-form pair kernels (0: default)
 };
@@ -25,12 +25,18 @@ int check_cuda(cudaError_t err) {
 
 namespace {
 
-size_t scratch_bytes() { return ((sizeof(Scratch) + 255) & ~(size_t)255) + fast_const_bytes(); }
+size_t exact_offset() { return ((sizeof(Scratch) + 255) & ~(size_t)255) + fast_const_bytes(); }
+
+size_t scratch_bytes() { return exact_offset() + cont_exact_bytes(); }
 
 Scratch *scratch_of(pg_plan *plan) { return static_cast<Scratch *>(plan->scratch); }
 
 void *fast_const_of(pg_plan *plan) {
     return static_cast<char *>(plan->scratch) + ((sizeof(Scratch) + 255) & ~(size_t)255);
+}
+
+uint32_t *exact_work_of(pg_plan *plan) {
+    return reinterpret_cast<uint32_t *>(static_cast<char *>(plan->scratch) + exact_offset());
 }
 
 bool finite_positive(double v) { return isfinite(v) && v > 0; }
@@ -487,8 +493,8 @@ int pg_cont_stacks_accumulate(pg_plan *plan, const pg_spectra *spectra,
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     plan->last_stream = st;
     if ((rc = reset_scratch(plan, st))) return rc;
-    return launch_cont_stacks(*spectra, *model, *fit, *stacks, scratch_of(plan), plan->num_sms,
-                              st);
+    return launch_cont_stacks(*spectra, *model, *fit, *stacks, exact_work_of(plan),
+                              cont_exact_bytes(), scratch_of(plan), plan->num_sms, st);
 }
 
 int pg_cont_deltas(pg_plan *plan, const pg_spectra *spectra, const pg_cont_model *model,

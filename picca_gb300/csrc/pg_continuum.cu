@@ -15,6 +15,8 @@
 // iminuit's MIGRAD.
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 #include "pg_cont_common.cuh"
 #include "pg_internal.cuh"
 
@@ -1313,8 +1315,23 @@ __global__ void __launch_bounds__(32 * kRefineWarps) cont_fit_refine_kernel(
 // stored as two floats) on the observed-frame grid and read for pixels on a
 // grid node (all of them for forests rebinned to the grid); others evaluate
 // them in FP64.
+//
+// EXACT: the histograms are 128-bit fixed-point numbers (four 32-bit words, the
+// last place 2^-kFixScale) instead of hi/lo pairs, in shared memory and across
+// the blocks, so that a sum does not depend on the order of its terms: the
+// same inputs give the same bits. With pairs the model of the next iteration
+// moved by its last bits from run to run, and the FP32 decisions of the mixed
+// fit on it moved single forests by up to 1e-6. A term of 2^kFineTop or more
+// goes to a second fixed-point number of its bin in global memory (last place
+// 2^-kCoarseScale), one of 2^kCoarseTop or more, or none, straight to the FP64
+// result. Calls whose words do not fit in shared memory keep the pairs. 1,024
+// threads (a block an SM; 512 leave the chains of word adds less to overlap
+// with). Five passes over 40,000 forests of 160 pixels: 1.45 ms in pairs, 1.67 ms
+// exact (1.95 ms in blocks of 512).
 constexpr int kStackBlock = 512;
 constexpr int kStackGroup = 8;
+constexpr int kFixScale = 88, kFineTop = 14;      // 2^25 terms of 2^14 stay below 2^39
+constexpr int kCoarseScale = 56, kCoarseTop = 46;  // and 2^25 of 2^46 below 2^71
 
 struct StackSlot {
     int64_t off;
@@ -1323,35 +1340,163 @@ struct StackSlot {
     float zr_hi, zr_lo;  // log10(1 + z) + rest grid start (log grid) or log10(1 + z) (linear)
 };
 
+// The size limit of a call (all histograms as hi/lo pairs).
 __host__ __device__ inline size_t stack_smem_bytes(const pg_cont_stacks &st, bool table) {
     const size_t nvar = (size_t)st.var_lambda_bins * kVarBins;
     return (size_t)8 * (2 * st.rest_bins + 2 * st.obs_bins + 3 * nvar) + (size_t)8 * nvar +
            (table ? (size_t)32 * st.obs_bins : 0) + 64;
 }
 
-__global__ void __launch_bounds__(kStackBlock) cont_stacks_kernel(
+// The wanted histograms as one array of cells, a word of a cell per plane (hi
+// and lo, or four words); then the counts of the variance bins.
+struct StackCells {
+    int mc_num, mc_w, s_num, s_w, v_mean, v_d2, v_d4, total, nvar;
+};
+
+__host__ __device__ inline StackCells stack_cells(const pg_cont_stacks &st) {
+    StackCells c;
+    const int r = st.mean_cont_num ? st.rest_bins : 0, o = st.stack_num ? st.obs_bins : 0;
+    c.nvar = st.var_mean ? st.var_lambda_bins * kVarBins : 0;
+    c.mc_num = 0;
+    c.mc_w = r;
+    c.s_num = 2 * r;
+    c.s_w = c.s_num + o;
+    c.v_mean = c.s_num + 2 * o;
+    c.v_d2 = c.v_mean + c.nvar;
+    c.v_d4 = c.v_d2 + c.nvar;
+    c.total = c.v_d4 + c.nvar;
+    return c;
+}
+
+__host__ __device__ inline size_t stack_bytes(const pg_cont_stacks &st, bool exact, bool table) {
+    const StackCells c = stack_cells(st);
+    return (size_t)(exact ? 16 : 8) * c.total + (size_t)8 * c.nvar +
+           (table ? (size_t)32 * st.obs_bins : 0) + 64;
+}
+
+// Adds the N two's complement numbers word[n][0..3] to the four words at
+// h[n], h[n] + stride, ...: the carry out of a word is seen by the add that
+// causes it. Word by word, so that the N round trips overlap.
+template <int N>
+__device__ __forceinline__ void fix_add_words(uint32_t *const h[N], int stride,
+                                              const uint32_t word[N][4]) {
+    uint32_t carry[N];
+#pragma unroll
+    for (int n = 0; n < N; ++n) carry[n] = 0u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        uint32_t x[N], old[N];
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            x[n] = word[n][k] + carry[n];
+            carry[n] = x[n] < carry[n] ? 1u : 0u;  // word + carry was 2^32: nothing to add
+            if (x[n]) old[n] = atomicAdd(h[n] + k * stride, x[n]);
+        }
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+            if (x[n]) carry[n] |= old[n] + x[n] < x[n] ? 1u : 0u;
+    }
+}
+
+// v in units of 2^-SCALE (to 2^-50 of v, and to a unit), |v| < 2^(102 - SCALE).
+template <int SCALE>
+__device__ __forceinline__ void fix_words(dfl v, uint32_t word[4]) {
+    const uint32_t u = __float_as_uint(v.hi);
+    const int e = (int)((u >> 23) & 0xFFu);
+    long long t;
+    int p = 0;
+    if (e >= 64) {
+        // t = v 2^(176 - e), the last place of hi at bit 26
+        const long long m = (u & 0x7FFFFFu) | 0x800000u;
+        const float lo = v.lo * __uint_as_float((uint32_t)(303 - e) << 23);
+        t = ((int)u < 0 ? -m : m) * (1LL << 26) + __float2int_rn(lo);
+        p = e - 176 + SCALE;
+        if (p < 0) {
+            t = (t + (1LL << (-p - 1))) >> -p;
+            p = 0;
+        }
+    } else {  // below 2^-63
+        t = __double2ll_rn(ldexp((double)v.hi + (double)v.lo, SCALE));
+    }
+    const int s = p & 31;
+    const unsigned long long low = (unsigned long long)t << s;
+    const uint32_t a = (uint32_t)low, b = (uint32_t)(low >> 32);
+    const uint32_t c = (uint32_t)((t >> 32) >> (32 - s));  // from bit 64 on
+    const bool up = p >= 32;
+    word[0] = up ? 0u : a;
+    word[1] = up ? a : b;
+    word[2] = up ? b : c;
+    word[3] = up ? c : (uint32_t)(t >> 63);
+}
+
+// The number in four words, in units of 2^-scale.
+__device__ __forceinline__ double fix_value(const uint32_t word[4], int scale) {
+    unsigned long long hi = (unsigned long long)word[3] << 32 | word[2];
+    unsigned long long lo = (unsigned long long)word[1] << 32 | word[0];
+    const bool negative = (long long)hi < 0;
+    if (negative) {
+        lo = 0ull - lo;
+        hi = ~hi + (lo == 0ull ? 1ull : 0ull);
+    }
+    const double v = ldexp((double)hi, 64 - scale) + ldexp((double)lo, -scale);
+    return negative ? -v : v;
+}
+
+// A term of 2^kFineTop or more: to its bin's coarse number, or (with infinities
+// and NaN) to the FP64 result.
+__device__ __noinline__ void stack_add_large(uint32_t *coarse, int stride, double *dst, dfl v) {
+    if (fabsf(v.hi) < (float)(1LL << kCoarseTop)) {
+        uint32_t word[1][4];
+        fix_words<kCoarseScale>(v, word[0]);
+        fix_add_words<1>(&coarse, stride, word);
+    } else {
+        atomicAdd(dst, (double)v.hi + (double)v.lo);
+    }
+}
+
+// exact_work (EXACT): 2 x 4 words of every cell, zeroed, the second four the
+// terms of 2^kFineTop and more.
+template <bool EXACT, int BLOCK>
+__global__ void __launch_bounds__(BLOCK) cont_stacks_kernel(
     const __grid_constant__ pg_spectra sp, const __grid_constant__ pg_cont_model m,
     const __grid_constant__ pg_cont_fit fit, const __grid_constant__ pg_cont_stacks st,
-    Scratch *scratch, int use_table) {
+    Scratch *scratch, int use_table, uint32_t *exact_work) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ uint32_t seen[kStackBlock / 32][64];  // per-warp bitmap of var bins (<= 2048)
-    __shared__ StackSlot s_slots[kStackBlock / 32][kStackGroup];
+    __shared__ uint32_t seen[BLOCK / 32][64];  // per-warp bitmap of var bins (<= 2048)
+    __shared__ StackSlot s_slots[BLOCK / 32][kStackGroup];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
-    const int nvar = st.var_lambda_bins * kVarBins;
+    const StackCells cells = stack_cells(st);
+    const int nvar = cells.nvar, nc = cells.total;
     const int mi = m.use_constant_weight ? 0 : m.num_var_intervals;
     const int R = st.rest_bins, O = st.obs_bins;
-    // layout: table (float4 x 2 per obs bin), then hi/lo FP32 histograms, then counts
+    // layout: table (float4 x 2 per obs bin), then the histograms, then counts
     float4 *table = reinterpret_cast<float4 *>(smem_raw);
-    float *hist = reinterpret_cast<float *>(smem_raw + (use_table ? (size_t)32 * O : 0));
-    float *mc_num_h = hist, *mc_num_l = mc_num_h + R, *mc_w_h = mc_num_l + R, *mc_w_l = mc_w_h + R;
-    float *s_num_h = mc_w_l + R, *s_num_l = s_num_h + O, *s_w_h = s_num_l + O, *s_w_l = s_w_h + O;
-    float *v_mean_h = s_w_l + O, *v_mean_l = v_mean_h + nvar;
-    float *v_d2_h = v_mean_l + nvar, *v_d2_l = v_d2_h + nvar;
-    float *v_d4_h = v_d2_l + nvar, *v_d4_l = v_d4_h + nvar;
-    uint32_t *v_np = reinterpret_cast<uint32_t *>(v_d4_l + nvar), *v_nq = v_np + nvar;
-    const int nwords = 4 * R + 4 * O + 8 * nvar;
-    for (int k = threadIdx.x; k < nwords; k += blockDim.x) hist[k] = 0.f;
+    uint32_t *hist =
+        reinterpret_cast<uint32_t *>(smem_raw + (use_table ? (size_t)32 * O : 0));
+    constexpr int kPlanes = EXACT ? 4 : 2;
+    uint32_t *v_np = hist + kPlanes * nc, *v_nq = v_np + nvar;
+    const int nwords = kPlanes * nc + 2 * nvar;
+    for (int k = threadIdx.x; k < nwords; k += blockDim.x) hist[k] = 0u;
+    // N terms v to the cells, whose FP64 results are at dst
+    auto add = [&](auto count, const int *cell, double *const *dst, const dfl *v) {
+        constexpr int N = decltype(count)::value;
+        if (!EXACT) {
+            float *h = reinterpret_cast<float *>(hist);
+#pragma unroll
+            for (int n = 0; n < N; ++n) hist_add(h, h + nc, cell[n], v[n]);
+            return;
+        }
+        uint32_t *at[N], word[N][4];
+#pragma unroll
+        for (int n = 0; n < N; ++n) {
+            const bool fine = fabsf(v[n].hi) < (float)(1 << kFineTop);
+            at[n] = hist + cell[n];
+            fix_words<kFixScale>(fine ? v[n] : dfl{0.f, 0.f}, word[n]);
+            if (!fine) stack_add_large(exact_work + 4 * nc + cell[n], nc, dst[n], v[n]);
+        }
+        fix_add_words<N>(at, nc, word);
+    };
     if (use_table) {
         // variance functions on the observed-frame grid nodes
         for (int j = threadIdx.x; j < O; j += blockDim.x) {
@@ -1491,8 +1636,11 @@ __global__ void __launch_bounds__(kStackBlock) cont_stacks_kernel(
                                     const double c64 = fit.continuum[off + p];
                                     ratio = dfl_of(sp.flux[off + p] / (c64 + 1e-16));
                                 }
-                                hist_add(mc_num_h, mc_num_l, bin, dfl_mul(ratio, w));
-                                hist_add(mc_w_h, mc_w_l, bin, w);
+                                const int cell[] = {cells.mc_num + bin, cells.mc_w + bin};
+                                double *const dst[] = {st.mean_cont_num + bin,
+                                                       st.mean_cont_weight + bin};
+                                const dfl v[] = {dfl_mul(ratio, w), w};
+                                add(std::integral_constant<int, 2>{}, cell, dst, v);
                             }
                         } else {
                             report_error(scratch, PG_ERR_BIN_RANGE, bin);
@@ -1502,8 +1650,10 @@ __global__ void __launch_bounds__(kStackBlock) cont_stacks_kernel(
                         // compute_delta_stack: delta = f / C where ivar > 0
                         if (jobs >= 0 && jobs < O) {
                             if (has_iv) {
-                                hist_add(s_num_h, s_num_l, jobs, dfl_mul(Q, w));
-                                hist_add(s_w_h, s_w_l, jobs, w);
+                                const int cell[] = {cells.s_num + jobs, cells.s_w + jobs};
+                                double *const dst[] = {st.stack_num + jobs, st.stack_weight + jobs};
+                                const dfl v[] = {dfl_mul(Q, w), w};
+                                add(std::integral_constant<int, 2>{}, cell, dst, v);
                             }
                         } else {
                             report_error(scratch, PG_ERR_BIN_RANGE, jobs);
@@ -1542,9 +1692,12 @@ __global__ void __launch_bounds__(kStackBlock) cont_stacks_kernel(
                         if (lbin >= 0 && bin >= 0 && bin < nvar) {
                             const dfl delta = dfl_add(Q, dfl{-1.f, 0.f});
                             const dfl d2 = dfl_mul(delta, delta);
-                            hist_add(v_mean_h, v_mean_l, (int)bin, delta);
-                            hist_add(v_d2_h, v_d2_l, (int)bin, d2);
-                            hist_add(v_d4_h, v_d4_l, (int)bin, dfl_mul(d2, d2));
+                            const int k = (int)bin;
+                            const int cell[] = {cells.v_mean + k, cells.v_d2 + k, cells.v_d4 + k};
+                            double *const dst[] = {st.var_mean + k, st.var_delta2 + k,
+                                                   st.var_delta4 + k};
+                            const dfl v[] = {delta, d2, dfl_mul(d2, d2)};
+                            add(std::integral_constant<int, 3>{}, cell, dst, v);
                             atomicAdd(&v_np[bin], 1u);
                             atomicOr(&seen[wib][bin >> 5], 1u << (bin & 31));
                         } else {
@@ -1569,28 +1722,62 @@ __global__ void __launch_bounds__(kStackBlock) cont_stacks_kernel(
         __syncwarp();
     }
     __syncthreads();
-    // one FP64 add per nonzero bin and block
-    auto flush = [&](double *dst, const float *h, const float *l, int count) {
-        if (!dst) return;
-        for (int k = threadIdx.x; k < count; k += blockDim.x)
-            if (h[k] != 0.f || l[k] != 0.f) atomicAdd(&dst[k], (double)h[k] + (double)l[k]);
-    };
     auto flush_count = [&](double *dst, const uint32_t *c, int count) {
-        if (!dst) return;
         for (int k = threadIdx.x; k < count; k += blockDim.x)
             if (c[k]) atomicAdd(&dst[k], (double)c[k]);
     };
-    flush(st.mean_cont_num, mc_num_h, mc_num_l, R);
-    flush(st.mean_cont_weight, mc_w_h, mc_w_l, R);
-    flush(st.stack_num, s_num_h, s_num_l, O);
-    flush(st.stack_weight, s_w_h, s_w_l, O);
     if (do_var) {
-        flush(st.var_mean, v_mean_h, v_mean_l, nvar);
-        flush(st.var_delta2, v_d2_h, v_d2_l, nvar);
-        flush(st.var_delta4, v_d4_h, v_d4_l, nvar);
         flush_count(st.var_npix, v_np, nvar);
         flush_count(st.var_nqso, v_nq, nvar);
     }
+    if (EXACT) {
+        for (int k = threadIdx.x; k < nc; k += blockDim.x) {
+            const uint32_t word[1][4] = {
+                {hist[k], hist[nc + k], hist[2 * nc + k], hist[3 * nc + k]}};
+            uint32_t *const at[1] = {exact_work + k};
+            fix_add_words<1>(at, nc, word);
+        }
+        return;
+    }
+    // one FP64 add per nonzero bin and block
+    const float *h = reinterpret_cast<const float *>(hist), *l = h + nc;
+    auto flush = [&](double *dst, int from, int count) {
+        for (int k = threadIdx.x; k < count; k += blockDim.x) {
+            const float hk = h[from + k], lk = l[from + k];
+            if (hk != 0.f || lk != 0.f) atomicAdd(&dst[k], (double)hk + (double)lk);
+        }
+    };
+    flush(st.mean_cont_num, cells.mc_num, cells.mc_w - cells.mc_num);
+    flush(st.mean_cont_weight, cells.mc_w, cells.s_num - cells.mc_w);
+    flush(st.stack_num, cells.s_num, cells.s_w - cells.s_num);
+    flush(st.stack_weight, cells.s_w, cells.v_mean - cells.s_w);
+    flush(st.var_mean, cells.v_mean, nvar);
+    flush(st.var_delta2, cells.v_d2, nvar);
+    flush(st.var_delta4, cells.v_d4, nvar);
+}
+
+// The fixed-point sums of all blocks, added to the FP64 results.
+__global__ void cont_stacks_finish_kernel(const __grid_constant__ pg_cont_stacks st,
+                                          const uint32_t *exact_work) {
+    const StackCells c = stack_cells(st);
+    const int k = blockIdx.x * blockDim.x + threadIdx.x, nc = c.total;
+    if (k >= nc) return;
+    double *dst;
+    int from;
+    if (k < c.mc_w) { dst = st.mean_cont_num; from = c.mc_num; }
+    else if (k < c.s_num) { dst = st.mean_cont_weight; from = c.mc_w; }
+    else if (k < c.s_w) { dst = st.stack_num; from = c.s_num; }
+    else if (k < c.v_mean) { dst = st.stack_weight; from = c.s_w; }
+    else if (k < c.v_d2) { dst = st.var_mean; from = c.v_mean; }
+    else if (k < c.v_d4) { dst = st.var_delta2; from = c.v_d2; }
+    else { dst = st.var_delta4; from = c.v_d4; }
+    uint32_t fine[4], coarse[4];
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+        fine[w] = exact_work[w * nc + k];
+        coarse[w] = exact_work[(4 + w) * nc + k];
+    }
+    dst[k - from] += fix_value(fine, kFixScale) + fix_value(coarse, kCoarseScale);
 }
 
 // Deltas and weights (populate_los_ids, extract_deltas). Bound: the FP64 pipe.
@@ -1815,29 +2002,56 @@ int launch_cont_fit(const pg_spectra &sp, const pg_cont_model &m, const double *
     return check_cuda(err);
 }
 
-int launch_cont_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_cont_fit &fit,
-                       const pg_cont_stacks &st, Scratch *scratch, int num_sms,
-                       cudaStream_t stream) {
-    if (sp.num <= 0) return PG_OK;
-    if (st.var_mean && st.var_lambda_bins * kVarBins > 2048) return PG_ERR_UNSUPPORTED;
-    const bool want_table = !m.use_constant_weight && (st.mean_cont_num || st.stack_num);
-    // the variance-function table when it fits beside the histograms
-    int use_table = want_table && stack_smem_bytes(st, true) <= 200 * 1024 ? 1 : 0;
-    const size_t smem = stack_smem_bytes(st, use_table != 0);
-    if (smem > 200 * 1024) return PG_ERR_UNSUPPORTED;
-    cudaError_t err = cudaFuncSetAttribute(cont_stacks_kernel,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+// Blocks of BLOCK threads as many as are resident; the variance-function table
+// where it fits beside the histograms.
+template <bool EXACT, int BLOCK>
+static int launch_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_cont_fit &fit,
+                         const pg_cont_stacks &st, bool use_table, uint32_t *exact_work,
+                         Scratch *scratch, int num_sms, cudaStream_t stream) {
+    const auto kernel = cont_stacks_kernel<EXACT, BLOCK>;
+    const size_t smem = stack_bytes(st, EXACT, use_table);
+    cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)smem);
     if (err != cudaSuccess) return check_cuda(err);
     int per_sm = 0;
-    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, cont_stacks_kernel, kStackBlock,
-                                                        smem);
+    err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, BLOCK, smem);
     if (err != cudaSuccess) return check_cuda(err);
     const int64_t groups = (sp.num + kStackGroup - 1) / kStackGroup;
-    int64_t blocks = (groups + kStackBlock / 32 - 1) / (kStackBlock / 32);
+    int64_t blocks = (groups + BLOCK / 32 - 1) / (BLOCK / 32);
     const int64_t resident = (int64_t)num_sms * (per_sm > 0 ? per_sm : 1);
     if (blocks > resident) blocks = resident;
-    cont_stacks_kernel<<<(unsigned)(blocks < 1 ? 1 : blocks), kStackBlock, smem, stream>>>(
-        sp, m, fit, st, scratch, use_table);
+    kernel<<<(unsigned)(blocks < 1 ? 1 : blocks), BLOCK, smem, stream>>>(
+        sp, m, fit, st, scratch, use_table, exact_work);
+    return check_cuda(cudaGetLastError());
+}
+
+constexpr size_t kStackLimit = 200 * 1024;  // shared memory of a block
+
+// 16 bytes of shared memory a cell, 32 of the work
+size_t cont_exact_bytes() { return 2 * kStackLimit; }
+
+int launch_cont_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_cont_fit &fit,
+                       const pg_cont_stacks &st, uint32_t *exact_work, size_t exact_bytes,
+                       Scratch *scratch, int num_sms, cudaStream_t stream) {
+    if (sp.num <= 0) return PG_OK;
+    if (st.var_mean && st.var_lambda_bins * kVarBins > 2048) return PG_ERR_UNSUPPORTED;
+    constexpr size_t limit = kStackLimit;
+    const bool want_table = !m.use_constant_weight && (st.mean_cont_num || st.stack_num);
+    const bool pair_table = want_table && stack_smem_bytes(st, true) <= limit;
+    if (stack_smem_bytes(st, pair_table) > limit) return PG_ERR_UNSUPPORTED;
+    const StackCells cells = stack_cells(st);
+    const size_t work = (size_t)cells.total * 32;
+    if (stack_bytes(st, true, false) > limit || work > exact_bytes)
+        return launch_stacks<false, kStackBlock>(sp, m, fit, st, pair_table, nullptr, scratch,
+                                                 num_sms, stream);
+    const bool table = want_table && stack_bytes(st, true, true) <= limit;
+    cudaError_t err = cudaMemsetAsync(exact_work, 0, work, stream);
+    if (err != cudaSuccess) return check_cuda(err);
+    const int rc = launch_stacks<true, 2 * kStackBlock>(sp, m, fit, st, table, exact_work,
+                                                        scratch, num_sms, stream);
+    if (rc) return rc;
+    if (cells.total > 0)
+        cont_stacks_finish_kernel<<<(cells.total + 255) / 256, 256, 0, stream>>>(st, exact_work);
     return check_cuda(cudaGetLastError());
 }
 
