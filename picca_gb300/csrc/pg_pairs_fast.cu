@@ -69,6 +69,8 @@ constexpr int kRunMax = 64;                   // pairs summed in FP32 registers 
 constexpr int kCfBlock = 640;
 constexpr int kCfParts = 8;                   // parts of a neighbour where there are few (auto)
 constexpr int kXcfBlock = 640;
+// dynamic shared memory of a CTA: 227 KB less the kernels' static arrays
+constexpr size_t kCfMaxSmem = 227 * 1024 - 1360, kXcfMaxSmem = 227 * 1024 - 16;
 
 // ---------------------------------------------------------------------------
 // shared-memory histograms: H_COUNT float arrays of stride hstride
@@ -288,11 +290,14 @@ __host__ __device__ inline CfSmem cf_smem(int nbins, int max_pix1, int nwarps) {
     CfSmem l;
     const size_t mp = (size_t)((max_pix1 + 1) & ~1);
     l.cells = 0;
-    // a lane off its diagonal's range reads up to kChunk + 31 pixels before
-    // forest 1 or kChunk after it (into the padding; the pair is not accepted)
-    l.p1 = (size_t)((nbins + 3) & ~3) * H_COUNT * 4 + (size_t)(kChunk + 32) * 16;
-    l.p1x = l.p1 + (mp + kChunk) * 16;
-    l.warps = l.p1x + mp * 16;
+    // A lane off its diagonal's range reads up to 31 pixels before p1 and 32
+    // from its last on: each diagonal of a group is within 31 of the ones whose
+    // ranges set the group's ends (the pair is not accepted). Before p1 lie the
+    // histograms and p1x, of 512 bytes or more together, after it the chunks.
+    const size_t cells = (size_t)((nbins + 3) & ~3) * H_COUNT * 4;
+    l.p1x = cells + mp * 16 < 512 ? 512 - mp * 16 : cells;
+    l.p1 = l.p1x + mp * 16;
+    l.warps = l.p1 + mp * 16;
     l.buf = 0;
     l.bufx = l.buf + (size_t)kChunk * 16;
     l.acc0 = l.bufx + (size_t)kChunk * 16;
@@ -641,8 +646,8 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
                         bool in = (unsigned)(js - sa) < len;
                         const int i = js - joff;
                         if (EXTRA && zerr_pair && in) in = ((veto1[i >> 5] >> (i & 31)) & 1u) == 0u;
-                        // a lane outside its range reads padding or a
-                        // neighbouring array: not accepted, not queued
+                        // a lane outside its range reads a neighbouring array
+                        // (see cf_smem): not accepted, not queued
                         const float4 q1 = p1[i];
                         const float4 q2 = buf[js];
                         const float pp = __fmaf_rn(cp, q1.x, q2.x);
@@ -1231,10 +1236,10 @@ int launch_cf_xi_fast(const Binning &b, double ang_max, const pg_forest_set &s1,
     // memory leaves room for
     int nwarps = kCfBlock / 32;
     if (tuning.warps > 0 && tuning.warps < nwarps) nwarps = tuning.warps;
-    while (nwarps > 1 && cf_smem(b.nbins, max_pix1, nwarps).total > kMaxDynSmem) --nwarps;
+    while (nwarps > 1 && cf_smem(b.nbins, max_pix1, nwarps).total > kCfMaxSmem) --nwarps;
     const int block = nwarps * 32;
     const size_t smem = cf_smem(b.nbins, max_pix1, nwarps).total;
-    if (smem > kMaxDynSmem) return PG_ERR_UNSUPPORTED;
+    if (smem > kCfMaxSmem) return PG_ERR_UNSUPPORTED;
     (void)ang_max;
     int rc = prepare_fast(b, fc, stream);
     if (rc) return rc;
@@ -1291,10 +1296,10 @@ int launch_xcf_xi_fast(const Binning &b, double ang_max, const pg_forest_set &fo
     // memory leaves room for (histograms, forest, per-warp rings and queues)
     int nwarps = kXcfBlock / 32;
     if (tuning.warps > 0 && tuning.warps < nwarps) nwarps = tuning.warps;
-    while (nwarps > 1 && smem_layout(b.nbins, max_pix1, nwarps, true).total > kMaxDynSmem) --nwarps;
+    while (nwarps > 1 && smem_layout(b.nbins, max_pix1, nwarps, true).total > kXcfMaxSmem) --nwarps;
     const int block = nwarps * 32;
     const size_t smem = smem_layout(b.nbins, max_pix1, nwarps, true).total;
-    if (smem > kMaxDynSmem) return PG_ERR_UNSUPPORTED;
+    if (smem > kXcfMaxSmem) return PG_ERR_UNSUPPORTED;
     (void)ang_max;
     int rc = prepare_fast(b, fc, stream);
     if (rc) return rc;
