@@ -110,13 +110,18 @@ __device__ __forceinline__ void flush_rows(float *h, const FastConst &fc, const 
         if (nb == 0) continue;
         // four FP64 operations a bin (conversions on the integer pipe, the
         // scales as products; with divisions and FP64-pipe conversions a flush
-        // of 2,500 bins was about 35 operations a bin, 23 us of the pipe)
-        auto at = [&](int k) { return f32_to_f64(h[k * hs + b]); };
+        // of 2,500 bins was about 35 operations a bin, 23 us of the pipe); sums
+        // below the FP32 normal range, whose pairs count like others, on the FP64
+        // pipe, which keeps them
+        auto at = [&](int k) {
+            const float v = h[k * hs + b];
+            return v != 0.f && fabsf(v) < 1.17549435e-38f ? (double)v : f32_to_f64(v);
+        };
         atomicAdd(&out.weights[o + b], at(H_WE) + at(H_WEL));
         atomicAdd(&out.xi[o + b], at(H_XI) + at(H_XIL));
         atomicAdd(&out.r_par[o + b], at(H_PW) * per_p);
         atomicAdd(&out.r_trans[o + b], at(H_TW) * per_t);
-        atomicAdd(&out.z[o + b], f32_to_f64(0.5f * h[H_ZW * hs + b]));
+        atomicAdd(&out.z[o + b], 0.5 * at(H_ZW));
         atomicAdd((unsigned long long *)&out.num_pairs[o + b], (unsigned long long)nb);
 #pragma unroll
         for (int k = 0; k < H_NB; ++k) h[k * hs + b] = 0.f;
