@@ -1096,7 +1096,7 @@ def xcf_leg(args, fs, ang_max, steps, warmup):
     """The delta x quasar cross-correlation of the same forests (picca_xcf.py:
     r_par -200 to 200 in 100 bins x r_trans 0-200 in 50), precision form: a
     step is quasar neighbours + pixel-quasar pairs of the whole survey. Per
-    bin error against the plain FP64 kernel on 1% of the forests, FP32
+    bin error against the plain all-FP64 kernel on 1% of the forests, FP32
     roofline of the pair kernel, and the CPU oracle on a sample."""
     import torch
 
@@ -1203,7 +1203,9 @@ def precision_check(engine, params, d1, d2, work, nrows, nbins, fraction, xcf=Fa
                       xcf=xcf)
     ev[1].record(stream)
     ev[2].record(stream)
+    engine.plan.set_all_fp64(True)  # no decision shared with the precision form
     engine.accumulate(params, d1, d2, offsets, index, sub, n_check, r64, pairs.MODE_FP64, xcf=xcf)
+    engine.plan.set_all_fp64(False)
     ev[3].record(stream)
     torch.cuda.synchronize()
     fast_s = ev[0].elapsed_time(ev[1]) / 1e3

@@ -66,7 +66,10 @@ extern "C" {
 #define PG_ERR_NO_DEVICE (-7)
 
 /* pg_cf_xi / pg_xcf_xi arithmetic modes */
-#define PG_MODE_FP64 0       /* all geometry and sums in FP64 (plain form)   */
+#define PG_MODE_FP64 0       /* all sums in FP64; with (r_par, r_trans) bins the
+                                pairs are decided in FP32 and near a bin edge
+                                or a cut in FP64, else all geometry in FP64
+                                (see pg_plan_set_all_fp64)                   */
 #define PG_MODE_FP32_GUARD 1 /* FP32 geometry, FP64 re-decision of pairs near
                                 a bin edge, FP32 block sums (xi compensated)
                                 merged into FP64 rows (precision form)       */
@@ -135,8 +138,8 @@ typedef struct pg_plan pg_plan;
 const char *pg_strerror(int status);
 int pg_version(void);
 
-/* Create a plan on the CURRENT device (allocates a few hundred bytes of
- * device scratch) / release it. */
+/* Create a plan on the CURRENT device (allocates 0.4 MB of device scratch)
+ * / release it. */
 int pg_plan_create(pg_plan **plan);
 int pg_plan_destroy(pg_plan *plan);
 
@@ -147,7 +150,7 @@ int pg_plan_stats(pg_plan *plan, pg_run_stats *stats);
  * counterpart in the reference): warps per CTA and CTAs per SM (each CTA
  * keeps its own shared-memory histogram, so CTAs per SM is the number of
  * histogram replicas on an SM). 0 selects the default: the most warps the
- * shared memory allows (20 for pg_cf_xi, 16 for pg_xcf_xi) and as many CTAs
+ * shared memory allows, at most 20, and as many CTAs
  * as fit. The results do not depend on the shape beyond the summation order
  * of the FP32-compensated sums (the pair counts are identical). The
  * no-allocation entry pg_cf_xi_static always uses the default. */
@@ -157,6 +160,11 @@ typedef struct pg_tuning {
 } pg_tuning;
 int pg_plan_set_tuning(pg_plan *plan, const pg_tuning *tuning);
 int pg_plan_get_tuning(pg_plan *plan, pg_tuning *tuning);
+
+/* on != 0: PG_MODE_FP64 calls of this plan form all geometry in FP64, with
+ * every binning (the plain loop: several times slower, the same pairs and
+ * bins). For verification of the forms that decide pairs in FP32. */
+int pg_plan_set_all_fp64(pg_plan *plan, int32_t on);
 
 /* Neighbour lists of every forest of s1 against s2 (s2 == NULL: auto-
  * correlation of s1 with itself, keeping ra1 > ra2 as cf.py:129-135).

@@ -103,6 +103,7 @@ def lib():
     handle.pg_plan_create.argtypes = [_P(ctypes.c_void_p)]
     handle.pg_plan_destroy.argtypes = [ctypes.c_void_p]
     handle.pg_plan_stats.argtypes = [ctypes.c_void_p, _P(RunStats)]
+    handle.pg_plan_set_all_fp64.argtypes = [ctypes.c_void_p, ctypes.c_int32]
     handle.pg_cf_neighbours.argtypes = [
         ctypes.c_void_p, _P(CorrParams), _P(ForestSetC), _P(ForestSetC), ctypes.c_void_p,
         ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]
@@ -164,6 +165,10 @@ class Plan:
         out = RunStats()
         check(lib().pg_plan_stats(self._handle, ctypes.byref(out)), "pg_plan_stats")
         return out
+
+    def set_all_fp64(self, on):
+        """MODE_FP64 calls with all geometry in FP64 (verification)."""
+        check(lib().pg_plan_set_all_fp64(self._handle, int(bool(on))), "pg_plan_set_all_fp64")
 
     def close(self):
         if self._handle:

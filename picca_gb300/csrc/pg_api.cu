@@ -12,6 +12,7 @@ struct pg_plan {
     void *scratch;      // pg::Scratch, the precision-form constants, the histograms' exact sums
     cudaStream_t last_stream;
     pg_tuning tuning;   // launch shapes of the precision-form pair kernels (0: default)
+    bool all_fp64;      // PG_MODE_FP64: the plain loop for every binning
 };
 
 namespace pg {
@@ -161,6 +162,12 @@ int pg_plan_get_tuning(pg_plan *plan, pg_tuning *tuning) {
     return PG_OK;
 }
 
+int pg_plan_set_all_fp64(pg_plan *plan, int32_t on) {
+    if (!plan) return PG_ERR_INVALID_ARGUMENT;
+    plan->all_fp64 = on != 0;
+    return PG_OK;
+}
+
 int pg_plan_stats(pg_plan *plan, pg_run_stats *stats) {
     if (!plan || !stats) return PG_ERR_INVALID_ARGUMENT;
     int rc = check_cuda(cudaStreamSynchronize(plan->last_stream));
@@ -290,8 +297,8 @@ int pg_cf_xi(pg_plan *plan, const pg_corr_params *params, const pg_forest_set *s
                                  fast_const_of(plan), plan->num_sms, st,
                                  LaunchTuning{plan->tuning.cf_warps, plan->tuning.cf_blocks_per_sm});
     return launch_cf_xi_fp64(b, *s1, other, nbr_offsets, nbr_index, nbr_angle, work_order,
-                             num_work, *out,
-                             scratch_of(plan), plan->num_sms, st);
+                             num_work, *out, scratch_of(plan), plan->num_sms, st,
+                             plan->all_fp64);
 }
 
 int pg_xcf_xi(pg_plan *plan, const pg_corr_params *params, const pg_forest_set *forests,
@@ -321,8 +328,8 @@ int pg_xcf_xi(pg_plan *plan, const pg_corr_params *params, const pg_forest_set *
             num_work, *out, scratch_of(plan), fast_const_of(plan), plan->num_sms, st,
             LaunchTuning{plan->tuning.xcf_warps, plan->tuning.xcf_blocks_per_sm});
     return launch_xcf_xi_fp64(b, *forests, *objs, nbr_offsets, nbr_index, nbr_angle, work_order,
-                              num_work,
-                              *out, scratch_of(plan), plan->num_sms, st);
+                              num_work, *out, scratch_of(plan), plan->num_sms, st,
+                              plan->all_fp64);
 }
 
 static int validate_dmat(const pg_corr_params *params, const pg_dmat_params *dparams) {

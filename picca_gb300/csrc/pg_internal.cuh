@@ -200,7 +200,8 @@ int launch_xcf_neighbours(const pg_corr_params &p, const pg_forest_set &forests,
 int launch_cf_xi_fp64(const Binning &b, const pg_forest_set &s1, const pg_forest_set &s2,
                       const int64_t *nbr_offsets, const int32_t *nbr_index, const double *nbr_angle,
                       const int32_t *work_order, int64_t num_work, const pg_xi_rows &out,
-                      Scratch *scratch, int num_sms, cudaStream_t stream);
+                      Scratch *scratch, int num_sms, cudaStream_t stream,
+                      bool all_fp64 = false);
 // FP64 sums with FP32 decisions (pg_pairs_runs64.cu), and what it covers.
 bool runs64_covers(const Binning &b, const pg_forest_set &s1, const pg_forest_set &s2,
                    int64_t num_work);
@@ -218,7 +219,8 @@ int launch_xcf_xi_runs64(const Binning &b, const pg_forest_set &fs, const pg_for
 int launch_xcf_xi_fp64(const Binning &b, const pg_forest_set &forests, const pg_forest_set &objs,
                        const int64_t *nbr_offsets, const int32_t *nbr_index, const double *nbr_angle,
                        const int32_t *work_order, int64_t num_work, const pg_xi_rows &out,
-                       Scratch *scratch, int num_sms, cudaStream_t stream);
+                       Scratch *scratch, int num_sms, cudaStream_t stream,
+                       bool all_fp64 = false);
 // Size of the device buffer holding the precision-form constants.
 size_t fast_const_bytes();
 // Launch shape of the precision-form pair kernels: warps per CTA (the CTA

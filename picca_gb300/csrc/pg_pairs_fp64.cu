@@ -1,6 +1,7 @@
 // Plain all-FP64 pair accumulation (the "plain GPU drop-in" form): the
-// angular and r-mu binnings and forests too long for the shared memory of
-// pg_pairs_runs64.cu.
+// angular and r-mu binnings, forests too long for the shared memory of
+// pg_pairs_runs64.cu, and, where the plan asks for it (pg_plan_set_all_fp64),
+// everything.
 //
 // Persistent kernel: each CTA pops a work item (one forest of set 1 with all
 // of its neighbours) from a global counter, accumulates every pixel pair in
@@ -277,9 +278,9 @@ size_t hist64_bytes(int nbins) { return (size_t)nbins * (5 * sizeof(double) + si
 int launch_cf_xi_fp64(const Binning &b, const pg_forest_set &s1, const pg_forest_set &s2,
                       const int64_t *nbr_offsets, const int32_t *nbr_index, const double *nbr_angle,
                       const int32_t *work_order, int64_t num_work, const pg_xi_rows &out,
-                      Scratch *scratch, int num_sms, cudaStream_t stream) {
+                      Scratch *scratch, int num_sms, cudaStream_t stream, bool all_fp64) {
     if (num_work <= 0) return PG_OK;
-    if (runs64_covers(b, s1, s2, num_work))
+    if (!all_fp64 && runs64_covers(b, s1, s2, num_work))
         return launch_cf_xi_runs64(b, s1, s2, nbr_offsets, nbr_index, nbr_angle, work_order,
                                    num_work, out, scratch, num_sms, stream);
     const size_t smem = hist64_bytes(b.nbins);
@@ -301,9 +302,9 @@ int launch_cf_xi_fp64(const Binning &b, const pg_forest_set &s1, const pg_forest
 int launch_xcf_xi_fp64(const Binning &b, const pg_forest_set &forests, const pg_forest_set &objs,
                        const int64_t *nbr_offsets, const int32_t *nbr_index, const double *nbr_angle,
                        const int32_t *work_order, int64_t num_work, const pg_xi_rows &out,
-                       Scratch *scratch, int num_sms, cudaStream_t stream) {
+                       Scratch *scratch, int num_sms, cudaStream_t stream, bool all_fp64) {
     if (num_work <= 0) return PG_OK;
-    if (xruns64_covers(b, forests, num_work))
+    if (!all_fp64 && xruns64_covers(b, forests, num_work))
         return launch_xcf_xi_runs64(b, forests, objs, nbr_offsets, nbr_index, nbr_angle,
                                     work_order, num_work, out, scratch, num_sms, stream);
     const size_t smem = hist64_bytes(b.nbins);
