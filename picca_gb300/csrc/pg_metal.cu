@@ -394,8 +394,9 @@ __global__ void __launch_bounds__(kMrWarps * 32, 5) metal_runs_kernel(
         ordered &= stage_metal<true>(s2, a2, p.o2, n2, ref, ref_a, cp, st, cpm, stm, 1., f2, q2,
                                      max_rho);
         ordered = __syncthreads_and(ordered) != 0;
-        const ParGuard gd = par_guard(&fd, __uint_as_float(max_rho[0]));
-        const ParGuard gm = par_guard(&fm, __uint_as_float(max_rho[1]));
+        const ParGuard gd = par_guard_exact(&fd, __uint_as_float(max_rho[0]));
+        const ParGuard gm = par_guard_exact(&fm, __uint_as_float(max_rho[1]));
+        ordered &= !gd.wide;
         // diagonals j - i that can hold a pair within one bin of the r_par
         // range (both forests in order; else all of them)
         int d_lo = -(n1 - 1), d_hi = n2;
@@ -469,7 +470,7 @@ __global__ void __launch_bounds__(kMrWarps * 32, 5) metal_runs_kernel(
                 const float pp = __fmaf_rn(cp, x.x, y.x), v = fabsf(pp);
                 const float xt = __fmaf_rn(st, x.y, y.y);
                 const float xp0 = (folded ? v : pp) - fd.pc;
-                const float xp = fd.lower_exact ? fmaxf(xp0, gd.low_clamp) : xp0;
+                const float xp = fd.lower_exact ? clamp_low(xp0, gd.low_clamp) : xp0;
                 float rem_p, rem_t;
                 const unsigned ip = round_rem(xp, rem_p), it = round_rem(xt, rem_t);
                 bool near = (fabsf(rem_p) > gd.h_par) | (fabsf(rem_t) > fd.h_tr);
@@ -482,7 +483,7 @@ __global__ void __launch_bounds__(kMrWarps * 32, 5) metal_runs_kernel(
                 const float pa = __fmaf_rn(cpm, x.z, y.z);
                 const float ta = __fmaf_rn(stm, x.w, y.w);
                 const float xa0 = (folded ? fabsf(pa) : pa) - fm.pc;
-                const float xa = fm.lower_exact ? fmaxf(xa0, gm.low_clamp) : xa0;
+                const float xa = fm.lower_exact ? clamp_low(xa0, gm.low_clamp) : xa0;
                 const unsigned mp = round_rem(xa, rem_p), mt = round_rem(ta, rem_t);
                 near |= ok & ((fabsf(rem_p) > gm.h_par) | (fabsf(rem_t) > fm.h_tr));
                 const bool live = in & (x.z < kFar) & (y.z < kFar);
@@ -525,10 +526,26 @@ __global__ void __launch_bounds__(kMrWarps * 32, 5) metal_runs_kernel(
     }
 }
 
-// What the sweeps cover: both forests staged, pixel indices of 16 bits.
-bool metal_runs_covers(const pg_forest_set &s1, const pg_forest_set &s2) {
+struct MetalFast {
+    FastConst data, model;
+};
+
+MetalFast metal_fast(const MetalConst &c) {
+    Binning data = c.b, model = c.b;
+    data.rmu = model.rmu = 0;
+    model.np = c.nmp;
+    model.nt = c.nmt;
+    model.nbins = c.nm;
+    return {make_fast_const(data), make_fast_const(model)};
+}
+
+// What the sweeps cover: both forests staged, pixel indices of 16 bits, bins
+// that FP32 resolves.
+bool metal_runs_covers(const MetalConst &c, const pg_forest_set &s1, const pg_forest_set &s2) {
+    const MetalFast f = metal_fast(c);
     return s1.max_pixels <= 65535 && s2.max_pixels <= 65535 &&
-           mr_smem(s1.max_pixels, s2.max_pixels).total <= kMaxDynSmem;
+           mr_smem(s1.max_pixels, s2.max_pixels).total <= kMaxDynSmem &&
+           fast_const_exact(f.data) && fast_const_exact(f.model);
 }
 
 int launch_metal_runs(const MetalConst &c, const pg_forest_set &s1, const pg_forest_set &s2,
@@ -536,11 +553,7 @@ int launch_metal_runs(const MetalConst &c, const pg_forest_set &s1, const pg_for
                       const int32_t *pair_first, const int32_t *pair_second,
                       const double *pair_angle, int64_t num_pairs, const pg_dmat_sums &out,
                       Scratch *scratch, int num_sms, cudaStream_t stream) {
-    Binning data = c.b, model = c.b;
-    data.rmu = model.rmu = 0;
-    model.np = c.nmp;
-    model.nt = c.nmt;
-    model.nbins = c.nm;
+    const MetalFast fast = metal_fast(c);
     const size_t smem = mr_smem(s1.max_pixels, s2.max_pixels).total;
     cudaError_t err = cudaFuncSetAttribute(
         metal_runs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -552,8 +565,8 @@ int launch_metal_runs(const MetalConst &c, const pg_forest_set &s1, const pg_for
     if (occ < 1) return PG_ERR_UNSUPPORTED;
     const int64_t grid = std::min<int64_t>((int64_t)num_sms * occ, num_pairs);
     metal_runs_kernel<<<(int)grid, kMrWarps * 32, smem, stream>>>(
-        c, make_fast_const(data), make_fast_const(model), s1, s2, a1, a2, pair_first, pair_second,
-        pair_angle, num_pairs, out, scratch, s1.max_pixels, s2.max_pixels);
+        c, fast.data, fast.model, s1, s2, a1, a2, pair_first, pair_second, pair_angle, num_pairs, out,
+        scratch, s1.max_pixels, s2.max_pixels);
     return check_cuda(cudaGetLastError());
 }
 
@@ -579,7 +592,7 @@ int launch_metal_dmat(const pg_corr_params &p, const pg_dmat_params &d, double z
         c.b.x_correlation = 1;
         c.b.remove_shp = 0;
     }
-    if (!xcf && metal_runs_covers(s1, s2))
+    if (!xcf && metal_runs_covers(c, s1, s2))
         return launch_metal_runs(c, s1, s2, a1, a2, pair_first, pair_second, pair_angle,
                                  num_pairs, out, scratch, num_sms, stream);
     int occ = 0;

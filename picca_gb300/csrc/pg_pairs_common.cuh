@@ -12,6 +12,7 @@ namespace {
 constexpr float kMagic = 12582912.0f;        // 1.5 * 2^23
 constexpr unsigned kMagicBits = 0x4B400000u;  // bits of 1.5 * 2^23
 constexpr float kFar = 1e30f;                 // nB, t and z of an empty slot
+constexpr float kMaxGuard = 0.05f;            // widest guard band (in bins)
 // cos(1e-3): above it (angles below 1e-3 rad, and the reference's flat-sky
 // branch below 2 arcsec) the pair kernels take cos and sin of half the angle
 // from the angle itself, not from the half-angle identities
@@ -42,17 +43,31 @@ struct ParGuard {
     float h_par;      // 1/2 - g
     float low_clamp;  // -1/2 + 2 g (auto-correlation with r_par_min = 0)
     float guard_v;    // half-plate cut guard (in units of p)
+    bool wide;        // the band reaches its limit: bins too narrow for FP32
 };
 
 __device__ __forceinline__ ParGuard par_guard(const FastConst *fcp, float max_rho) {
     float g = fcp->g0_par + fcp->g_rho * max_rho;
-    if (!(g < 0.05f)) g = 0.05f;  // absurd bin counts: almost everything is re-decided
     ParGuard pg;
+    pg.wide = !(g < kMaxGuard);
+    if (pg.wide) g = kMaxGuard;  // absurd bin counts: almost everything is re-decided
     pg.h_par = 0.5f - g;
     pg.low_clamp = -0.5f + 2.f * g;
     pg.guard_v = g;
     return pg;
 }
+
+// par_guard for kernels whose every decision has to be the FP64 one: with bins
+// too narrow for FP32 (100,000 of them or more in half a forest) no remainder
+// is certain, and the caller does not skip pairs by FP32 searches.
+__device__ __forceinline__ ParGuard par_guard_exact(const FastConst *fcp, float max_rho) {
+    ParGuard pg = par_guard(fcp, max_rho);
+    if (pg.wide) pg.h_par = -1.f;
+    return pg;
+}
+
+// x, or low where x is below it; NaN stays NaN (decided by no bin).
+__device__ __forceinline__ float clamp_low(float x, float low) { return x < low ? low : x; }
 
 // FP32 value of a weight that stays nonzero when the FP64 weight is nonzero
 // (a weight below the FP32 range still counts its pairs, as in FP64).
@@ -154,7 +169,7 @@ inline FastConst make_fast_const(const Binning &b) {
     double g_tr = 16 * u * (b.nt + 2) + 1e-6;
     // r-mu: r also carries the reciprocal square root and the sum of squares
     if (b.rmu) g_tr = 32 * u * (b.nt + 2) + 1e-6;
-    if (!(g_tr < 0.05)) g_tr = 0.05;
+    if (!(g_tr < (double)kMaxGuard)) g_tr = kMaxGuard;
     fc.h_tr = (float)(0.5 - g_tr);
     fc.guard_z = 1e-5f;  // z1 + z2 < 20: FP32 error below 5e-6
     fc.zmin2 = (float)(2 * b.z_min);
@@ -165,6 +180,13 @@ inline FastConst make_fast_const(const Binning &b) {
     fc.hstride = (b.nbins + 3) & ~3;
     fc.lower_exact = (!b.x_correlation && b.r_par_min == 0.0) ? 1 : 0;
     return fc;
+}
+
+// Whether FP32 decides the bins of any geometry outside the guard bands (bins
+// along r_trans: all but 50,000 of them; r_par depends on the forest, see
+// par_guard_exact).
+[[maybe_unused]] inline bool fast_const_exact(const FastConst &fc) {
+    return fc.h_tr > 0.5f - kMaxGuard && fc.g0_par < kMaxGuard;
 }
 
 }  // namespace

@@ -208,8 +208,9 @@ __global__ void __launch_bounds__(kR64Warps * 32, 2) cf_xi_runs64_kernel(
                            (float)s1.dist_m[a0 + i + 1] >= d;
         }
         if (local_max > 0.f) atomicMax(&max_rho_bits, __float_as_uint(local_max));
-        const bool sorted1 = __syncthreads_and(ordered) != 0;
-        const ParGuard pg = par_guard(&fc, __uint_as_float(max_rho_bits));
+        bool sorted1 = __syncthreads_and(ordered) != 0;
+        const ParGuard pg = par_guard_exact(&fc, __uint_as_float(max_rho_bits));
+        sorted1 &= !pg.wide;
         const float h_par = pg.h_par, low_clamp = pg.low_clamp, h_tr = fc.h_tr, pc = fc.pc;
         const double x1 = s1.x_cart[f1], y1 = s1.y_cart[f1], zc1 = s1.z_cart[f1];
         for (;;) {
@@ -355,7 +356,7 @@ __global__ void __launch_bounds__(kR64Warps * 32, 2) cf_xi_runs64_kernel(
                         const float v = fabsf(pp);
                         const float pv = AUTO ? v : pp;
                         const float xt = __fmaf_rn(st, f1p.y, f2p.y);
-                        const float xp = LOWX ? fmaxf(pv - pc, low_clamp) : pv - pc;
+                        const float xp = LOWX ? clamp_low(pv - pc, low_clamp) : pv - pc;
                         float fp, ft;
                         const unsigned ip = round_rem(xp, fp), it = round_rem(xt, ft);
                         bool near = (fabsf(fp) > h_par) | (fabsf(ft) > h_tr);
@@ -617,7 +618,8 @@ __global__ void __launch_bounds__(kR64Warps * 32, 3) xcf_xi_runs64_kernel(
         for (int i = threadIdx.x; i + 1 < n1; i += blockDim.x)
             sorted1 &= p1[i + 1].x >= p1[i].x && p1[i + 1].y >= p1[i].y;
         sorted1 = __syncthreads_and(sorted1) != 0;
-        const ParGuard pg = par_guard(&fc, __uint_as_float(max_rho_bits));
+        const ParGuard pg = par_guard_exact(&fc, __uint_as_float(max_rho_bits));
+        sorted1 &= !pg.wide;
 
         for (int64_t kb = k_lo; kb < k_hi; kb += kXr64Block) {
             const int nq = (int)min((int64_t)kXr64Block, k_hi - kb);
@@ -746,12 +748,13 @@ __global__ void __launch_bounds__(kR64Warps * 32, 3) xcf_xi_runs64_kernel(
                     bool ok = (ip < np) & (it < nt);
                     if (EXTRA) {
                         const float zs = q.z + zv;
+                        const float gz = fc.guard_z * fmaxf(1.f, 0.05f * fabsf(zs));
                         if (b.zmin_on) {
-                            near |= fabsf(zs - fc.zmin2) < fc.guard_z;
+                            near |= fabsf(zs - fc.zmin2) < gz;
                             ok &= !(zs < fc.zmin2);
                         }
                         if (b.zmax_on) {
-                            near |= fabsf(zs - fc.zmax2) < fc.guard_z;
+                            near |= fabsf(zs - fc.zmax2) < gz;
                             ok &= !(zs > fc.zmax2);
                         }
                     }
@@ -859,13 +862,14 @@ int launch_runs64(const Binning &b, const pg_forest_set &s1, const pg_forest_set
 }  // namespace
 
 // The (r_par, r_trans) geometry with any cut; pixel indices of a queued pair
-// are 16 bits, forest 1 must fit in shared memory, and the work counter (an
-// int) counts slices. The r-mu and angular binnings and longer forests stay
+// are 16 bits, forest 1 must fit in shared memory, the work counter (an int)
+// counts slices, and FP32 has to resolve the bins. The r-mu and angular binnings and longer forests stay
 // on the all-FP64 loop.
 bool runs64_covers(const Binning &b, const pg_forest_set &s1, const pg_forest_set &s2,
                    int64_t num_work) {
     return !b.rmu && !b.ang_corr && s1.max_pixels <= 65535 && s2.max_pixels <= 65535 &&
-           r64_smem(s1.max_pixels).total <= kMaxDynSmem && num_work < (INT32_MAX >> 5);
+           r64_smem(s1.max_pixels).total <= kMaxDynSmem && num_work < (INT32_MAX >> 5) &&
+           fast_const_exact(make_fast_const(b));
 }
 
 int launch_cf_xi_runs64(const Binning &b, const pg_forest_set &s1, const pg_forest_set &s2,
@@ -888,7 +892,8 @@ int launch_cf_xi_runs64(const Binning &b, const pg_forest_set &s1, const pg_fore
 // The same for delta x quasar.
 bool xruns64_covers(const Binning &b, const pg_forest_set &fs, int64_t num_work) {
     return !b.rmu && !b.ang_corr && fs.max_pixels <= 65535 &&
-           xr64_smem(fs.max_pixels).total <= kMaxDynSmem && num_work < (INT32_MAX >> 5);
+           xr64_smem(fs.max_pixels).total <= kMaxDynSmem && num_work < (INT32_MAX >> 5) &&
+           fast_const_exact(make_fast_const(b));
 }
 
 int launch_xcf_xi_runs64(const Binning &b, const pg_forest_set &fs, const pg_forest_set &objs,

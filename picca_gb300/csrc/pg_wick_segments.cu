@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(kWsBlock) wick_list_kernel(
     for (int i = tid; i < n1; i += kWsBlock)
         atomicMax(&max_rho_bits, __float_as_uint(fabsf((float)(s1.r_comov[o1 + i] - r_ref))));
     __syncthreads();
-    const ParGuard pg = par_guard(&fc, __uint_as_float(max_rho_bits));
+    const ParGuard pg = par_guard_exact(&fc, __uint_as_float(max_rho_bits));
     const float pc = fc.pc, h_tr = fc.h_tr;
     // a thread per row: bins, and runs of one bin into the per-bin sums
     for (int i = tid; i < n1; i += kWsBlock) {
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kWsBlock) wick_list_kernel(
         for (int j = 0; j < n2; ++j) {
             const float pp = __fmaf_rn(cp, rho1, rho2[j]);
             const float pv = b.x_correlation ? pp : fabsf(pp);
-            const float xp = fc.lower_exact ? fmaxf(pv - pc, pg.low_clamp) : pv - pc;
+            const float xp = fc.lower_exact ? clamp_low(pv - pc, pg.low_clamp) : pv - pc;
             const float xt = __fmaf_rn(st, d1, tr2[j]);
             float fp, ft;
             const unsigned ip = round_rem(xp, fp), it = round_rem(xt, ft);
