@@ -418,8 +418,9 @@ __global__ void __launch_bounds__(kMrWarps * 32, 5) metal_runs_kernel(
                 atomicMax(&band[1], hi);
             }
             __syncthreads();
-            d_lo = band[0];
-            d_hi = band[1];
+            const bool any = band[0] < band[1];
+            d_lo = any ? band[0] : 0;
+            d_hi = any ? band[1] : 0;
         }
         const bool t_trim = ordered && st > 0.f;
         int head = 0, tail = 0, qn = 0;  // run ring and queue (warp-uniform)
