@@ -626,7 +626,13 @@ typedef struct pg_wick_sums {
  * listed exactly once. work: pg_cf_wick_work_bytes() bytes of device
  * scratch (16-byte aligned; max_ctas: the number of units, for a smaller
  * buffer when there are few); fewer bytes run fewer units at a time. Forests must have
- * at most 32767 pixels. */
+ * at most 32767 pixels.
+ * pg_cf_wick_slices: *useful = 0 where pg_cf_wick with such a buffer takes
+ * pairs over segments of equal bin, up to about 800 pixels: rows of a pair
+ * are then shared out in any case, its slice 0 does all of it and the others
+ * only take room and time, so list each pair once; 1 for longer forests. */
+int pg_cf_wick_slices(pg_plan *plan, const pg_corr_params *params, int32_t max_pixels1,
+                      int32_t max_pixels2, int32_t *useful);
 int pg_cf_wick_work_bytes(pg_plan *plan, const pg_corr_params *params, int32_t max_pixels1,
                           int32_t max_pixels2, int64_t max_ctas, uint64_t *bytes);
 int pg_cf_wick(pg_plan *plan, const pg_corr_params *params, const pg_forest_set *s1,

@@ -715,6 +715,21 @@ int pg_cf_wick_work_bytes(pg_plan *plan, const pg_corr_params *params, int32_t m
     return PG_OK;
 }
 
+int pg_cf_wick_slices(pg_plan *plan, const pg_corr_params *params, int32_t max_pixels1,
+                      int32_t max_pixels2, int32_t *useful) {
+    if (!plan || !useful || max_pixels1 < 1 || max_pixels2 < 1 || max_pixels1 > 32767 ||
+        max_pixels2 > 32767)
+        return PG_ERR_INVALID_ARGUMENT;
+    int nb = 0;
+    const int rc = wick_bins(params, &nb);
+    if (rc) return rc;
+    *useful = wick_segments_covers(nb, max_pixels1, max_pixels2,
+                                   wick_segments_bytes(nb, max_pixels1, max_pixels2, 0))
+                  ? 0
+                  : 1;
+    return PG_OK;
+}
+
 int pg_cf_wick(pg_plan *plan, const pg_corr_params *params, const pg_forest_set *s1,
                const pg_forest_set *s2, const double *zw1, const double *zw2,
                const int64_t *x_offsets1, const double *arena1, const int64_t *x_offsets2,

@@ -468,9 +468,10 @@ uint64_t wick_segments_bytes(int nb, int max1, int max2, int64_t num_pairs) {
     return n * per;
 }
 
-// Lists and V in shared memory: up to about 780 pixels and 9,000 bins; longer
-// forests and finer grids stay on the sweep over listed pairs (wick_t123_kernel),
-// and so does a work buffer that holds no pair's lists.
+// Lists and V in shared memory: up to about 810 pixels (V; the lists hold the
+// 6,000 bins that a call may have up to 3,600 pixels). Longer forests stay on the
+// sweep over listed pairs (wick_t123_kernel), and so does a work buffer that holds
+// no pair's lists.
 bool wick_segments_covers(int nb, int max1, int max2, uint64_t work_bytes) {
     return nb < 65535 && max1 <= 32767 && max2 <= 32767 && list_smem(nb, max2) <= kWsMaxSmem &&
            rows_smem(max1, max2) <= kWsMaxSmem &&

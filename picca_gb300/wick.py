@@ -46,6 +46,8 @@ def _bind():
         lib.pg_cf_wick_work_bytes.restype = ctypes.c_int
         lib.pg_cf_wick_work_bytes.argtypes = [vp, _P(_native.CorrParams), i32, i32, i64,
                                               _P(ctypes.c_uint64)]
+        lib.pg_cf_wick_slices.restype = ctypes.c_int
+        lib.pg_cf_wick_slices.argtypes = [vp, _P(_native.CorrParams), i32, i32, _P(i32)]
         lib.pg_cf_wick.restype = ctypes.c_int
         lib.pg_cf_wick.argtypes = [vp, _P(_native.CorrParams), _P(_native.ForestSetC),
                                    _P(_native.ForestSetC), vp, vp, vp, vp, vp, vp, vp, vp, vp,
@@ -203,11 +205,18 @@ class WickEngine:
 
     def plan_pairs(self, dev, first, second, num_pairs, angles=None):
         """Work units of pg_cf_wick: the forest pairs, costly ones cut into
-        slices (``slice_units``), as device arrays."""
+        slices (``slice_units``) where pg_cf_wick sweeps them, as device
+        arrays."""
         npix = torch.from_numpy(np.asarray(dev.npix, dtype=np.int64)).to(self.device)
         num_pairs = int(num_pairs)
         cost = (npix[first[:num_pairs].long()] * npix[second[:num_pairs].long()]).cpu().numpy()
-        unit, sl, sls = slice_units(cost)
+        # the answer does not depend on the binning: with the most bins
+        most = _pairs.make_params(0.0, 1.0, 1.0, 75, 80, 1.0)
+        useful = ctypes.c_int32()
+        check(_bind().pg_cf_wick_slices(self.engine.plan.handle, ctypes.byref(most),
+                                        int(dev.max_pixels), int(dev.max_pixels),
+                                        ctypes.byref(useful)), "Wick slices")
+        unit, sl, sls = slice_units(cost, MAX_SLICES if useful.value else 1)
         u = torch.from_numpy(unit).to(self.device)
         return {"first": first[u].contiguous(), "second": second[u].contiguous(),
                 "angles": angles[u].contiguous() if angles is not None else None,
@@ -310,12 +319,12 @@ SLICE_TARGET = 2.0e9
 MAX_SLICES = 128
 
 
-def slice_units(cost):
-    """Cut work units into slices by their bound on the sweep, (pixel pairs
-    of the unit)^2: returns (unit index, slice, slices) per entry, costliest
-    slices first."""
+def slice_units(cost, most=None):
+    """Cut work units into slices (``most`` of a unit, MAX_SLICES by default)
+    by their bound on the sweep, (pixel pairs of the unit)^2: returns (unit
+    index, slice, slices) per entry, costliest slices first."""
     cost = np.asarray(cost, dtype=np.float64)
-    slices = np.clip(np.ceil(cost * cost / SLICE_TARGET), 1, MAX_SLICES).astype(np.int64)
+    slices = np.clip(np.ceil(cost * cost / SLICE_TARGET), 1, most or MAX_SLICES).astype(np.int64)
     unit = np.repeat(np.arange(cost.size, dtype=np.int64), slices)
     start = np.concatenate([[0], np.cumsum(slices)[:-1]]) if cost.size else np.zeros(0, np.int64)
     sl = np.arange(unit.size, dtype=np.int64) - np.repeat(start, slices)
