@@ -729,9 +729,10 @@ def wick_leg(args, fs, params, ang_max):
             stats = engine.stats()
         kernel_s = times[-1]
         pairs2 = float(stats.visited_pairs)
-        # the sweep (auto): one FMA per pair of listed pairs; the factored
-        # cross: its GEMM multiply-adds
-        flops = 2.0 * (pairs2 if qs is None else float(stats.gemm_macs))
+        # FP64 operations executed (auto: FMAs over segments and additions of
+        # the row sums; the sweep, which does not count them: an FMA per pair
+        # of listed pairs; the factored cross: its GEMM multiply-adds)
+        flops = 2.0 * (float(stats.gemm_macs) or pairs2)
         achieved = flops / kernel_s / 1e12
         cpu_units, cpu_pairs2, desc, cores = wick_cpu_sample(
             fs, qs, cparams, units, cf1d, min(args.cpu_seconds, 15.0), cross=qs is not None)
@@ -747,9 +748,8 @@ def wick_leg(args, fs, params, ang_max):
             "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak,
                          "unit": "TFLOP/s", "frac": achieved / peak,
                          "peak_source": "cuBLAS DGEMM 4096^3 measured in this run",
-                         "achieved_counts": "2 flops (one FMA) per pair of listed pixel pairs, "
-                         "the reference's count (the kernel sums over segments of equal bin and "
-                         "executes fewer)" if qs is None else "2 flops per GEMM multiply-add (U^T X U, W^T cW; "
+                         "achieved_counts": "2 flops per executed FP64 operation of T3 (FMAs over "
+                         "segments of equal bin, additions of the row sums)" if qs is None else "2 flops per GEMM multiply-add (U^T X U, W^T cW; "
                          "the direct same-quasar sums and the scatter not counted)"},
             "cpu_baseline": {"value": cpu_units, "unit": unit,
                              "pairs_of_pixel_pairs_per_s": cpu_pairs2, "cores": cores,

@@ -127,7 +127,8 @@ typedef struct pg_run_stats {
     int64_t work_items;         /* work items processed; pg_cont_fit_select in
                                    PG_FIT_MIXED: forests finished in two-float */
     int64_t gemm_macs;          /* pg_cf_dmat: multiply-adds of the per-pair
-                                   products of the eta terms               */
+                                   products of the eta terms; pg_cf_wick
+                                   over segments: the FP64 operations of T3 */
     int64_t visited_pairs;      /* FP32_GUARD cf: lane steps of the diagonal
                                    sweeps (pixel pairs evaluated, idle lanes
                                    included)                                   */

@@ -297,6 +297,7 @@ __global__ void __launch_bounds__(kWsBlock, 3) wick_rows_kernel(
     uint32_t *keys = reinterpret_cast<uint32_t *>(x1row + u.max1), *sorted = keys + cap_n;
     int32_t *p_start = reinterpret_cast<int32_t *>(sorted + cap_n);  // [cap_n + 1]
     const int per_pair = u.max1 + u.max2;
+    unsigned long long macs = 0;  // FMAs of T3 and additions of V
     for (;;) {
         __syncthreads();
         if (tid == 0) s_task = atomicAdd(&scratch->work_counter, 1);
@@ -404,6 +405,9 @@ __global__ void __launch_bounds__(kWsBlock, 3) wick_rows_kernel(
             // shared among the warps at bin boundaries
             const int p0 = (int)(sorted[p_start[g0]] >> 16);
             const int lo = l.q_start[p0], hi = l.head[1];
+            if (tid == 0)
+                macs += (unsigned long long)(hi - lo) * min(kWsLanes, bins - g0) +
+                        (unsigned long long)(p_start[min(bins, g0 + kWsLanes)] - my_s0) * n2;
             auto first_bin = [&](int w) {
                 const int target = lo + (int)((int64_t)(hi - lo) * w / kWarps);
                 int a = p0, z = nz;
@@ -456,6 +460,7 @@ __global__ void __launch_bounds__(kWsBlock, 3) wick_rows_kernel(
             }
         }
     }
+    if (tid == 0 && macs) atomicAdd(&scratch->gemm_macs, macs);
 }
 
 }  // namespace
