@@ -71,8 +71,14 @@ def _ptrs(tensors):
 
 
 def _aligned(t, nbytes):
-    """The tensor, or a copy where its storage starts off a wide load's boundary."""
-    return t.clone() if t.data_ptr() % nbytes else t
+    """The tensor, or a copy with the same row stride where its storage starts
+    off a wide load's boundary."""
+    if t.data_ptr() % nbytes == 0:
+        return t
+    if t.dim() != 2:
+        return t.clone()
+    rows, cols = t.shape
+    return t.new_zeros(rows, max(t.stride(0), cols))[:, :cols].copy_(t)
 
 
 class WarmStartMLP:
