@@ -420,7 +420,9 @@ int pg_mlp_gemm(const uint16_t *a, int64_t sam, int64_t sak, const uint16_t *b, 
 int pg_mlp_colsum(const uint16_t *x, int32_t m, int32_t n, int64_t ldx, float *out,
                   void *stream);
 
-/* dy = 2 (y - t) / m as bf16 ([m, n]); loss += sum (y - t)^2 / m if loss. */
+/* dy = 2 (y - t) / m as bf16 ([m, n]); loss += sum (y - t)^2 / m if loss.
+ * (This and the column sums serve other networks: pg_mlp_train_backward
+ * forms both itself.) */
 int pg_mlp_mse_grad(const float *y, const float *t, int32_t m, int32_t n, uint16_t *dy,
                     float *loss, void *stream);
 

@@ -385,7 +385,7 @@ void add_bias(GemmGroup &grp, const __nv_bfloat16 *x, int m, int n, int ld, floa
 }
 
 // 64 x 64 tiles load half the operand bytes per product of 32 x 32 ones; the
-// small tiles are taken where the large ones would not reach every SM (152):
+// small tiles are taken where the large ones would not reach every SM (of 152):
 // a layer of batch 4,096 (256 large tiles) takes 8.6 us in 64 x 64 and 14.3 us
 // in 32 x 32 tiles, its weight gradients (40 large tiles) 39.9 us and 27.6 us.
 // Stages: a stage is 16 KB and one of them is being read, so a K <= 256
@@ -419,7 +419,12 @@ int launch_group(GemmGroup &grp, cudaStream_t stream) {
     int64_t large = 0;
     for (int p = 0; p < grp.count; ++p)
         large += ((int64_t)(grp.g[p].m + 63) / 64) * ((grp.g[p].n + 63) / 64);
-    return large >= 152 ? launch_tiles<64>(grp, stream) : launch_tiles<32>(grp, stream);
+    int device = 0, sms = 0;
+    cudaError_t err = cudaGetDevice(&device);
+    if (err == cudaSuccess)
+        err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (err != cudaSuccess) return check_cuda(err);
+    return large >= sms ? launch_tiles<64>(grp, stream) : launch_tiles<32>(grp, stream);
 }
 
 // ---------------------------------------------------------------------------
