@@ -386,7 +386,8 @@ __global__ void __launch_bounds__(kMrWarps * 32, 5) metal_runs_kernel(
         }
         const int n1 = (int)n1_64, n2 = (int)n2_64;
         if (n1 < 1 || n2 < 1) continue;
-        const double ref = s1.r_comov[p.o1 + n1 / 2], ref_a = a1.r_comov[p.o1 + n1 / 2];
+        const double ref = reference_distance(s1.r_comov[p.o1 + n1 / 2], &max_rho[0]);
+        const double ref_a = reference_distance(a1.r_comov[p.o1 + n1 / 2], &max_rho[1]);
         const float cp = (float)(p.cc * fd.inv_p), st = (float)(p.ss * fd.inv_t);
         const float cpm = (float)(p.cc * fm.inv_p), stm = (float)(p.ss * fm.inv_t);
         bool ordered = stage_metal<false>(s1, a1, p.o1, n1, ref, ref_a, cp, st, cpm, stm,

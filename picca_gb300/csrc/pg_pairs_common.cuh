@@ -66,6 +66,15 @@ __device__ __forceinline__ ParGuard par_guard_exact(const FastConst *fcp, float 
     return pg;
 }
 
+// The distance that a forest's others are taken relative to: its middle pixel's,
+// or 0 where that is not a number or infinite; *max_rho_bits then starts at
+// infinity, so that the band is wide.
+__device__ __forceinline__ double reference_distance(double middle, unsigned *max_rho_bits) {
+    if (isfinite(middle)) return middle;
+    atomicMax(max_rho_bits, 0x7F800000u);
+    return 0.;
+}
+
 // x, or low where x is below it; NaN stays NaN (decided by no bin).
 __device__ __forceinline__ float clamp_low(float x, float low) { return x < low ? low : x; }
 

@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kR64Warps * 32, 2) cf_xi_runs64_kernel(
         }
         const int n1 = (int)n1_64;
         if (n1 < 1 || k_lo == k_hi) continue;
-        const double r_ref = s1.r_comov[a0 + n1 / 2];
+        const double r_ref = reference_distance(s1.r_comov[a0 + n1 / 2], &max_rho_bits);
         // forest 1: FP32 relative to its middle pixel, and FP64
         bool ordered = true;
         float local_max = 0.f;
@@ -598,7 +598,7 @@ __global__ void __launch_bounds__(kR64Warps * 32, 3) xcf_xi_runs64_kernel(
         if (threadIdx.x == 0)
             ctx = {a0, 0, fs.x_cart[f], fs.y_cart[f], fs.z_cart[f], fs.ra[f], fs.dec[f],
                    fs.cos_dec[f]};
-        const double r_ref = fs.r_comov[a0 + n1 / 2];
+        const double r_ref = reference_distance(fs.r_comov[a0 + n1 / 2], &max_rho_bits);
         float local_max = 0.f;
         for (int i = threadIdx.x; i < n1; i += blockDim.x) {
             const double w = fs.weights[a0 + i], r = fs.r_comov[a0 + i];

@@ -161,7 +161,8 @@ __global__ void __launch_bounds__(kWsBlock) wick_list_kernel(
                                 s2.dec[g]);
     const double cc = cos(ang / 2), ss = sin(ang / 2);
     const float cp = (float)(cc * fc.inv_p), st = (float)(ss * fc.inv_t);
-    const double r_ref = s1.r_comov[o1 + n1 / 2];
+    __syncthreads();  // max_rho_bits
+    const double r_ref = reference_distance(s1.r_comov[o1 + n1 / 2], &max_rho_bits);
     for (int k = tid; k < nb; k += kWsBlock) {
         wall[k] = t1[k] = 0.;
         count[k] = 0;
