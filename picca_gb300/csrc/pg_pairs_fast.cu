@@ -406,19 +406,6 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
         const int item = FEW ? unit / slices : unit, slice = FEW ? unit - item * slices : 0;
         const int64_t f1 = work_order ? work_order[item] : item;
         const int32_t row = s1.row[f1];
-        // this slice's neighbours, each in up to kCfParts parts of its
-        // diagonals so that a slice has at least two tasks for every warp (a
-        // part stages the neighbour again; the runs stay whole)
-        const int64_t k0 = nbr_offsets[f1], nk = nbr_offsets[f1 + 1] - k0;
-        int64_t k_lo = k0, k1 = k0 + nk;
-        int part_bits = 0;
-        if (FEW) {
-            const int cut = (int)max((int64_t)1, min((int64_t)slices, nk * kCfParts / (2 * nwarps)));
-            if (slice >= cut) continue;
-            k_lo = k0 + nk * slice / cut;
-            k1 = k0 + nk * (slice + 1) / cut;
-            while (1 << part_bits < kCfParts && (k1 - k_lo) << part_bits < 2 * nwarps) ++part_bits;
-        }
         const int64_t a0 = s1.pix_offset[f1];
         const int64_t n1_64 = s1.pix_offset[f1 + 1] - a0;
         if (n1_64 > max_pix1 || n1_64 > 65535 || n1_64 < 1) {
@@ -426,6 +413,27 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
             continue;
         }
         const int n1 = (int)n1_64;
+        // this slice's neighbours, each in up to kCfParts parts of its
+        // diagonals so that a slice has at least two tasks for every warp (a
+        // part stages the neighbour again; the runs stay whole). A neighbour has
+        // as many parts as groups of 32 diagonals within r_par_max, by the mean
+        // spacing of forest 1's pixels: 40 forests to 20 Mpc/h, 135 us with parts
+        // that found none
+        const int64_t k0 = nbr_offsets[f1], nk = nbr_offsets[f1 + 1] - k0;
+        int64_t k_lo = k0, k1 = k0 + nk;
+        int part_bits = 0;
+        if (FEW) {
+            const float span = (float)fabs(s1.r_comov[a0 + n1 - 1] - s1.r_comov[a0]);
+            const float diagonals = fminf(2.f * p_hi * (float)(n1 - 1) / (span * (float)fcp->geom_p),
+                                          2.f * (float)n1);
+            int most = 1;
+            while (most < kCfParts && (float)(2 * most) * 32.f <= diagonals) most *= 2;
+            const int cut = (int)max((int64_t)1, min((int64_t)slices, nk * most / (2 * nwarps)));
+            if (slice >= cut) continue;
+            k_lo = k0 + nk * slice / cut;
+            k1 = k0 + nk * (slice + 1) / cut;
+            while (1 << part_bits < most && (k1 - k_lo) << part_bits < 2 * nwarps) ++part_bits;
+        }
         // forest 1 in FP32 relative to the distance of its middle pixel
         const double r_ref = s1.r_comov[a0 + n1 / 2];
         if (threadIdx.x == 0) {
@@ -1255,13 +1263,15 @@ int launch_cf_xi_fast(const Binning &b, double ang_max, const pg_forest_set &s1,
     int grid = 0;
     // few forests: several CTAs share one, each with a slice of its
     // neighbours (a slice costs a staging and a flush), and few neighbours are
-    // cut into parts for the warps. 150 forests: 1.32 ms for the kernel with whole
-    // forests, 0.96 ms in up to four slices of whole neighbours, 0.86 ms with up
-    // to eight parts (four parts 0.91 ms). Parts of the pixels instead of the
-    // diagonals, 0.83 ms, cut the runs and so round their FP32 sums otherwise.
-    // A kernel of its own (FEW): the parts cost the sweeps of many forests 0.8 %
+    // cut into parts for the warps. 150 forests: 1.68 ms for the kernel with
+    // whole forests, 0.92 ms in two slices and up to eight parts (four slices
+    // 1.05 ms). The line: up to 1.5 slices an SM, 220 forests take 2.29 ms whole
+    // and 1.66 ms in slices, 300 forests 3.17 ms whole and 3.38 ms in slices.
+    // Parts of the pixels instead of the diagonals cut the runs and so round
+    // their FP32 sums otherwise. A kernel of its own (FEW): the parts cost the
+    // sweeps of many forests 0.8 %
     int slices = 1;
-    while (slices < 4 && num_work * slices < 4 * (int64_t)num_sms) slices *= 2;
+    while (slices < 4 && 2 * num_work * slices < 3 * (int64_t)num_sms) slices *= 2;
 #define PG_LAUNCH_CF_F(A, E, L, R, F)                                                           \
     rc = persistent_grid(cf_xi_diag_kernel<A, E, L, R, F>, block, smem, num_sms,               \
                          num_work * slices, &grid, tuning.blocks_per_sm);                      \

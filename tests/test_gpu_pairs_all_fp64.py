@@ -52,3 +52,13 @@ def test_groups(quasars):
     assert _compare(fs, qs, dict(r_par_min=-200.0, r_par_max=200.0, r_trans_max=200.0,
                                  num_bins_r_par=100, num_bins_r_trans=50,
                                  x_correlation=True)) > 0
+
+
+@pytest.mark.parametrize("forests,r_max,bins", [(30, 20.0, 10), (3, 20.0, 10), (30, 80.0, 20),
+                                                (2, 2.0, 1), (120, 60.0, 15)])
+def test_few_short_range(forests, r_max, bins):
+    """Few diagonals within r_par_max: fewer parts a neighbour, down to one."""
+    from picca_gb300 import synthetic
+    fs = synthetic.make_forests(forests, 3, (150.0, 150.4), (0.0, 0.4), 2.4, 2.6, "uniform")
+    assert _compare(fs, None, dict(r_par_min=0.0, r_par_max=r_max, r_trans_max=200.0,
+                                   num_bins_r_par=bins, num_bins_r_trans=50)) > 0
