@@ -110,18 +110,27 @@ __device__ __forceinline__ void flush_rows(float *h, const FastConst &fc, const 
         if (nb == 0) continue;
         // four FP64 operations a bin (conversions on the integer pipe, the
         // scales as products; with divisions and FP64-pipe conversions a flush
-        // of 2,500 bins was about 35 operations a bin, 23 us of the pipe); sums
-        // below the FP32 normal range, whose pairs count like others, on the FP64
-        // pipe, which keeps them
-        auto at = [&](int k) {
-            const float v = h[k * hs + b];
-            return v != 0.f && fabsf(v) < 1.17549435e-38f ? (double)v : f32_to_f64(v);
-        };
-        atomicAdd(&out.weights[o + b], at(H_WE) + at(H_WEL));
-        atomicAdd(&out.xi[o + b], at(H_XI) + at(H_XIL));
-        atomicAdd(&out.r_par[o + b], at(H_PW) * per_p);
-        atomicAdd(&out.r_trans[o + b], at(H_TW) * per_t);
-        atomicAdd(&out.z[o + b], 0.5 * at(H_ZW));
+        // of 2,500 bins was about 35 operations a bin, 23 us of the pipe)
+        float v[H_NB];
+        bool small = false;  // a sum below the FP32 normal range
+#pragma unroll
+        for (int k = 0; k < H_NB; ++k) {
+            v[k] = h[k * hs + b];
+            small |= (__float_as_uint(v[k]) & 0x7FFFFFFFu) - 1u < 0x7FFFFFu;
+        }
+        if (!small) {
+            atomicAdd(&out.weights[o + b], f32_to_f64(v[H_WE]) + f32_to_f64(v[H_WEL]));
+            atomicAdd(&out.xi[o + b], f32_to_f64(v[H_XI]) + f32_to_f64(v[H_XIL]));
+            atomicAdd(&out.r_par[o + b], f32_to_f64(v[H_PW]) * per_p);
+            atomicAdd(&out.r_trans[o + b], f32_to_f64(v[H_TW]) * per_t);
+            atomicAdd(&out.z[o + b], f32_to_f64(0.5f * v[H_ZW]));
+        } else {  // its pairs count like others: the FP64 pipe's conversions keep it
+            atomicAdd(&out.weights[o + b], (double)v[H_WE] + (double)v[H_WEL]);
+            atomicAdd(&out.xi[o + b], (double)v[H_XI] + (double)v[H_XIL]);
+            atomicAdd(&out.r_par[o + b], (double)v[H_PW] * per_p);
+            atomicAdd(&out.r_trans[o + b], (double)v[H_TW] * per_t);
+            atomicAdd(&out.z[o + b], 0.5 * (double)v[H_ZW]);
+        }
         atomicAdd((unsigned long long *)&out.num_pairs[o + b], (unsigned long long)nb);
 #pragma unroll
         for (int k = 0; k < H_NB; ++k) h[k * hs + b] = 0.f;
