@@ -424,19 +424,19 @@ __global__ void __launch_bounds__(kCfBlock, 1) cf_xi_diag_kernel(
         const int n1 = (int)n1_64;
         // this slice's neighbours, each in up to kCfParts parts of its
         // diagonals so that a slice has at least two tasks for every warp (a
-        // part stages the neighbour again; the runs stay whole). A neighbour has
-        // as many parts as groups of 32 diagonals within r_par_max, by the mean
-        // spacing of forest 1's pixels: 40 forests to 20 Mpc/h, 135 us with parts
-        // that found none
+        // part stages the neighbour again; the runs stay whole), but no more than
+        // groups of 32 diagonals within r_par_max, by the mean spacing of forest
+        // 1's pixels (40 forests to 20 Mpc/h: 137 us with parts that found none,
+        // 74 us; whole neighbours 75 us)
         const int64_t k0 = nbr_offsets[f1], nk = nbr_offsets[f1 + 1] - k0;
         int64_t k_lo = k0, k1 = k0 + nk;
         int part_bits = 0;
         if (FEW) {
             const float span = (float)fabs(s1.r_comov[a0 + n1 - 1] - s1.r_comov[a0]);
             const float diagonals = fminf(2.f * p_hi * (float)(n1 - 1) / (span * (float)fcp->geom_p),
-                                          2.f * (float)n1);
+                                          (float)(n1 + s2.max_pixels));
             int most = 1;
-            while (most < kCfParts && (float)(2 * most) * 32.f <= diagonals) most *= 2;
+            while (most < kCfParts && (float)(32 * most) < diagonals) most *= 2;
             const int cut = (int)max((int64_t)1, min((int64_t)slices, nk * most / (2 * nwarps)));
             if (slice >= cut) continue;
             k_lo = k0 + nk * slice / cut;
@@ -1272,15 +1272,16 @@ int launch_cf_xi_fast(const Binning &b, double ang_max, const pg_forest_set &s1,
     int grid = 0;
     // few forests: several CTAs share one, each with a slice of its
     // neighbours (a slice costs a staging and a flush), and few neighbours are
-    // cut into parts for the warps. 150 forests: 1.68 ms for the kernel with
-    // whole forests, 0.92 ms in two slices and up to eight parts (four slices
-    // 1.05 ms). The line: up to 1.5 slices an SM, 220 forests take 2.29 ms whole
-    // and 1.66 ms in slices, 300 forests 3.17 ms whole and 3.38 ms in slices.
-    // Parts of the pixels instead of the diagonals cut the runs and so round
-    // their FP32 sums otherwise. A kernel of its own (FEW): the parts cost the
-    // sweeps of many forests 0.8 %
+    // cut into parts for the warps. 150 forests: 1.69 ms for the kernel with
+    // whole forests, 1.05 ms in up to four slices and eight parts. Two slices of
+    // them take 0.92 ms, and 300 to 600 forests are up to 4 % faster whole, but
+    // a block's FP32 sums then hold two to four times the terms (r_par, r_trans
+    // and z sums 1.2e-8 off 64 bits in four slices, 1.5e-8 in two). Parts of the
+    // pixels instead of the diagonals cut the runs and so round their FP32 sums
+    // otherwise. A kernel of its own (FEW): the parts cost the sweeps of many
+    // forests 0.8 %
     int slices = 1;
-    while (slices < 4 && 2 * num_work * slices < 3 * (int64_t)num_sms) slices *= 2;
+    while (slices < 4 && num_work * slices < 4 * (int64_t)num_sms) slices *= 2;
 #define PG_LAUNCH_CF_F(A, E, L, R, F)                                                           \
     rc = persistent_grid(cf_xi_diag_kernel<A, E, L, R, F>, block, smem, num_sms,               \
                          num_work * slices, &grid, tuning.blocks_per_sm);                      \
