@@ -471,9 +471,11 @@ int launch_fit64(const pg_spectra &sp, const pg_cont_model &m, const double *sta
     // 100 forests in CTAs of 16 warps: 785 us, 434 us spread)
     const int64_t share = (count + num_sms - 1) / num_sms;
     const int warps = (int)(share < fit64_warps<K>() ? share : fit64_warps<K>());
-    const size_t smem = (size_t)warps * 6 * 32 * K * sizeof(double);
-    cudaError_t err = cudaFuncSetAttribute(
-        cont_fit64_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr size_t warp_bytes = (size_t)6 * 32 * K * sizeof(double);
+    const size_t smem = warps * warp_bytes;
+    cudaError_t err = cudaFuncSetAttribute(cont_fit64_kernel<K>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)(fit64_warps<K>() * warp_bytes));
     if (err != cudaSuccess) return check_cuda(err);
     int64_t blocks = (count + warps - 1) / warps;
     if (blocks > num_sms) blocks = num_sms;
@@ -2005,6 +2007,8 @@ int launch_cont_fit(const pg_spectra &sp, const pg_cont_model &m, const double *
     return check_cuda(err);
 }
 
+constexpr size_t kStackLimit = 200 * 1024;  // shared memory of a block
+
 // Blocks of BLOCK threads as many as are resident; the variance-function table
 // where it fits beside the histograms.
 template <bool EXACT, int BLOCK>
@@ -2014,7 +2018,7 @@ static int launch_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_
     const auto kernel = cont_stacks_kernel<EXACT, BLOCK>;
     const size_t smem = stack_bytes(st, EXACT, use_table);
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem);
+                                           (int)kStackLimit);
     if (err != cudaSuccess) return check_cuda(err);
     int per_sm = 0;
     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, BLOCK, smem);
@@ -2028,8 +2032,6 @@ static int launch_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_
         sp, m, fit, st, scratch, use_table, exact_work);
     return check_cuda(cudaGetLastError());
 }
-
-constexpr size_t kStackLimit = 200 * 1024;  // shared memory of a block
 
 // 16 bytes of shared memory a cell, 32 of the work
 size_t cont_exact_bytes() { return 2 * kStackLimit; }
@@ -2108,7 +2110,8 @@ int launch_cont_deltas(const pg_spectra &sp, const pg_cont_model &m, const pg_co
         return check_cuda(cudaGetLastError());
     }
     cudaError_t err = cudaFuncSetAttribute(cont_deltas_kernel<true>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)kMaxDynSmem);
     if (err != cudaSuccess) return check_cuda(err);
     cont_deltas_kernel<true><<<blocks, kContBlock, smem, stream>>>(sp, m, fit, delta, weights);
     return check_cuda(cudaGetLastError());

@@ -19,7 +19,9 @@ constexpr double kPi = 3.141592653589793;
 constexpr double kSmallAngle = 2. / 3600. * 3.141592653589793 / 180.;
 
 // Dynamic shared memory of a CTA: the 227 KB of an SM less what the kernels'
-// static arrays take (at most 1,360 bytes).
+// static arrays take (at most 1,360 bytes). Kernels with a limit of their own
+// set the same one on each call, whatever the call needs: the attribute belongs
+// to the kernel, and another thread's call may be between it and its launch.
 constexpr size_t kMaxDynSmem = 227 * 1024 - 1536;
 
 // Scratch owned by a plan (device memory, a few hundred bytes).

@@ -558,7 +558,7 @@ int launch_metal_runs(const MetalConst &c, const pg_forest_set &s1, const pg_for
     const MetalFast fast = metal_fast(c);
     const size_t smem = mr_smem(s1.max_pixels, s2.max_pixels).total;
     cudaError_t err = cudaFuncSetAttribute(
-        metal_runs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        metal_runs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynSmem);
     if (err != cudaSuccess) return check_cuda(err);
     int occ = 0;
     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, metal_runs_kernel, kMrWarps * 32,

@@ -822,7 +822,7 @@ int launch_xruns64(const Binning &b, const pg_forest_set &fs, const pg_forest_se
     auto kernel = xcf_xi_runs64_kernel<EXTRA>;
     const size_t smem = xr64_smem(fs.max_pixels).total;
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem);
+                                           (int)kMaxDynSmem);
     if (err != cudaSuccess) return check_cuda(err);
     int per_sm = 0;
     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kR64Warps * 32, smem);
@@ -845,7 +845,7 @@ int launch_runs64(const Binning &b, const pg_forest_set &s1, const pg_forest_set
     auto kernel = cf_xi_runs64_kernel<AUTO, EXTRA, LOWX>;
     const size_t smem = r64_smem(s1.max_pixels).total;
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem);
+                                           (int)kMaxDynSmem);
     if (err != cudaSuccess) return check_cuda(err);
     int per_sm = 0;
     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kR64Warps * 32, smem);

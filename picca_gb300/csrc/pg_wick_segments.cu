@@ -507,10 +507,10 @@ int launch_wick_segments(const pg_corr_params &p, const pg_forest_set &s1,
     u.nb = b.nbins;
     const size_t smem_a = list_smem(u.nb, u.max2), smem_b = rows_smem(u.max1, u.max2);
     cudaError_t err = cudaFuncSetAttribute(
-        wick_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_a);
+        wick_list_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWsMaxSmem);
     if (err != cudaSuccess) return check_cuda(err);
     err = cudaFuncSetAttribute(wick_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)smem_b);
+                               (int)kWsMaxSmem);
     if (err != cudaSuccess) return check_cuda(err);
     int occ = 0;
     err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, wick_rows_kernel, kWsBlock, smem_b);
