@@ -1326,17 +1326,21 @@ __global__ void __launch_bounds__(32 * kRefineWarps) cont_fit_refine_kernel(
 // the blocks, so that a sum does not depend on the order of its terms: the
 // same inputs give the same bits. With pairs the model of the next iteration
 // moved by its last bits from run to run, and the FP32 decisions of the mixed
-// fit on it moved single forests by up to 1e-6. A term of 2^kFineTop or more
-// goes to a second fixed-point number of its bin in global memory (last place
-// 2^-kCoarseScale), one of 2^kCoarseTop or more, or none, straight to the FP64
-// result. Calls whose words do not fit in shared memory keep the pairs. 1,024
+// fit on it moved single forests by up to 1e-6. Two more numbers of a bin in
+// global memory, with other last places, take the terms of 2^kFineTop and more
+// and what terms below 2^kFineLow have under the first one's last place, so that
+// every sum keeps the 2^-50 of its terms; terms of 2^kCoarseTop and more, below
+// 2^-78, or none go straight to the FP64 result. Calls whose words do not fit in shared memory keep the pairs. 1,024
 // threads (a block an SM; 512 leave the chains of word adds less to overlap
 // with). Five passes over 40,000 forests of 160 pixels: 1.45 ms in pairs, 1.67 ms
 // exact (1.95 ms in blocks of 512).
 constexpr int kStackBlock = 512;
 constexpr int kStackGroup = 8;
-constexpr int kFixScale = 88, kFineTop = 14;      // 2^25 terms of 2^14 stay below 2^39
-constexpr int kCoarseScale = 56, kCoarseTop = 46;  // and 2^25 of 2^46 below 2^71
+// 2^25 terms at the top of each range stay below 2^(127 - scale)
+constexpr int kFixScale = 88, kFineLow = -39, kFineTop = 14;
+constexpr int kCoarseScale = 56, kCoarseTop = 46;
+constexpr int kSmallScale = 168;  // parts below 2^-kFixScale
+constexpr int kStackNumbers = 3;  // of a cell in global memory
 
 struct StackSlot {
     int64_t off;
@@ -1403,35 +1407,28 @@ __device__ __forceinline__ void fix_add_words(uint32_t *const h[N], int stride,
     }
 }
 
-// v in units of 2^-SCALE (to 2^-50 of v, and to a unit), |v| < 2^(102 - SCALE).
-template <int SCALE>
-__device__ __forceinline__ void fix_words(dfl v, uint32_t word[4]) {
-    const uint32_t u = __float_as_uint(v.hi);
-    const int e = (int)((u >> 23) & 0xFFu);
-    long long t;
-    int p = 0;
-    if (e >= 64) {
-        // t = v 2^(176 - e), the last place of hi at bit 26
-        const long long m = (u & 0x7FFFFFu) | 0x800000u;
-        const float lo = v.lo * __uint_as_float((uint32_t)(303 - e) << 23);
-        t = ((int)u < 0 ? -m : m) * (1LL << 26) + __float2int_rn(lo);
-        p = e - 176 + SCALE;
-        if (p < 0) {
-            t = (t + (1LL << (-p - 1))) >> -p;
-            p = 0;
-        }
-    } else {  // below 2^-63
-        t = __double2ll_rn(ldexp((double)v.hi + (double)v.lo, SCALE));
-    }
+// t 2^p as four words, |t| < 2^51, 0 <= p < 64 (WIDE: 96).
+template <bool WIDE>
+__device__ __forceinline__ void fix_words(long long t, int p, uint32_t word[4]) {
     const int s = p & 31;
     const unsigned long long low = (unsigned long long)t << s;
     const uint32_t a = (uint32_t)low, b = (uint32_t)(low >> 32);
     const uint32_t c = (uint32_t)((t >> 32) >> (32 - s));  // from bit 64 on
-    const bool up = p >= 32;
+    const uint32_t sign = (uint32_t)(t >> 63);
+    const bool up = p >= 32, upper = WIDE && p >= 64;
     word[0] = up ? 0u : a;
-    word[1] = up ? a : b;
-    word[2] = up ? b : c;
-    word[3] = up ? c : (uint32_t)(t >> 63);
+    word[1] = upper ? 0u : (up ? a : b);
+    word[2] = upper ? a : (up ? b : c);
+    word[3] = upper ? b : (up ? c : sign);
+}
+
+// v = t 2^(e - 176) to 2^-50 of it, the last place of v.hi at bit 26 of t (e:
+// exponent of v.hi, 49 to 254).
+__device__ __forceinline__ long long fix_digits(dfl v, int e) {
+    const uint32_t u = __float_as_uint(v.hi);
+    const long long m = (u & 0x7FFFFFu) | 0x800000u;
+    const float lo = v.lo * __uint_as_float((uint32_t)(303 - e) << 23);
+    return ((int)u < 0 ? -m : m) * (1LL << 26) + __float2int_rn(lo);
 }
 
 // The number in four words, in units of 2^-scale.
@@ -1447,20 +1444,37 @@ __device__ __forceinline__ double fix_value(const uint32_t word[4], int scale) {
     return negative ? -v : v;
 }
 
-// A term of 2^kFineTop or more: to its bin's coarse number, or (with infinities
-// and NaN) to the FP64 result.
-__device__ __noinline__ void stack_add_large(uint32_t *coarse, int stride, double *dst, dfl v) {
-    if (fabsf(v.hi) < (float)(1LL << kCoarseTop)) {
-        uint32_t word[1][4];
-        fix_words<kCoarseScale>(v, word[0]);
-        fix_add_words<1>(&coarse, stride, word);
-    } else {
+// The terms that the fine number alone does not hold: of 2^kFineTop or more to
+// the bin's coarse number; below 2^kFineLow the part in units of 2^-kFixScale to
+// the fine number (of the block, at fine) and what is left of it to the small
+// number; infinities, NaN and what no number holds to the FP64 result.
+__device__ __noinline__ void stack_add_rare(uint32_t *fine, uint32_t *work, int nc, int cell,
+                                            double *dst, dfl v) {
+    const int e = (int)((__float_as_uint(v.hi) >> 23) & 0xFFu);
+    uint32_t word[1][4];
+    if (e >= 127 + kCoarseTop || e < 127 - 78) {
         atomicAdd(dst, (double)v.hi + (double)v.lo);
+        return;
     }
+    const long long t = fix_digits(v, e);
+    uint32_t *at[1] = {work + 4 * nc + cell};
+    if (e >= 127 + kFineTop) {
+        fix_words<false>(t, e - 176 + kCoarseScale, word[0]);
+        fix_add_words<1>(at, nc, word);
+        return;
+    }
+    const int below = 176 - kFixScale - e;  // bits of t below the fine number's last place
+    const long long whole = t >> below;
+    uint32_t *at_fine[1] = {fine};
+    fix_words<false>(whole, 0, word[0]);
+    fix_add_words<1>(at_fine, nc, word);
+    at[0] = work + 8 * nc + cell;
+    fix_words<true>(t - whole * (1LL << below), e - 176 + kSmallScale, word[0]);
+    fix_add_words<1>(at, nc, word);
 }
 
-// exact_work (EXACT): 2 x 4 words of every cell, zeroed, the second four the
-// terms of 2^kFineTop and more.
+// exact_work (EXACT): kStackNumbers x 4 words of every cell, zeroed: the blocks'
+// sums, the terms of 2^kFineTop and more, the parts below 2^-kFixScale.
 template <bool EXACT, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) cont_stacks_kernel(
     const __grid_constant__ pg_spectra sp, const __grid_constant__ pg_cont_model m,
@@ -1495,10 +1509,13 @@ __global__ void __launch_bounds__(BLOCK) cont_stacks_kernel(
         uint32_t *at[N], word[N][4];
 #pragma unroll
         for (int n = 0; n < N; ++n) {
-            const bool fine = fabsf(v[n].hi) < (float)(1 << kFineTop);
+            const int e = (int)((__float_as_uint(v[n].hi) >> 23) & 0xFFu);
+            const bool fine = e >= 127 + kFineLow && e < 127 + kFineTop;
             at[n] = hist + cell[n];
-            fix_words<kFixScale>(fine ? v[n] : dfl{0.f, 0.f}, word[n]);
-            if (!fine) stack_add_large(exact_work + 4 * nc + cell[n], nc, dst[n], v[n]);
+            fix_words<false>(fine ? fix_digits(v[n], e) : 0, fine ? e - 176 + kFixScale : 0,
+                             word[n]);
+            if (!fine && v[n].hi != 0.f)
+                stack_add_rare(hist + cell[n], exact_work, nc, cell[n], dst[n], v[n]);
         }
         fix_add_words<N>(at, nc, word);
     };
@@ -1776,13 +1793,11 @@ __global__ void cont_stacks_finish_kernel(const __grid_constant__ pg_cont_stacks
     else if (k < c.v_d2) { dst = st.var_mean; from = c.v_mean; }
     else if (k < c.v_d4) { dst = st.var_delta2; from = c.v_d2; }
     else { dst = st.var_delta4; from = c.v_d4; }
-    uint32_t fine[4], coarse[4];
+    uint32_t word[kStackNumbers][4];
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-        fine[w] = exact_work[w * nc + k];
-        coarse[w] = exact_work[(4 + w) * nc + k];
-    }
-    dst[k - from] += fix_value(fine, kFixScale) + fix_value(coarse, kCoarseScale);
+    for (int w = 0; w < kStackNumbers * 4; ++w) word[w >> 2][w & 3] = exact_work[w * nc + k];
+    dst[k - from] += fix_value(word[0], kFixScale) + fix_value(word[1], kCoarseScale) +
+                     fix_value(word[2], kSmallScale);
 }
 
 // Deltas and weights (populate_los_ids, extract_deltas). Bound: the FP64 pipe.
@@ -2033,8 +2048,8 @@ static int launch_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_
     return check_cuda(cudaGetLastError());
 }
 
-// 16 bytes of shared memory a cell, 32 of the work
-size_t cont_exact_bytes() { return 2 * kStackLimit; }
+// 16 bytes of shared memory a cell, as many of the work for each number
+size_t cont_exact_bytes() { return kStackNumbers * kStackLimit; }
 
 int launch_cont_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_cont_fit &fit,
                        const pg_cont_stacks &st, uint32_t *exact_work, size_t exact_bytes,
@@ -2046,7 +2061,7 @@ int launch_cont_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_co
     const bool pair_table = want_table && stack_smem_bytes(st, true) <= limit;
     if (stack_smem_bytes(st, pair_table) > limit) return PG_ERR_UNSUPPORTED;
     const StackCells cells = stack_cells(st);
-    const size_t work = (size_t)cells.total * 32;
+    const size_t work = (size_t)cells.total * 16 * kStackNumbers;
     if (stack_bytes(st, true, false) > limit || work > exact_bytes)
         return launch_stacks<false, kStackBlock>(sp, m, fit, st, pair_table, nullptr, scratch,
                                                  num_sms, stream);

@@ -67,7 +67,7 @@ def test_loop(wave):
         assert np.array_equal(a, b, equal_nan=True), k
 
 
-@pytest.mark.parametrize("eta", [1.0, 1e-6, 1e-16])
+@pytest.mark.parametrize("eta", [1.0, 1e-6, 1e-16, 1e10, 1e18, 1e26])
 def test_values(eta):
     from picca_gb300 import continuum
     raw, spectra = _spectra(800, "log")
