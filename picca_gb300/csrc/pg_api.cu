@@ -36,8 +36,9 @@ void *fast_const_of(pg_plan *plan) {
     return static_cast<char *>(plan->scratch) + ((sizeof(Scratch) + 255) & ~(size_t)255);
 }
 
-uint32_t *exact_work_of(pg_plan *plan) {
-    return reinterpret_cast<uint32_t *>(static_cast<char *>(plan->scratch) + exact_offset());
+unsigned long long *exact_work_of(pg_plan *plan) {
+    return reinterpret_cast<unsigned long long *>(static_cast<char *>(plan->scratch) +
+                                                  exact_offset());
 }
 
 bool finite_positive(double v) { return isfinite(v) && v > 0; }

@@ -1332,8 +1332,8 @@ __global__ void __launch_bounds__(32 * kRefineWarps) cont_fit_refine_kernel(
 // every sum keeps the 2^-50 of its terms; terms of 2^kCoarseTop and more, below
 // 2^-78, or none go straight to the FP64 result. Calls whose words do not fit in shared memory keep the pairs. 1,024
 // threads (a block an SM; 512 leave the chains of word adds less to overlap
-// with). Five passes over 40,000 forests of 160 pixels: 1.45 ms in pairs, 1.67 ms
-// exact (1.95 ms in blocks of 512).
+// with). Five passes over 40,000 forests of 160 pixels: 1.45 ms in pairs, 1.57 ms
+// exact (1.60 where the blocks end on carries in global memory, 1.95 in blocks of 512).
 constexpr int kStackBlock = 512;
 constexpr int kStackGroup = 8;
 // 2^25 terms at the top of each range stay below 2^(127 - scale)
@@ -1407,14 +1407,22 @@ __device__ __forceinline__ void fix_add_words(uint32_t *const h[N], int stride,
     }
 }
 
+// Adds a number to one in global memory, whose words are added to 64-bit counters
+// (at sum, sum + stride, ...; up to 2^32 numbers) so that no carry is waited for.
+__device__ __forceinline__ void fix_add_global(unsigned long long *sum, int stride,
+                                               const uint32_t word[4]) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (word[k]) atomicAdd(sum + k * stride, (unsigned long long)word[k]);
+}
+
 // t 2^p as four words, |t| < 2^51, 0 <= p < 64 (WIDE: 96).
 template <bool WIDE>
 __device__ __forceinline__ void fix_words(long long t, int p, uint32_t word[4]) {
-    const int s = p & 31;
-    const unsigned long long low = (unsigned long long)t << s;
-    const uint32_t a = (uint32_t)low, b = (uint32_t)(low >> 32);
-    const uint32_t c = (uint32_t)((t >> 32) >> (32 - s));  // from bit 64 on
-    const uint32_t sign = (uint32_t)(t >> 63);
+    const uint32_t lo = (uint32_t)t, hi = (uint32_t)((unsigned long long)t >> 32);
+    const uint32_t sign = (uint32_t)((int)hi >> 31);
+    const uint32_t a = lo << (p & 31);  // the shifts go by the low five bits of p
+    const uint32_t b = __funnelshift_l(lo, hi, p), c = __funnelshift_l(hi, sign, p);
     const bool up = p >= 32, upper = WIDE && p >= 64;
     word[0] = up ? 0u : a;
     word[1] = upper ? 0u : (up ? a : b);
@@ -1426,15 +1434,16 @@ __device__ __forceinline__ void fix_words(long long t, int p, uint32_t word[4]) 
 // exponent of v.hi, 49 to 254).
 __device__ __forceinline__ long long fix_digits(dfl v, int e) {
     const uint32_t u = __float_as_uint(v.hi);
-    const long long m = (u & 0x7FFFFFu) | 0x800000u;
+    const int m = (int)((u & 0x7FFFFFu) | 0x800000u);
     const float lo = v.lo * __uint_as_float((uint32_t)(303 - e) << 23);
-    return ((int)u < 0 ? -m : m) * (1LL << 26) + __float2int_rn(lo);
+    return (long long)((int)u < 0 ? -m : m) * (1 << 26) + __float2int_rn(lo);
 }
 
-// The number in four words, in units of 2^-scale.
-__device__ __forceinline__ double fix_value(const uint32_t word[4], int scale) {
-    unsigned long long hi = (unsigned long long)word[3] << 32 | word[2];
-    unsigned long long lo = (unsigned long long)word[1] << 32 | word[0];
+// The number whose words were added to sum[0..3], in units of 2^-scale.
+__device__ __forceinline__ double fix_value(const unsigned long long sum[4], int scale) {
+    const unsigned long long s1 = sum[1] + (sum[0] >> 32), s2 = sum[2] + (s1 >> 32);
+    unsigned long long hi = ((sum[3] + (s2 >> 32)) << 32) | (s2 & 0xFFFFFFFFull);
+    unsigned long long lo = (s1 << 32) | (sum[0] & 0xFFFFFFFFull);
     const bool negative = (long long)hi < 0;
     if (negative) {
         lo = 0ull - lo;
@@ -1448,8 +1457,8 @@ __device__ __forceinline__ double fix_value(const uint32_t word[4], int scale) {
 // the bin's coarse number; below 2^kFineLow the part in units of 2^-kFixScale to
 // the fine number (of the block, at fine) and what is left of it to the small
 // number; infinities, NaN and what no number holds to the FP64 result.
-__device__ __noinline__ void stack_add_rare(uint32_t *fine, uint32_t *work, int nc, int cell,
-                                            double *dst, dfl v) {
+__device__ __noinline__ void stack_add_rare(uint32_t *fine, unsigned long long *work, int nc,
+                                            int cell, double *dst, dfl v) {
     const int e = (int)((__float_as_uint(v.hi) >> 23) & 0xFFu);
     uint32_t word[1][4];
     if (e >= 127 + kCoarseTop || e < 127 - 78) {
@@ -1457,10 +1466,9 @@ __device__ __noinline__ void stack_add_rare(uint32_t *fine, uint32_t *work, int 
         return;
     }
     const long long t = fix_digits(v, e);
-    uint32_t *at[1] = {work + 4 * nc + cell};
     if (e >= 127 + kFineTop) {
         fix_words<false>(t, e - 176 + kCoarseScale, word[0]);
-        fix_add_words<1>(at, nc, word);
+        fix_add_global(work + 4 * nc + cell, nc, word[0]);
         return;
     }
     const int below = 176 - kFixScale - e;  // bits of t below the fine number's last place
@@ -1468,18 +1476,17 @@ __device__ __noinline__ void stack_add_rare(uint32_t *fine, uint32_t *work, int 
     uint32_t *at_fine[1] = {fine};
     fix_words<false>(whole, 0, word[0]);
     fix_add_words<1>(at_fine, nc, word);
-    at[0] = work + 8 * nc + cell;
     fix_words<true>(t - whole * (1LL << below), e - 176 + kSmallScale, word[0]);
-    fix_add_words<1>(at, nc, word);
+    fix_add_global(work + 8 * nc + cell, nc, word[0]);
 }
 
-// exact_work (EXACT): kStackNumbers x 4 words of every cell, zeroed: the blocks'
-// sums, the terms of 2^kFineTop and more, the parts below 2^-kFixScale.
+// exact_work (EXACT): kStackNumbers x 4 counters of every cell, zeroed: the
+// blocks' sums, the terms of 2^kFineTop and more, the parts below 2^-kFixScale.
 template <bool EXACT, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) cont_stacks_kernel(
     const __grid_constant__ pg_spectra sp, const __grid_constant__ pg_cont_model m,
     const __grid_constant__ pg_cont_fit fit, const __grid_constant__ pg_cont_stacks st,
-    Scratch *scratch, int use_table, uint32_t *exact_work) {
+    Scratch *scratch, int use_table, unsigned long long *exact_work) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ uint32_t seen[BLOCK / 32][64];  // per-warp bitmap of var bins (<= 2048)
     __shared__ StackSlot s_slots[BLOCK / 32][kStackGroup];
@@ -1754,10 +1761,8 @@ __global__ void __launch_bounds__(BLOCK) cont_stacks_kernel(
     }
     if (EXACT) {
         for (int k = threadIdx.x; k < nc; k += blockDim.x) {
-            const uint32_t word[1][4] = {
-                {hist[k], hist[nc + k], hist[2 * nc + k], hist[3 * nc + k]}};
-            uint32_t *const at[1] = {exact_work + k};
-            fix_add_words<1>(at, nc, word);
+            const uint32_t word[4] = {hist[k], hist[nc + k], hist[2 * nc + k], hist[3 * nc + k]};
+            fix_add_global(exact_work + k, nc, word);
         }
         return;
     }
@@ -1780,7 +1785,7 @@ __global__ void __launch_bounds__(BLOCK) cont_stacks_kernel(
 
 // The fixed-point sums of all blocks, added to the FP64 results.
 __global__ void cont_stacks_finish_kernel(const __grid_constant__ pg_cont_stacks st,
-                                          const uint32_t *exact_work) {
+                                          const unsigned long long *exact_work) {
     const StackCells c = stack_cells(st);
     const int k = blockIdx.x * blockDim.x + threadIdx.x, nc = c.total;
     if (k >= nc) return;
@@ -1793,11 +1798,11 @@ __global__ void cont_stacks_finish_kernel(const __grid_constant__ pg_cont_stacks
     else if (k < c.v_d2) { dst = st.var_mean; from = c.v_mean; }
     else if (k < c.v_d4) { dst = st.var_delta2; from = c.v_d2; }
     else { dst = st.var_delta4; from = c.v_d4; }
-    uint32_t word[kStackNumbers][4];
+    unsigned long long sum[kStackNumbers][4];
 #pragma unroll
-    for (int w = 0; w < kStackNumbers * 4; ++w) word[w >> 2][w & 3] = exact_work[w * nc + k];
-    dst[k - from] += fix_value(word[0], kFixScale) + fix_value(word[1], kCoarseScale) +
-                     fix_value(word[2], kSmallScale);
+    for (int w = 0; w < kStackNumbers * 4; ++w) sum[w >> 2][w & 3] = exact_work[w * nc + k];
+    dst[k - from] += fix_value(sum[0], kFixScale) + fix_value(sum[1], kCoarseScale) +
+                     fix_value(sum[2], kSmallScale);
 }
 
 // Deltas and weights (populate_los_ids, extract_deltas). Bound: the FP64 pipe.
@@ -2028,8 +2033,9 @@ constexpr size_t kStackLimit = 200 * 1024;  // shared memory of a block
 // where it fits beside the histograms.
 template <bool EXACT, int BLOCK>
 static int launch_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_cont_fit &fit,
-                         const pg_cont_stacks &st, bool use_table, uint32_t *exact_work,
-                         Scratch *scratch, int num_sms, cudaStream_t stream) {
+                         const pg_cont_stacks &st, bool use_table,
+                         unsigned long long *exact_work, Scratch *scratch, int num_sms,
+                         cudaStream_t stream) {
     const auto kernel = cont_stacks_kernel<EXACT, BLOCK>;
     const size_t smem = stack_bytes(st, EXACT, use_table);
     cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2048,12 +2054,13 @@ static int launch_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_
     return check_cuda(cudaGetLastError());
 }
 
-// 16 bytes of shared memory a cell, as many of the work for each number
-size_t cont_exact_bytes() { return kStackNumbers * kStackLimit; }
+// 16 bytes of shared memory a cell, 32 of the work for each number
+size_t cont_exact_bytes() { return 2 * kStackNumbers * kStackLimit; }
 
 int launch_cont_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_cont_fit &fit,
-                       const pg_cont_stacks &st, uint32_t *exact_work, size_t exact_bytes,
-                       Scratch *scratch, int num_sms, cudaStream_t stream) {
+                       const pg_cont_stacks &st, unsigned long long *exact_work,
+                       size_t exact_bytes, Scratch *scratch, int num_sms,
+                       cudaStream_t stream) {
     if (sp.num <= 0) return PG_OK;
     if (st.var_mean && st.var_lambda_bins * kVarBins > 2048) return PG_ERR_UNSUPPORTED;
     constexpr size_t limit = kStackLimit;
@@ -2061,7 +2068,7 @@ int launch_cont_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_co
     const bool pair_table = want_table && stack_smem_bytes(st, true) <= limit;
     if (stack_smem_bytes(st, pair_table) > limit) return PG_ERR_UNSUPPORTED;
     const StackCells cells = stack_cells(st);
-    const size_t work = (size_t)cells.total * 16 * kStackNumbers;
+    const size_t work = (size_t)cells.total * 32 * kStackNumbers;
     if (stack_bytes(st, true, false) > limit || work > exact_bytes)
         return launch_stacks<false, kStackBlock>(sp, m, fit, st, pair_table, nullptr, scratch,
                                                  num_sms, stream);

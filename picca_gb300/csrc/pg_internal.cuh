@@ -343,7 +343,8 @@ int launch_cont_fit(const pg_spectra &sp, const pg_cont_model &m, const double *
                     const pg_cont_fit &out, Scratch *scratch, int num_sms, cudaStream_t stream,
                     float cert_chi2 = 0.f, float cert_ab = 0.f);
 int launch_cont_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_cont_fit &fit,
-                       const pg_cont_stacks &st, uint32_t *exact_work, size_t exact_bytes,
+                       const pg_cont_stacks &st, unsigned long long *exact_work,
+                       size_t exact_bytes,
                        Scratch *scratch, int num_sms, cudaStream_t stream);
 // work of the histograms' fixed-point sums that holds any covered call's
 size_t cont_exact_bytes();
