@@ -1340,7 +1340,6 @@ constexpr int kStackGroup = 8;
 constexpr int kFixScale = 88, kFineLow = -39, kFineTop = 14;
 constexpr int kCoarseScale = 56, kCoarseTop = 46;
 constexpr int kSmallScale = 168;  // parts below 2^-kFixScale
-constexpr int kStackNumbers = 3;  // of a cell in global memory
 
 struct StackSlot {
     int64_t off;
@@ -1457,8 +1456,8 @@ __device__ __forceinline__ double fix_value(const unsigned long long sum[4], int
 // the bin's coarse number; below 2^kFineLow the part in units of 2^-kFixScale to
 // the fine number (of the block, at fine) and what is left of it to the small
 // number; infinities, NaN and what no number holds to the FP64 result.
-__device__ __noinline__ void stack_add_rare(uint32_t *fine, unsigned long long *work, int nc,
-                                            int cell, double *dst, dfl v) {
+__device__ __noinline__ void stack_add_rare(uint32_t *fine, uint32_t *rare, int nc, int cell,
+                                            double *dst, dfl v) {
     const int e = (int)((__float_as_uint(v.hi) >> 23) & 0xFFu);
     uint32_t word[1][4];
     if (e >= 127 + kCoarseTop || e < 127 - 78) {
@@ -1466,9 +1465,10 @@ __device__ __noinline__ void stack_add_rare(uint32_t *fine, unsigned long long *
         return;
     }
     const long long t = fix_digits(v, e);
+    uint32_t *at[1] = {rare + cell};
     if (e >= 127 + kFineTop) {
         fix_words<false>(t, e - 176 + kCoarseScale, word[0]);
-        fix_add_global(work + 4 * nc + cell, nc, word[0]);
+        fix_add_words<1>(at, nc, word);
         return;
     }
     const int below = 176 - kFixScale - e;  // bits of t below the fine number's last place
@@ -1476,12 +1476,13 @@ __device__ __noinline__ void stack_add_rare(uint32_t *fine, unsigned long long *
     uint32_t *at_fine[1] = {fine};
     fix_words<false>(whole, 0, word[0]);
     fix_add_words<1>(at_fine, nc, word);
+    at[0] = rare + 4 * nc + cell;
     fix_words<true>(t - whole * (1LL << below), e - 176 + kSmallScale, word[0]);
-    fix_add_global(work + 8 * nc + cell, nc, word[0]);
+    fix_add_words<1>(at, nc, word);
 }
 
-// exact_work (EXACT): kStackNumbers x 4 counters of every cell, zeroed: the
-// blocks' sums, the terms of 2^kFineTop and more, the parts below 2^-kFixScale.
+// exact_work (EXACT), zeroed: 4 counters of every cell for the blocks' sums, then
+// 4 words for the terms of 2^kFineTop and more, 4 for the parts below 2^-kFixScale.
 template <bool EXACT, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) cont_stacks_kernel(
     const __grid_constant__ pg_spectra sp, const __grid_constant__ pg_cont_model m,
@@ -1504,6 +1505,7 @@ __global__ void __launch_bounds__(BLOCK) cont_stacks_kernel(
     uint32_t *v_np = hist + kPlanes * nc, *v_nq = v_np + nvar;
     const int nwords = kPlanes * nc + 2 * nvar;
     for (int k = threadIdx.x; k < nwords; k += blockDim.x) hist[k] = 0u;
+    uint32_t *const rare = reinterpret_cast<uint32_t *>(exact_work + 4 * nc);
     // N terms v to the cells, whose FP64 results are at dst
     auto add = [&](auto count, const int *cell, double *const *dst, const dfl *v) {
         constexpr int N = decltype(count)::value;
@@ -1522,7 +1524,7 @@ __global__ void __launch_bounds__(BLOCK) cont_stacks_kernel(
             fix_words<false>(fine ? fix_digits(v[n], e) : 0, fine ? e - 176 + kFixScale : 0,
                              word[n]);
             if (!fine && v[n].hi != 0.f)
-                stack_add_rare(hist + cell[n], exact_work, nc, cell[n], dst[n], v[n]);
+                stack_add_rare(hist + cell[n], rare, nc, cell[n], dst[n], v[n]);
         }
         fix_add_words<N>(at, nc, word);
     };
@@ -1798,11 +1800,16 @@ __global__ void cont_stacks_finish_kernel(const __grid_constant__ pg_cont_stacks
     else if (k < c.v_d2) { dst = st.var_mean; from = c.v_mean; }
     else if (k < c.v_d4) { dst = st.var_delta2; from = c.v_d2; }
     else { dst = st.var_delta4; from = c.v_d4; }
-    unsigned long long sum[kStackNumbers][4];
+    const uint32_t *rare = reinterpret_cast<const uint32_t *>(exact_work + 4 * nc);
+    unsigned long long fine[4], coarse[4], small[4];
 #pragma unroll
-    for (int w = 0; w < kStackNumbers * 4; ++w) sum[w >> 2][w & 3] = exact_work[w * nc + k];
-    dst[k - from] += fix_value(sum[0], kFixScale) + fix_value(sum[1], kCoarseScale) +
-                     fix_value(sum[2], kSmallScale);
+    for (int w = 0; w < 4; ++w) {
+        fine[w] = exact_work[w * nc + k];
+        coarse[w] = rare[w * nc + k];
+        small[w] = rare[(4 + w) * nc + k];
+    }
+    dst[k - from] += fix_value(fine, kFixScale) + fix_value(coarse, kCoarseScale) +
+                     fix_value(small, kSmallScale);
 }
 
 // Deltas and weights (populate_los_ids, extract_deltas). Bound: the FP64 pipe.
@@ -2054,8 +2061,10 @@ static int launch_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_
     return check_cuda(cudaGetLastError());
 }
 
-// 16 bytes of shared memory a cell, 32 of the work for each number
-size_t cont_exact_bytes() { return 2 * kStackNumbers * kStackLimit; }
+// a cell has 16 bytes of shared memory and kStackWork of the work (with 32 more,
+// all numbers in counters, a plan takes over 1 MB and 0.07 ms more to make)
+constexpr size_t kStackWork = 64;
+size_t cont_exact_bytes() { return kStackLimit / 16 * kStackWork; }
 
 int launch_cont_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_cont_fit &fit,
                        const pg_cont_stacks &st, unsigned long long *exact_work,
@@ -2068,7 +2077,7 @@ int launch_cont_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_co
     const bool pair_table = want_table && stack_smem_bytes(st, true) <= limit;
     if (stack_smem_bytes(st, pair_table) > limit) return PG_ERR_UNSUPPORTED;
     const StackCells cells = stack_cells(st);
-    const size_t work = (size_t)cells.total * 32 * kStackNumbers;
+    const size_t work = (size_t)cells.total * kStackWork;
     if (stack_bytes(st, true, false) > limit || work > exact_bytes)
         return launch_stacks<false, kStackBlock>(sp, m, fit, st, pair_table, nullptr, scratch,
                                                  num_sms, stream);
