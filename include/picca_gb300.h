@@ -139,7 +139,7 @@ typedef struct pg_plan pg_plan;
 const char *pg_strerror(int status);
 int pg_version(void);
 
-/* Create a plan on the CURRENT device (allocates 0.8 MB of device scratch)
+/* Create a plan on the CURRENT device (allocates 0.9 MB of device scratch)
  * / release it. */
 int pg_plan_create(pg_plan **plan);
 int pg_plan_destroy(pg_plan *plan);

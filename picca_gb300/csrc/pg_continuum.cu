@@ -1340,6 +1340,7 @@ constexpr int kStackGroup = 8;
 constexpr int kFixScale = 88, kFineLow = -39, kFineTop = 14;
 constexpr int kCoarseScale = 56, kCoarseTop = 46;
 constexpr int kSmallScale = 168;  // parts below 2^-kFixScale
+constexpr int kStackNumbers = 3;  // of a cell in global memory
 
 struct StackSlot {
     int64_t off;
@@ -1406,13 +1407,15 @@ __device__ __forceinline__ void fix_add_words(uint32_t *const h[N], int stride,
     }
 }
 
-// Adds a number to one in global memory, whose words are added to 64-bit counters
-// (at sum, sum + stride, ...; up to 2^32 numbers) so that no carry is waited for.
+// Adds a number to one in global memory: three 64-bit counters (at sum, sum +
+// stride, ...) take word 0, word 1 and the upper half, so that no carry is waited
+// for (up to 2^32 numbers).
 __device__ __forceinline__ void fix_add_global(unsigned long long *sum, int stride,
                                                const uint32_t word[4]) {
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        if (word[k]) atomicAdd(sum + k * stride, (unsigned long long)word[k]);
+    const unsigned long long upper = (unsigned long long)word[3] << 32 | word[2];
+    if (word[0]) atomicAdd(sum, (unsigned long long)word[0]);
+    if (word[1]) atomicAdd(sum + stride, (unsigned long long)word[1]);
+    if (upper) atomicAdd(sum + 2 * stride, upper);
 }
 
 // t 2^p as four words, |t| < 2^51, 0 <= p < 64 (WIDE: 96).
@@ -1438,10 +1441,10 @@ __device__ __forceinline__ long long fix_digits(dfl v, int e) {
     return (long long)((int)u < 0 ? -m : m) * (1 << 26) + __float2int_rn(lo);
 }
 
-// The number whose words were added to sum[0..3], in units of 2^-scale.
-__device__ __forceinline__ double fix_value(const unsigned long long sum[4], int scale) {
-    const unsigned long long s1 = sum[1] + (sum[0] >> 32), s2 = sum[2] + (s1 >> 32);
-    unsigned long long hi = ((sum[3] + (s2 >> 32)) << 32) | (s2 & 0xFFFFFFFFull);
+// The number in three counters, in units of 2^-scale.
+__device__ __forceinline__ double fix_value(const unsigned long long sum[3], int scale) {
+    const unsigned long long s1 = sum[1] + (sum[0] >> 32);
+    unsigned long long hi = sum[2] + (s1 >> 32);
     unsigned long long lo = (s1 << 32) | (sum[0] & 0xFFFFFFFFull);
     const bool negative = (long long)hi < 0;
     if (negative) {
@@ -1456,8 +1459,8 @@ __device__ __forceinline__ double fix_value(const unsigned long long sum[4], int
 // the bin's coarse number; below 2^kFineLow the part in units of 2^-kFixScale to
 // the fine number (of the block, at fine) and what is left of it to the small
 // number; infinities, NaN and what no number holds to the FP64 result.
-__device__ __noinline__ void stack_add_rare(uint32_t *fine, uint32_t *rare, int nc, int cell,
-                                            double *dst, dfl v) {
+__device__ __noinline__ void stack_add_rare(uint32_t *fine, unsigned long long *work, int nc,
+                                            int cell, double *dst, dfl v) {
     const int e = (int)((__float_as_uint(v.hi) >> 23) & 0xFFu);
     uint32_t word[1][4];
     if (e >= 127 + kCoarseTop || e < 127 - 78) {
@@ -1465,10 +1468,9 @@ __device__ __noinline__ void stack_add_rare(uint32_t *fine, uint32_t *rare, int 
         return;
     }
     const long long t = fix_digits(v, e);
-    uint32_t *at[1] = {rare + cell};
     if (e >= 127 + kFineTop) {
         fix_words<false>(t, e - 176 + kCoarseScale, word[0]);
-        fix_add_words<1>(at, nc, word);
+        fix_add_global(work + 3 * nc + cell, nc, word[0]);
         return;
     }
     const int below = 176 - kFixScale - e;  // bits of t below the fine number's last place
@@ -1476,13 +1478,12 @@ __device__ __noinline__ void stack_add_rare(uint32_t *fine, uint32_t *rare, int 
     uint32_t *at_fine[1] = {fine};
     fix_words<false>(whole, 0, word[0]);
     fix_add_words<1>(at_fine, nc, word);
-    at[0] = rare + 4 * nc + cell;
     fix_words<true>(t - whole * (1LL << below), e - 176 + kSmallScale, word[0]);
-    fix_add_words<1>(at, nc, word);
+    fix_add_global(work + 6 * nc + cell, nc, word[0]);
 }
 
-// exact_work (EXACT), zeroed: 4 counters of every cell for the blocks' sums, then
-// 4 words for the terms of 2^kFineTop and more, 4 for the parts below 2^-kFixScale.
+// exact_work (EXACT): kStackNumbers x 3 counters of every cell, zeroed: the
+// blocks' sums, the terms of 2^kFineTop and more, the parts below 2^-kFixScale.
 template <bool EXACT, int BLOCK>
 __global__ void __launch_bounds__(BLOCK) cont_stacks_kernel(
     const __grid_constant__ pg_spectra sp, const __grid_constant__ pg_cont_model m,
@@ -1505,7 +1506,6 @@ __global__ void __launch_bounds__(BLOCK) cont_stacks_kernel(
     uint32_t *v_np = hist + kPlanes * nc, *v_nq = v_np + nvar;
     const int nwords = kPlanes * nc + 2 * nvar;
     for (int k = threadIdx.x; k < nwords; k += blockDim.x) hist[k] = 0u;
-    uint32_t *const rare = reinterpret_cast<uint32_t *>(exact_work + 4 * nc);
     // N terms v to the cells, whose FP64 results are at dst
     auto add = [&](auto count, const int *cell, double *const *dst, const dfl *v) {
         constexpr int N = decltype(count)::value;
@@ -1524,7 +1524,7 @@ __global__ void __launch_bounds__(BLOCK) cont_stacks_kernel(
             fix_words<false>(fine ? fix_digits(v[n], e) : 0, fine ? e - 176 + kFixScale : 0,
                              word[n]);
             if (!fine && v[n].hi != 0.f)
-                stack_add_rare(hist + cell[n], rare, nc, cell[n], dst[n], v[n]);
+                stack_add_rare(hist + cell[n], exact_work, nc, cell[n], dst[n], v[n]);
         }
         fix_add_words<N>(at, nc, word);
     };
@@ -1800,16 +1800,11 @@ __global__ void cont_stacks_finish_kernel(const __grid_constant__ pg_cont_stacks
     else if (k < c.v_d2) { dst = st.var_mean; from = c.v_mean; }
     else if (k < c.v_d4) { dst = st.var_delta2; from = c.v_d2; }
     else { dst = st.var_delta4; from = c.v_d4; }
-    const uint32_t *rare = reinterpret_cast<const uint32_t *>(exact_work + 4 * nc);
-    unsigned long long fine[4], coarse[4], small[4];
+    unsigned long long sum[kStackNumbers][3];
 #pragma unroll
-    for (int w = 0; w < 4; ++w) {
-        fine[w] = exact_work[w * nc + k];
-        coarse[w] = rare[w * nc + k];
-        small[w] = rare[(4 + w) * nc + k];
-    }
-    dst[k - from] += fix_value(fine, kFixScale) + fix_value(coarse, kCoarseScale) +
-                     fix_value(small, kSmallScale);
+    for (int w = 0; w < kStackNumbers * 3; ++w) sum[w / 3][w % 3] = exact_work[w * nc + k];
+    dst[k - from] += fix_value(sum[0], kFixScale) + fix_value(sum[1], kCoarseScale) +
+                     fix_value(sum[2], kSmallScale);
 }
 
 // Deltas and weights (populate_los_ids, extract_deltas). Bound: the FP64 pipe.
@@ -2061,9 +2056,9 @@ static int launch_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_
     return check_cuda(cudaGetLastError());
 }
 
-// a cell has 16 bytes of shared memory and kStackWork of the work (with 32 more,
-// all numbers in counters, a plan takes over 1 MB and 0.07 ms more to make)
-constexpr size_t kStackWork = 64;
+// a cell has 16 bytes of shared memory and kStackWork of the work (a plan with
+// over 1 MB, as four counters a number would need, takes 0.07 ms more to make)
+constexpr size_t kStackWork = 24 * kStackNumbers;
 size_t cont_exact_bytes() { return kStackLimit / 16 * kStackWork; }
 
 int launch_cont_stacks(const pg_spectra &sp, const pg_cont_model &m, const pg_cont_fit &fit,
